@@ -52,7 +52,10 @@ enum { TDCC_T1 = 0, TDCC_T2 = 1, TDCC_L1 = 2, TDCC_L2 = 3 };
 
 /* contraction arithmetic */
 enum {
-  TDCC_PREC_FP64 = 0,      /* every contraction in FP64 (the plain form)   */
+  TDCC_PREC_FP64 = 0,      /* the plain form: contractions in 56-bit block
+                              fixed point with exact sums, rounded to FP64
+                              once per K chunk of at most 60; FP64 everywhere
+                              else                                         */
   TDCC_PREC_MIXED = 1      /* large contractions as split-BF16 tcgen05
                               products, FP64 everywhere else               */
 };

@@ -356,13 +356,15 @@ void coalesce(AddArgs& a);
 // op inherits the varying / constant flags of the forward op it reverses.
 void build_adjoint(const Program& f, Program& a, std::vector<int>& adj_of);
 
-// FP64 contraction tile shapes (kernels.cu)
-constexpr int kNumTiles = 7;
+// fixed-point contraction of the FP64 form: tile shapes, and the tile and K
+// splits of given extents (gemm_fx.cu; tile >= 0: that one)
+constexpr int kNumTiles = 5;
 extern const int kTiles[kNumTiles][2];
-int choose_tile(long long M, long long N);
-bool tile_fits(int tile, long long M);  // the M tiles fit the launch grid
+bool tile_fits(int tile, bool real_operands);
+void choose_fx(long long M, long long N, long long K, long long nb, bool ac, bool bc, bool allow_split, int tile,
+               int* best_tile, int* best_splits);
 
-// kernel launchers (kernels.cu)
+// kernel launchers
 cudaError_t launch_gemm(const Op& op, const void* A, const void* B, void* C, cudaStream_t st);
 cudaError_t launch_pack(const PackArgs& p, cudaStream_t st);
 cudaError_t launch_ozaki(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st);

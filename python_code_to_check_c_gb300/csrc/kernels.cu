@@ -1,6 +1,5 @@
-// FP64 kernels of the plain form: strided tensor contraction (GEMM over
-// flattened mode groups), elementwise accumulate with antisymmetrisers, and
-// the dipole trace.  All complex data is interleaved (double2).
+// Elementwise accumulate with antisymmetrisers, reductions and the dipole
+// trace, in FP64.  All complex data is interleaved (double2).
 #include <atomic>
 #include <cstdio>
 #include <type_traits>
@@ -13,253 +12,7 @@ static std::atomic<long long> g_launches{0};
 void count_launch(long long k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(); }
 
-// ---------------------------------------------------------------------------
-// helpers
-// ---------------------------------------------------------------------------
-template <bool CPLX>
-struct Elem;
-template <>
-struct Elem<true> {
-  using T = double2;
-};
-template <>
-struct Elem<false> {
-  using T = double;
-};
-
 __device__ __forceinline__ double2 cz() { return make_double2(0.0, 0.0); }
-
-__device__ __forceinline__ double2 as2(double x) { return make_double2(x, 0.0); }
-__device__ __forceinline__ double2 as2(double2 x) { return x; }
-
-// acc += a * b for the four real/complex combinations
-__device__ __forceinline__ void mac(double2& c, double a, double b) { c.x = fma(a, b, c.x); }
-__device__ __forceinline__ void mac(double2& c, double a, double2 b) {
-  c.x = fma(a, b.x, c.x);
-  c.y = fma(a, b.y, c.y);
-}
-__device__ __forceinline__ void mac(double2& c, double2 a, double b) {
-  c.x = fma(a.x, b, c.x);
-  c.y = fma(a.y, b, c.y);
-}
-__device__ __forceinline__ void mac(double2& c, double2 a, double2 b) {
-  c.x = fma(a.x, b.x, c.x);
-  c.x = fma(-a.y, b.y, c.x);
-  c.y = fma(a.x, b.y, c.y);
-  c.y = fma(a.y, b.x, c.y);
-}
-
-__device__ __forceinline__ void decomp(const ModeGroup& g, int l, long long& o0, long long& o1) {
-  o0 = 0;
-  o1 = 0;
-#pragma unroll
-  for (int q = kMaxModes - 1; q >= 0; --q) {
-    if (q < g.n) {
-      const int d = g.dim[q];
-      const int r = l % d;
-      l /= d;
-      o0 += (long long)r * g.s0[q];
-      o1 += (long long)r * g.s1[q];
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// FP64 contraction: C[m,n] (+)= alpha * sum_k A[m,k] B[k,n]
-// BM x BN output tile, K step 16, 256 threads, TM x TN outputs per thread
-// (strided by BM/TM and BN/TN so shared-memory reads are conflict free).  On
-// GB300 the FP64 pipe (~1.2 TFLOP/s) is the bound, so the tile shape is
-// chosen per contraction to minimise padded (wasted) multiply-adds.
-// ---------------------------------------------------------------------------
-constexpr int GBK = 16;
-
-template <bool AC, bool BC, bool CC, int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(256) gemm_f64_kernel(const GemmArgs g) {
-  static_assert((BM / TM) * (BN / TN) == 256, "256 threads");
-  static_assert(256 % BM == 0 && 256 % BN == 0, "tile rows divide the CTA");
-  using TA = typename Elem<AC>::T;
-  using TB = typename Elem<BC>::T;
-  constexpr int RX = BN / TN, RY = BM / TM;  // thread grid
-  constexpr int LA = BM * GBK / 256, LB = BN * GBK / 256;
-  __shared__ TA As[GBK][BM];
-  __shared__ TB Bs[GBK][BN];
-
-  const int tid = threadIdx.x;
-  const int tx = tid % RX, ty = tid / RX;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int zb = blockIdx.z / g.nsplit;          // batch
-  const int ks = blockIdx.z - zb * g.nsplit;     // K split
-  const int kbeg = ks * g.kchunk;
-  const int kend = min(g.K, kbeg + g.kchunk);
-
-  const TA* A = static_cast<const TA*>(g.A) + zb * g.bsA;
-  const TB* B = static_cast<const TB*>(g.B) + zb * g.bsB;
-
-  // this thread's load row (A) / column (B) and their base offsets
-  const int ar = tid % BM, ak0 = tid / BM;
-  const int br = tid % BN, bk0 = tid / BN;
-  const int am = m0 + ar, bn = n0 + br;
-  long long aoff = 0, boff = 0, dummy;
-  if (am < g.M) decomp(g.gm, am, aoff, dummy);
-  if (bn < g.N) decomp(g.gn, bn, boff, dummy);
-
-  double2 acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = cz();
-
-  for (int k0 = kbeg; k0 < kend; k0 += GBK) {
-#pragma unroll
-    for (int r = 0; r < LA; ++r) {
-      const int kk = ak0 + (256 / BM) * r;
-      const int k = k0 + kk;
-      TA av{};
-      if (k < kend && am < g.M) {
-        long long ka, kb;
-        decomp(g.gk, k, ka, kb);
-        av = A[aoff + ka];
-      }
-      As[kk][ar] = av;
-    }
-#pragma unroll
-    for (int r = 0; r < LB; ++r) {
-      const int kk = bk0 + (256 / BN) * r;
-      const int k = k0 + kk;
-      TB bv{};
-      if (k < kend && bn < g.N) {
-        long long ka, kb;
-        decomp(g.gk, k, ka, kb);
-        bv = B[boff + kb];
-      }
-      Bs[kk][br] = bv;
-    }
-    __syncthreads();
-    // the last K step of a short K range stops at its end (K = o = 10 would
-    // otherwise spend 6 of 16 multiply-adds on zero padding)
-    const int kmax = min(GBK, kend - k0);
-#pragma unroll 4
-    for (int kk = 0; kk < kmax; ++kk) {
-      TA a[TM];
-      TB b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty + RY * i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx + RX * j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) mac(acc[i][j], a[i], b[j]);
-    }
-    __syncthreads();
-  }
-
-  long long coffm[TM], coffn[TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty + RY * i;
-    coffm[i] = 0;
-    if (m < g.M) decomp(g.gm, m, dummy, coffm[i]);
-  }
-#pragma unroll
-  for (int j = 0; j < TN; ++j) {
-    const int n = n0 + tx + RX * j;
-    coffn[j] = 0;
-    if (n < g.N) decomp(g.gn, n, dummy, coffn[j]);
-  }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty + RY * i;
-    if (m >= g.M) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int n = n0 + tx + RX * j;
-      if (n >= g.N) continue;
-      const double2 s = acc[i][j];
-      const long long off = coffm[i] + coffn[j];
-      if constexpr (CC) {
-        double2* C = static_cast<double2*>(g.C) + zb * g.bsC;
-        const double2 v = make_double2(g.ar * s.x - g.ai * s.y, g.ar * s.y + g.ai * s.x);
-        if (g.atomic || g.acc) {  // L2 reductions (one writer per element unless split)
-          atomicAdd(&C[off].x, v.x);
-          atomicAdd(&C[off].y, v.y);
-        } else {
-          C[off] = v;
-        }
-      } else {
-        double* C = static_cast<double*>(g.C) + zb * g.bsC;
-        const double v = g.ar * s.x;
-        if (g.atomic || g.acc)
-          atomicAdd(&C[off], v);
-        else
-          C[off] = v;
-      }
-    }
-  }
-}
-
-// tile shapes: {BM, BN}
-const int kTiles[kNumTiles][2] = {{64, 64}, {32, 64}, {64, 32}, {32, 32}, {16, 16}, {16, 128}, {128, 16}};
-
-bool tile_fits(int t, long long M) { return (M + kTiles[t][0] - 1) / kTiles[t][0] <= 65535; }  // grid.y
-
-int choose_tile(long long M, long long N) {
-  int best = 0;
-  double bc = 1e300;
-  for (int t = 0; t < kNumTiles; ++t) {
-    if (!tile_fits(t, M)) continue;
-    const long long bm = kTiles[t][0], bn = kTiles[t][1];
-    // padded multiply-adds, with a small penalty for less operand reuse
-    const double pen = (bm * bn >= 4096) ? 1.0 : (bm * bn >= 1024) ? 1.06 : 1.15;
-    const double cost = (double)((M + bm - 1) / bm * bm) * (double)((N + bn - 1) / bn * bn) * pen;
-    if (cost < bc) {
-      bc = cost;
-      best = t;
-    }
-  }
-  return best;
-}
-
-template <bool AC, bool BC, bool CC>
-static void launch_typed(int tile, dim3 grid, const GemmArgs& g, cudaStream_t st) {
-  switch (tile) {
-    case 0: gemm_f64_kernel<AC, BC, CC, 64, 64, 4, 4><<<grid, 256, 0, st>>>(g); break;
-    case 1: gemm_f64_kernel<AC, BC, CC, 32, 64, 2, 4><<<grid, 256, 0, st>>>(g); break;
-    case 2: gemm_f64_kernel<AC, BC, CC, 64, 32, 4, 2><<<grid, 256, 0, st>>>(g); break;
-    case 3: gemm_f64_kernel<AC, BC, CC, 32, 32, 2, 2><<<grid, 256, 0, st>>>(g); break;
-    case 5: gemm_f64_kernel<AC, BC, CC, 16, 128, 1, 8><<<grid, 256, 0, st>>>(g); break;
-    case 6: gemm_f64_kernel<AC, BC, CC, 128, 16, 8, 1><<<grid, 256, 0, st>>>(g); break;
-    default: gemm_f64_kernel<AC, BC, CC, 16, 16, 1, 1><<<grid, 256, 0, st>>>(g); break;
-  }
-}
-
-cudaError_t launch_gemm(const Op& op, const void* A, const void* B, void* C, cudaStream_t st) {
-  GemmArgs g = op.g;
-  g.A = A;
-  g.B = B;
-  g.C = C;
-  const int bm = kTiles[op.tile][0], bn = kTiles[op.tile][1];
-  const int gx = (g.N + bn - 1) / bn, gy = (g.M + bm - 1) / bm;
-  if (g.nb < 1) g.nb = 1;
-  if (g.nsplit < 1) g.nsplit = 1;
-  if ((long long)g.nsplit * g.kchunk < g.K) return cudaErrorInvalidValue;
-  const long long gz = (long long)g.nb * g.nsplit;
-  dim3 grid(gx, gy, (unsigned)gz);
-  if (gy > 65535 || gz > 65535) return cudaErrorInvalidConfiguration;
-  const bool ac = op.dta == C64, bc = op.dtb == C64, cc = op.dtc == C64;
-  if (ac && bc)
-    launch_typed<true, true, true>(op.tile, grid, g, st);
-  else if (ac && !bc)
-    launch_typed<true, false, true>(op.tile, grid, g, st);
-  else if (!ac && bc)
-    launch_typed<false, true, true>(op.tile, grid, g, st);
-  else if (cc)
-    launch_typed<false, false, true>(op.tile, grid, g, st);
-  else
-    launch_typed<false, false, false>(op.tile, grid, g, st);
-  count_launch();
-  return cudaGetLastError();
-}
 
 // ---------------------------------------------------------------------------
 // elementwise: C[idx] (+)= sum_t coef_t * A_t[idx] (* B_t[idx])

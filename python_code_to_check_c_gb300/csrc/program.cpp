@@ -223,6 +223,9 @@ void Program::ein(const char* spec, double ar, double ai, const View& A, const V
   g.ai = ai;
   g.acc = acc ? 1 : 0;
   g.nb = 1;
+  op.dta = A.dt;
+  op.dtb = B.dt;
+  op.dtc = C.dt;
   plan_gemm(op, true);
   op.sa = A.slot;
   op.sb = B.slot;
@@ -230,9 +233,6 @@ void Program::ein(const char* spec, double ar, double ai, const View& A, const V
   op.oa = A.off;
   op.ob = B.off;
   op.oc = C.off;
-  op.dta = A.dt;
-  op.dtb = B.dt;
-  op.dtc = C.dt;
   if (C.dt == R64 && (A.dt == C64 || B.dt == C64))
     throw std::runtime_error("einsum: complex product into real output: " + s);
   const int mult = (A.dt == C64 && B.dt == C64) ? 8 : (A.dt == C64 || B.dt == C64) ? 4 : 2;
@@ -253,27 +253,16 @@ void Program::ein(const char* spec, double ar, double ai, const View& A, const V
   ops.push_back(op);
 }
 
-// Tile shape, then split-K so that few output tiles still fill the 152 SMs
-// (only where the output is zeroed or accumulated into: splits add with
-// atomics).
+// Tile shape and K splits (splits only where the output is zeroed or
+// accumulated into: they add with atomics), from the kernel's cost model.
 void Program::plan_gemm(Op& op, bool allow_split, int tile) {
   GemmArgs& g = op.g;
-  const long long M = g.M, N = g.N, K = g.K, nbt = std::max(g.nb, 1);
-  op.tile = tile >= 0 ? tile : choose_tile(M, N);
-  const long long tiles = ((M + kTiles[op.tile][0] - 1) / kTiles[op.tile][0]) *
-                          ((N + kTiles[op.tile][1] - 1) / kTiles[op.tile][1]) * nbt;
-  long long splits = 1;
-  if (allow_split && tiles < 2 * 152 && K >= 64) {
-    splits = (2 * 152 + tiles - 1) / tiles;
-    splits = std::min<long long>(splits, K / 32);
-    splits = std::max<long long>(splits, 1);
-  }
-  long long kchunk = (K + splits - 1) / splits;
-  kchunk = ((kchunk + 15) / 16) * 16;
-  g.kchunk = (int)std::max<long long>(kchunk, 16);
-  splits = (K + g.kchunk - 1) / g.kchunk;
-  g.nsplit = (int)std::max<long long>(splits, 1);
-  g.atomic = splits > 1 ? 1 : 0;
+  const long long K = g.K;
+  int splits = 1;
+  choose_fx(g.M, g.N, K, std::max(g.nb, 1), op.dta == C64, op.dtb == C64, allow_split, tile, &op.tile, &splits);
+  g.kchunk = (int)std::max<long long>((K + splits - 1) / splits, 1);
+  g.nsplit = (int)std::max<long long>((K + g.kchunk - 1) / g.kchunk, 1);
+  g.atomic = g.nsplit > 1 ? 1 : 0;
 }
 
 void Program::add(const View& C, bool acc, const std::vector<Term>& terms) {
