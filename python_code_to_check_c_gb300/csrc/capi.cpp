@@ -1,6 +1,7 @@
 // extern "C" entry points of libtdcc.so (declared in include/tdcc.h).
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -10,6 +11,7 @@
 #include "engine.h"
 #include "gemm_tc.h"
 #include "ground.h"
+#include "phase.h"
 #include "post.h"
 #include "rk4.h"
 
@@ -32,6 +34,8 @@ void build_density(Program& p, int n_mu);
 // Tensor-core backend hooks (gemm_tc.cu); FP64 only when not compiled in.
 bool tc_available();
 
+constexpr int kPhaseBlocks = 152, kPhaseBlocksStep = 76;
+
 struct ProgInst {
   std::unique_ptr<Program> prog;
   std::vector<void*> bases;
@@ -48,6 +52,10 @@ struct ProgInst {
   long long bytes = 0;
   bool setup_done = false;   // integral-only ops (e.g. packed integral blocks) ran
   DagExec dag;               // streams/events for concurrent execution of the ops
+  PhaseKernel phase[5];      // phases that run as one launch (small FP64 programs)
+  void build_phases(std::initializer_list<Program::Phase> phs) {
+    for (Program::Phase ph : phs) phase[ph].build(*prog, ph, owned, bytes);
+  }
   // runs the integral-only ops once, eagerly, on `st`
   cudaError_t setup(cudaStream_t st) {
     if (setup_done) return cudaSuccess;
@@ -76,8 +84,12 @@ struct ProgInst {
     for (int i : used)
       if (!bases[i]) throw std::runtime_error("unbound buffer slot " + prog->slots[i].name + " in " + prog->name);
   }
-  // phase ops as a dependency DAG (serially, in program order, when timed)
-  cudaError_t exec(cudaStream_t st, Program::Phase ph, std::vector<Program::Timed>* timed = nullptr) {
+  // phase ops as one launch where the phase qualifies, else as a dependency
+  // DAG (serially, in program order, when timed).  `blocks`: thread blocks
+  // of the one launch at most (kPhaseBlocks; a quarter of the resident ones
+  // where the four blocks of a step run at once).
+  cudaError_t exec(cudaStream_t st, Program::Phase ph, std::vector<Program::Timed>* timed = nullptr,
+                   int blocks = kPhaseBlocks) {
     check_bound();
     // TDCC_SERIAL=1 issues every op in program order on `st` (debugging aid)
     static const bool serial = [] {
@@ -85,6 +97,11 @@ struct ProgInst {
       return e && e[0] == '1';
     }();
     if (timed || serial) return prog->run(bases, st, ph, timed);
+    if (phase[ph].ok) {
+      const cudaError_t e = phase[ph].launch(bases, blocks, st);
+      if (e != cudaSuccess) set_error("phase launch failed in " + prog->name + ": " + cudaGetErrorString(e));
+      return e;
+    }
     return prog->run_dag(bases, st, ph, dag);
   }
 };
@@ -239,6 +256,9 @@ ProgInst& get_rhs(tdcc_system s, int method, int block) {
   s->ws_bytes += pi->bytes;
   bind_fixed(s, pi->bases);
   pi->dag.init(p.ops.size(), 4);
+  const long long ws0 = pi->bytes;
+  pi->build_phases({Program::PROLOGUE, Program::STAGE, Program::DYNAMIC});
+  s->ws_bytes += pi->bytes - ws0;
   slot = std::move(pi);
   return *slot;
 }
@@ -259,6 +279,9 @@ ProgInst& get_density(tdcc_system s) {
   s->ws_bytes += pi->bytes;
   bind_fixed(s, pi->bases);
   pi->dag.init(pi->prog->ops.size(), 4);
+  const long long ws0 = pi->bytes;
+  pi->build_phases({Program::ALL});
+  s->ws_bytes += pi->bytes - ws0;
   s->dens = std::move(pi);
   return *s->dens;
 }
@@ -299,6 +322,12 @@ ProgInst& get_adj(tdcc_system s, int method, int block) {
   s->ws_bytes += pi->bytes;
   pi->setup_done = true;  // no integral-only ops in a reverse-mode program
   pi->dag.init(pi->prog->ops.size(), 4);
+  const long long ws0 = pi->bytes;
+  if (block == 4)
+    pi->build_phases({Program::ALL});
+  else
+    pi->build_phases({Program::PROLOGUE, Program::STAGE});
+  s->ws_bytes += pi->bytes - ws0;
   if (block < 4) {
     const ActPlan ap = plan_activations(*pi->prog, pi->nfwd, *get_rhs(s, method, block).prog);
     pi->act_slot = ap.slot;
@@ -440,7 +469,7 @@ void run_block(tdcc_system s, int method, int b, double2* const in[4], double2* 
   std::vector<Program::Timed> tm;
   B[S_F] = s->Fs;
   CK(pi.setup(st));
-  CK(pi.exec(st, Program::PROLOGUE, pf ? &tm : nullptr));
+  CK(pi.exec(st, Program::PROLOGUE, pf ? &tm : nullptr, kPhaseBlocksStep));
   if (pf) pf->add_prog(tm, b, 0);
   const ProgInst* act = ss && ss->act[b] ? s->adjp[method][b].get() : nullptr;
   if (act) store_activations(s->ctx, *act, pi, *ss, b, 0, st);
@@ -448,7 +477,7 @@ void run_block(tdcc_system s, int method, int b, double2* const in[4], double2* 
     B[S_T1 + b] = stage == 1 ? in[b] : s->yin[b];
     B[S_F] = s->Fs + (stage == 1 ? 0 : stage < 4 ? 1 : 2) * nn;
     tm.clear();
-    CK(pi.exec(st, Program::STAGE, pf ? &tm : nullptr));
+    CK(pi.exec(st, Program::STAGE, pf ? &tm : nullptr, kPhaseBlocksStep));
     if (pf) pf->add_prog(tm, b, stage);
     if (act) store_activations(s->ctx, *act, pi, *ss, b, stage, st);
     const double h = stage < 3 ? dt / 2.0 : dt;
@@ -944,7 +973,19 @@ int tdcc_check_errors(tdcc_system s) {
   if (ce != cudaSuccess) return fail(TDCC_ERR_CUDA, std::string("device error: ") + cudaGetErrorString(ce));
   for (auto* slot : all_programs(s)) {
     auto& pi = *slot;
-    if (!pi || pi->prog->err_slot < 0) continue;
+    if (!pi) continue;
+    for (const PhaseKernel& k : pi->phase) {
+      int flag = 0;
+      if (!k.ok) continue;
+      if (cudaMemcpy(&flag, k.error_flag(), sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return fail(TDCC_ERR_CUDA, "reading a phase kernel's error flag failed");
+      if (flag) {
+        cudaMemset(k.error_flag(), 0, sizeof(int));
+        return fail(TDCC_ERR_CUDA, "the phase kernel of " + pi->prog->name + " gave up waiting (code " +
+                                       std::to_string(flag) + ")");
+      }
+    }
+    if (pi->prog->err_slot < 0) continue;
     int flag = 0;
     void* p = pi->bases[pi->prog->err_slot];
     if (cudaMemcpy(&flag, p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -1190,11 +1231,11 @@ int tdcc_autotune(tdcc_system s, int method, const void* t1, const void* t2, con
       ProgInst& pi = *pip;
       pi.check_bound();
       for (Op& op : pi.prog->ops) {
-        if (op.kind == OP_GEMM && op.backend == GB_FP64) {
+        if (op.kind == OP_GEMM && op.backend == GB_FP64 && op.dot < 0) {
           const double t_cur = time_op(pi, op);
           double best = t_cur;
           Op best_op = op;
-          for (int tile = 0; tile < kNumTiles; ++tile)
+          for (int tile = 0; tile < 5; ++tile)  // fixed-point tiles
             for (int split = 0; split < 2; ++split) {
               if (!tile_fits(tile, op.dta != C64 && op.dtb != C64)) continue;
               Op c = op;
@@ -1456,14 +1497,14 @@ int tdcc_adjoint(tdcc_system s, int method, const void* t1, const void* t2, cons
         for (int q = 0; q < 4; ++q) B[S_T1 + q] = gy[q];
         B[S_OUT] = s->kbuf[b];
         B[S_F] = gF;
-        if (!use_act) CK(pi.exec(sb, Program::PROLOGUE));
+        if (!use_act) CK(pi.exec(sb, Program::PROLOGUE, nullptr, kPhaseBlocksStep));
         // a_k(s) = c w_s a_out, c = -i dt/6 (T) or +i dt/6 (Lambda)
         const double ci = (b == TDCC_T1 || b == TDCC_T2) ? -c6 : c6;
         for (int st = 0; st < 4; ++st) CK(launch_caxpy(ak[b][st], ay[b], nel(b), 0.0, wst[st] * ci, 0, sb));
         for (int st = 4; st >= 1; --st) {
           B[S_T1 + b] = st == 1 ? gy[b] : gst[b][st - 2];
           B[S_F] = gF + (size_t)(st == 1 ? 0 : st < 4 ? 1 : 2) * nb * nn;
-          if (!use_act) CK(pi.exec(sb, Program::STAGE));
+          if (!use_act) CK(pi.exec(sb, Program::STAGE, nullptr, kPhaseBlocksStep));
           for (size_t i = 0; i < ai.nfwd; ++i) ai.bases[i] = B[i];
           if (use_act)
             for (size_t j = 0; j < ai.act_slot.size(); ++j)
@@ -1479,12 +1520,12 @@ int tdcc_adjoint(tdcc_system s, int method, const void* t1, const void* t2, cons
           }
           for (int q = 0; q < 4; ++q)
             if (q != b && aof[S_T1 + q] >= 0) ai.bases[aof[S_T1 + q]] = contrib[b][q];
-          CK(ai.exec(sb, Program::STAGE));
+          CK(ai.exec(sb, Program::STAGE, nullptr, kPhaseBlocksStep));
           if (aof[S_F] >= 0) CK(launch_field_grad(aF[b], s->mu, s->d_pol, n, nb, gE + b * gEn, rctx, st - 1, sb));
           CK(launch_caxpy(contrib[b][b], aY[b], nel(b), 1.0, 0.0, 1, sb));
           if (st > 1) CK(launch_caxpy(ak[b][st - 2], aY[b], nel(b), hst[st - 1], 0.0, 1, sb));
         }
-        CK(ai.exec(sb, Program::PROLOGUE));
+        CK(ai.exec(sb, Program::PROLOGUE, nullptr, kPhaseBlocksStep));
         CK(cudaEventRecord(s->ev_join[b], sb));
       }
       for (int b = 0; b < 4; ++b) CK(cudaStreamWaitEvent(m, s->ev_join[b], 0));

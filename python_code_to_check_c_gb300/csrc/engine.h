@@ -186,7 +186,8 @@ struct Op {
   int dta = C64, dtb = C64, dtc = C64;
   GemmArgs g{};
   int backend = GB_FP64;
-  int tile = 0;            // FP64 tile shape index (kTiles)
+  int tile = 0;            // FP64 form index (kTiles)
+  int dot = -2;            // FP64 dot products: log2 of the lanes per output (-1: fixed-point tiles, -2: undecided)
   bool zeroed = false;     // C is zeroed (or accumulated into) before: split-K allowed
   long long flops = 0;     // real flops of this contraction
   long long bytes = 0;     // compulsory bytes read + written
@@ -356,13 +357,25 @@ void coalesce(AddArgs& a);
 // op inherits the varying / constant flags of the forward op it reverses.
 void build_adjoint(const Program& f, Program& a, std::vector<int>& adj_of);
 
-// fixed-point contraction of the FP64 form: tile shapes, and the tile and K
-// splits of given extents (gemm_fx.cu; tile >= 0: that one)
-constexpr int kNumTiles = 5;
+// contraction of the FP64 form (fixed-point tiles, dot products): the form and K
+// splits of given extents (gemm_fx.cu; tile >= 0: that one, -1: any tile, -2:
+// the phase kernel's tile, -3: any form)
+constexpr int kNumTiles = 6;
 extern const int kTiles[kNumTiles][2];
 bool tile_fits(int tile, bool real_operands);
 void choose_fx(long long M, long long N, long long K, long long nb, bool ac, bool bc, bool allow_split, int tile,
                int* best_tile, int* best_splits);
+int dot_lanes(long long outputs, long long K);
+
+// how a block walks a contraction (after the operands are put in order)
+struct FxPlan {
+  int tile, mtiles, kc, flags;
+  int p2, e2, neg;    // alpha = +-2^e2
+  int ac, bc, cc;     // complex operands / output
+  int swapped;        // the op's A and B change places
+  long long tiles;    // output tiles (per batch and split)
+};
+cudaError_t fx_plan(const Op& op, GemmArgs& g, FxPlan& f);
 
 // kernel launchers
 cudaError_t launch_gemm(const Op& op, const void* A, const void* B, void* C, cudaStream_t st);

@@ -253,13 +253,25 @@ void Program::ein(const char* spec, double ar, double ai, const View& A, const V
   ops.push_back(op);
 }
 
-// Tile shape and K splits (splits only where the output is zeroed or
-// accumulated into: they add with atomics), from the kernel's cost model.
+// Form and K splits (splits only where the output is zeroed or accumulated
+// into: they add with atomics), from the kernels' cost model.  Dot products or
+// fixed-point tiles is decided once, from the extents the op is first planned
+// with: a batched program then rounds as its single-trajectory one does.
 void Program::plan_gemm(Op& op, bool allow_split, int tile) {
   GemmArgs& g = op.g;
-  const long long K = g.K;
+  const long long K = g.K, nb = std::max(g.nb, 1);
+  const bool ac = op.dta == C64, bc = op.dtb == C64;
   int splits = 1;
-  choose_fx(g.M, g.N, K, std::max(g.nb, 1), op.dta == C64, op.dtb == C64, allow_split, tile, &op.tile, &splits);
+  if (op.dot == -2) {
+    choose_fx(g.M, g.N, K, nb, ac, bc, allow_split, -3, &op.tile, &splits);
+    op.dot = op.tile == 5 ? dot_lanes((long long)g.M * g.N * nb, K) : -1;
+  }
+  if (op.dot >= 0) {
+    op.tile = 5;
+    splits = 1;
+  } else {
+    choose_fx(g.M, g.N, K, nb, ac, bc, allow_split, tile, &op.tile, &splits);
+  }
   g.kchunk = (int)std::max<long long>((K + splits - 1) / splits, 1);
   g.nsplit = (int)std::max<long long>((K + g.kchunk - 1) / g.kchunk, 1);
   g.atomic = g.nsplit > 1 ? 1 : 0;

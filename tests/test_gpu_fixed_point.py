@@ -83,3 +83,47 @@ def test_residuals_at_ragged_sizes(o, v, nb, method):
                 assert rel_err(got[z], getattr(orc, name)(*a, F[z])) < 1e-12, (name, z)
     finally:
         eng.close()
+
+
+def test_small_systems_on_several_threads_and_streams():
+    """The one-launch phases of several engines at a time: each has its own barrier and temporaries."""
+    import threading
+
+    import torch
+
+    from python_code_to_check_c_gb300._lib import make_field
+    from python_code_to_check_c_gb300.engine import CCEngine
+    from python_code_to_check_c_gb300.system import mp2_guess, synthetic_system
+    sizes = [(3, 5), (4, 8), (2, 7), (4, 6)]
+    field, jobs, got, errors = make_field("sin", 0.002, 0.923), [], {}, []
+
+    def work(k):
+        eng, st, stream = jobs[k]
+        with torch.cuda.stream(stream):
+            fin, mu = eng.propagate("CCSD", st, 0.0, 0.01, 40, field)
+            res = [mu] + list(fin) + [eng.rhs("CCSD", b, *st) for b in range(4)]
+            eng.check_errors()
+            return [x.cpu().numpy() for x in res]
+
+    def thread(k):
+        try:
+            got[k] = [work(k) for _ in range(5)]
+        except Exception as ex:  # noqa: BLE001 - reported by the main thread
+            errors.append(ex)
+
+    for k, (o, v) in enumerate(sizes):
+        s = synthetic_system(o, v, 40, seed=9 + k)
+        t1, t2 = np.full((o, v), 0.01 + 0.002j), mp2_guess(s.tei(), s.eps(), o) + 0j
+        jobs.append((CCEngine.from_system(s, device_integrals=False), (t1, t2, t1, t2), torch.cuda.Stream()))
+    want = [work(k) for k in range(len(sizes))]  # builds the programs and captures the steps
+    ts = [threading.Thread(target=thread, args=(k,)) for k in range(len(sizes))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    for k in range(len(sizes)):
+        for run in got[k]:
+            for a, b in zip(want[k], run):
+                assert rel_err(b, a) < 1e-12
+        jobs[k][0].close()
