@@ -52,10 +52,12 @@ enum { TDCC_T1 = 0, TDCC_T2 = 1, TDCC_L1 = 2, TDCC_L2 = 3 };
 
 /* contraction arithmetic */
 enum {
-  TDCC_PREC_FP64 = 0,      /* the plain form: contractions in 56-bit block
-                              fixed point with exact sums, rounded to FP64
-                              once per K chunk of at most 60; FP64 everywhere
-                              else                                         */
+  TDCC_PREC_FP64 = 0,      /* the plain form, FP64 accuracy: small
+                              contractions as FP64 dot products, larger ones
+                              in 56-bit fixed point under each row's maximum
+                              with exact sums (integer pipe, or eight-slice
+                              tensor-core products), rounded to FP64 at the
+                              end; FP64 everywhere else                    */
   TDCC_PREC_MIXED = 1      /* large contractions as split-BF16 tcgen05
                               products, FP64 everywhere else               */
 };

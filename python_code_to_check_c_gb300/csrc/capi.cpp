@@ -223,6 +223,17 @@ void bind_fixed(tdcc_system s, std::vector<void*>& b) {
   b[S_MU] = const_cast<double*>(s->mu);
 }
 
+// bytes the packed operands of one FP64 program may take: a sixth of what is
+// free (a step holds four programs and the density's, reverse mode as many again)
+long long deep_budget() {
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return (long long)(fr / 6);
+}
+
 ProgInst& get_rhs(tdcc_system s, int method, int block) {
   auto& slot = s->rhs[method][block];
   if (slot) return *slot;
@@ -247,7 +258,7 @@ ProgInst& get_rhs(tdcc_system s, int method, int block) {
     build_l2_cc2(p, p.ones("ones_v", s->dims.v));
   p.batch(s->nb);
   p.select_backend(s->prec_mode, s->tc_min_macs, s->slices, s->tc_min_k, s->tc_min_mn, s->simt_max_k,
-                          s->simt_min_macs);
+                          s->simt_min_macs, deep_budget());
   // the block's own amplitude and the dressed Fock vary across RK4 stages
   p.analyse({S_T1 + block, S_F});
   if (s->share_mem && workspace_estimate(p) > (s->share_min < 0 ? kShareMinBytes : s->share_min)) p.plan_memory();
@@ -270,7 +281,7 @@ ProgInst& get_density(tdcc_system s) {
   build_density(*pi->prog, s->n_mu);
   pi->prog->batch(s->nb);
   pi->prog->select_backend(s->prec_mode, s->tc_min_macs, s->slices, s->tc_min_k, s->tc_min_mn, s->simt_max_k,
-                          s->simt_min_macs);
+                          s->simt_min_macs, deep_budget());
   pi->prog->analyse({});
   if (s->share_mem && workspace_estimate(*pi->prog) > (s->share_min < 0 ? kShareMinBytes : s->share_min))
     pi->prog->plan_memory();
@@ -315,7 +326,7 @@ ProgInst& get_adj(tdcc_system s, int method, int block) {
   pi->prog = std::make_unique<Program>(s->dims, "adj");
   build_adjoint(f, *pi->prog, s->adj_of[method][block]);
   pi->prog->select_backend(s->prec_mode, s->tc_min_macs, s->slices, s->tc_min_k, s->tc_min_mn, s->simt_max_k,
-                          s->simt_min_macs);
+                          s->simt_min_macs, deep_budget());
   pi->nfwd = f.slots.size();
   pi->bases.assign(pi->prog->slots.size(), nullptr);
   pi->bytes = pi->prog->allocate(pi->bases, pi->owned, pi->nfwd, true);
@@ -1253,7 +1264,7 @@ int tdcc_autotune(tdcc_system s, int method, const void* t1, const void* t2, con
             op = best_op;
             ++tuned;
           }
-        } else if (op.kind == OP_TCGEMM) {
+        } else if (op.kind == OP_TCGEMM && op.tc.variant != 4) {
           const double t_cur = time_op(pi, op);
           double best = t_cur;
           TcArgs best_a = op.tc;

@@ -154,7 +154,7 @@ struct TcArgs {
   int M, N;                 // logical output extents (per batch)
   int rowsA_pad, rowsB_pad; // packed rows per batch
   int nb, nsplit;           // blockIdx.z = batch * nsplit + split
-  int variant;              // 0: 64-wide tile, one CTA per SM; 1: 32-wide, two per SM; 2: 128-wide; 3: persistent 64-wide
+  int variant;              // 0: 64-wide tile, one CTA per SM; 1: 32-wide, two per SM; 2: 128-wide; 3: persistent 64-wide; 4: deep
   int m_fast;               // launch order: M tiles fastest (set by the launcher)
   int bat_a, bat_b;         // A / B packed per batch (else shared by all batches)
   long long bsC;            // output batch stride in elements
@@ -171,6 +171,11 @@ struct TcArgs {
   int alpha_e, alpha_neg;
   int acc, atomic;
   int* err;
+  // the operands themselves (deep form: rows that digits cannot hold)
+  const void *srcA, *srcB;
+  ModeGroup gmA, gnB, gkAB;  // offsets in s0 (A / B); gkAB: A in s0, B in s1
+  long long bsA, bsB;
+  int K;
 };
 
 // GB_SIMT: exact BF16-digit slice products on the FP32 pipe for short
@@ -214,6 +219,7 @@ struct Op {
   // TCGEMM: packed A / B slots, output C, error-flag slot
   TcArgs tc{};
   int tc_pa = -1, tc_pb = -1, tc_err = -1;
+  int tc_sa = -1, tc_sb = -1;  // deep form: the operands' own slots, offsets and types (oa, ob, dta, dtb)
   long long tc_expa_off = 0, tc_expb_off = 0;
   // dependency analysis
   std::vector<int> reads;
@@ -339,8 +345,10 @@ class Program {
   // tensor-core slice product with `slices` BF16 slices per operand
   // contractions left out with K <= simt_max_k and at least simt_min_macs
   // multiply-adds run as slice products on the FP32 pipe (GB_SIMT)
+  // prec_mode 0 (FP64): the contractions that are faster so become 8-slice
+  // products (deep form), if their packed operands fit in deep_bytes
   void select_backend(int prec_mode, long long min_macs, int slices, int min_k, int min_mn, int simt_max_k,
-                      long long simt_min_macs);
+                      long long simt_min_macs, long long deep_bytes);
   int err_slot = -1;  // U8 slot holding the tensor-core kernels' error flag
 };
 

@@ -51,23 +51,41 @@
 #include "engine.h"
 #include "gemm_tc.h"
 #include "slice_math.cuh"
+#include "tc_ptx.cuh"
 
 namespace tdcc {
 
 // ---------------------------------------------------------------------------
 // packing
 // ---------------------------------------------------------------------------
+// Stored exponent of a row whose largest |x| has bits mx (biased exponent E).
+// The deep form marks rows that digits cannot hold (infinities, NaNs, nothing
+// but subnormals): its drain does their outputs by FP64 dot products.
+template <int SMAX>
+__device__ __forceinline__ int packed_exponent(unsigned long long mx, int E) {
+  if (mx == 0) return 0;
+  if (SMAX > TC_MAX_SLICES && (E == 0 || E == 2047)) return kExpMarked;
+  return (E > 0 ? E - 1022 : -1022) + kExpBias;
+}
+
 // Digits of two neighbouring elements of a packed row (same exponent e), one
 // BF16 pair per slice: out is the packed buffer as BF16 pairs, plane2 the
 // pairs per slice, idx2 the pair's index within a slice.
+// SMAX > TC_MAX_SLICES (the deep form): the last digit is rounded, not cut.
+template <int SMAX>
 __device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, size_t idx2, double x0, double x1,
                                                  int e, int nbits, int S) {
-  int q0[TC_MAX_SLICES], q1[TC_MAX_SLICES];
-  balanced_digits(fixed_point(x0, e, nbits), S, q0);
-  balanced_digits(fixed_point(x1, e, nbits), S, q1);
+  int q0[SMAX], q1[SMAX];
+  if constexpr (SMAX > TC_MAX_SLICES) {
+    balanced_digits(fixed_point_rounded(x0, e, nbits), S, q0);
+    balanced_digits(fixed_point_rounded(x1, e, nbits), S, q1);
+  } else {
+    balanced_digits(fixed_point(x0, e, nbits), S, q0);
+    balanced_digits(fixed_point(x1, e, nbits), S, q1);
+  }
   const bool n0 = __double_as_longlong(x0) < 0, n1 = __double_as_longlong(x1) < 0;  // sign bits
 #pragma unroll
-  for (int s = 0; s < TC_MAX_SLICES; ++s)
+  for (int s = 0; s < SMAX; ++s)
     if (s < S) out[s * plane2 + idx2] = digit_pair_bf16x2(n0 ? -q0[s] : q0[s], n1 ? -q1[s] : q1[s]);
 }
 
@@ -87,6 +105,7 @@ __device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, s
 // With tab set, the K offsets (the same for every row) are decoded once per
 // block into shared memory as 32-bit integers (K of them) and both passes
 // read them there.
+template <int SMAX>
 __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
   extern __shared__ int kofs[];
   const int per = p.cplx ? 2 : 1;
@@ -141,7 +160,7 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
   mx = 0;
   for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx = max(mx, wmax[w]);
   const int E = (int)(mx >> 52);
-  const int eb = mx != 0 ? (E > 0 ? E - 1022 : -1022) + kExpBias : 0;
+  const int eb = packed_exponent<SMAX>(mx, E);
   const size_t prow = (size_t)z * p.rows_pad + (size_t)m * per;  // first packed row
   if (threadIdx.x == 0) {
     p.exps[prow] = eb;
@@ -178,7 +197,7 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
       const int k = k0 + 2 * j * blockDim.x;
       if (k >= p.K_pad) break;
       for (int part = 0; part < per; ++part)
-        store_digit_pair(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, nbits,
+        store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, nbits,
                          p.S);
     }
   }
@@ -190,7 +209,7 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
 // once: the exponent comes from shuffles (and shared memory across the W
 // warps), the digits from the registers (same exponent, digits and layout as
 // pack_kernel).
-template <int KP, int W>
+template <int KP, int W, int SMAX>
 __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
   static_assert(W == 1 || W == 2 || W == 4 || W == 8, "warps per row divide the block");
   constexpr int RPB = 8 / W;
@@ -239,7 +258,7 @@ __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
   }
   if (!live) return;
   const int E = (int)(mx >> 52);
-  const int eb = mx != 0 ? (E > 0 ? E - 1022 : -1022) + kExpBias : 0;
+  const int eb = packed_exponent<SMAX>(mx, E);
   const size_t prow = (size_t)z * p.rows_pad + (size_t)m * per;
   if (wr == 0 && lane == 0) {
     p.exps[prow] = eb;
@@ -254,110 +273,13 @@ __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
     const int k = 2 * (32 * wr + lane + 32 * W * j);
     if (k >= p.K_pad) break;
     for (int part = 0; part < per; ++part)
-      store_digit_pair(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, nbits, p.S);
+      store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, nbits, p.S);
   }
-}
-
-// ---------------------------------------------------------------------------
-// PTX wrappers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint32_t a, uint32_t c) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(c));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t a) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(a), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait: false after `limit` polls (each poll may suspend briefly)
-__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, int limit) {
-  for (int i = 0; i < limit; ++i)
-    if (mbar_try(a, parity)) return true;
-  return false;
-}
-__device__ __forceinline__ void tma3d(uint32_t dst, const CUtensorMap* tm, int x, int y, int z, uint32_t mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-          dst),
-      "l"((uint64_t)tm), "r"(x), "r"(y), "r"(z), "r"(mbar)
-      : "memory");
-}
-// UMMA shared-memory descriptor: K-major, SWIZZLE_128B, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// instruction descriptor: kind::f16, A = B = BF16, D = F32, both K-major
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-__device__ __forceinline__ void umma(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
-      "l"(a), "l"(b), "r"(id), "r"(acc));
-}
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16u(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;");
-}
-// issue only: the caller waits (tcgen05.wait::ld) before reading r
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st16u(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 // ---------------------------------------------------------------------------
 // slice-product kernel
 // ---------------------------------------------------------------------------
-constexpr int kWaitLimit = 1 << 22;
-
 template <class C>
 struct TcShared {
   uint64_t full[C::STAGES];
@@ -368,12 +290,6 @@ struct TcShared {
   long long col_off[C::BN];  // output offset of each logical column of the tile (-1: outside)
   int col_exp[C::BN];        // exponent of each packed column of B
 };
-
-template <class SH>
-__device__ __forceinline__ void fail(SH* sh, int* err, int code) {
-  sh->abort = 1;
-  atomicCAS(err, 0, code);
-}
 
 template <bool AC, bool BC, class C>
 __global__ void __launch_bounds__(C::THREADS, C::MINB)
@@ -1649,7 +1565,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 // [S][rows_pad][K_pad] BF16, box = (64 K, box_rows rows, 1 slice).
 // Encoded maps are cached by (address, layout): a packed buffer keeps its
 // address for the life of its program.
-static CUtensorMap slice_map(const void* base, int S, int rows_pad, int K_pad, int box_rows) {
+CUtensorMap slice_map(const void* base, int S, int rows_pad, int K_pad, int box_rows) {
   static std::mutex mu;
   static std::map<std::tuple<const void*, int, int, int, int>, CUtensorMap> cache;
   const auto key = std::make_tuple(base, S, rows_pad, K_pad, box_rows);
@@ -1672,12 +1588,8 @@ static CUtensorMap slice_map(const void* base, int S, int rows_pad, int K_pad, i
   return m;
 }
 
-cudaError_t launch_pack(const PackArgs& p, cudaStream_t st) {
-  if (p.nb < 1 || p.rows < 1 || p.rows_pad % (p.cplx ? 2 : 1) != 0 || p.rows * (p.cplx ? 2 : 1) > p.rows_pad ||
-      p.K_pad % 2 != 0 || p.K > p.K_pad)
-    return cudaErrorInvalidValue;
-  const long long blocks = (long long)p.nb * p.rows;
-  if (blocks > 0x7FFFFFFFLL) return cudaErrorInvalidConfiguration;
+template <int SMAX>
+static cudaError_t launch_pack_slices(const PackArgs& p, long long blocks, cudaStream_t st) {
   if (p.K_pad <= 2048) {
     // rows held in registers, read once: up to 256 elements per warp (8 per
     // lane), up to eight warps per row
@@ -1685,17 +1597,17 @@ cudaError_t launch_pack(const PackArgs& p, cudaStream_t st) {
       kern<<<(unsigned)((blocks + rows_per_block - 1) / rows_per_block), 256, 0, st>>>(p);
     };
     if (p.K_pad <= 64)
-      go(pack_rows_regs_kernel<1, 1>, 8);
+      go(pack_rows_regs_kernel<1, 1, SMAX>, 8);
     else if (p.K_pad <= 128)
-      go(pack_rows_regs_kernel<2, 1>, 8);
+      go(pack_rows_regs_kernel<2, 1, SMAX>, 8);
     else if (p.K_pad <= 256)
-      go(pack_rows_regs_kernel<4, 1>, 8);
+      go(pack_rows_regs_kernel<4, 1, SMAX>, 8);
     else if (p.K_pad <= 512)
-      go(pack_rows_regs_kernel<4, 2>, 4);
+      go(pack_rows_regs_kernel<4, 2, SMAX>, 4);
     else if (p.K_pad <= 1024)
-      go(pack_rows_regs_kernel<4, 4>, 2);
+      go(pack_rows_regs_kernel<4, 4, SMAX>, 2);
     else
-      go(pack_rows_regs_kernel<4, 8>, 1);
+      go(pack_rows_regs_kernel<4, 8, SMAX>, 1);
   } else {
     // long rows: a block per row; few long rows (the K = o v^2 operands)
     // take more threads per row so that the SMs still fill
@@ -1708,17 +1620,27 @@ cudaError_t launch_pack(const PackArgs& p, cudaStream_t st) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
     std::call_once(once[dev], [dev] {
-      attr_err[dev] = cudaFuncSetAttribute(pack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      attr_err[dev] = cudaFuncSetAttribute(pack_kernel<SMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            kTabMax * (int)sizeof(int));
     });
     long long span = 0;  // largest K offset
     for (int q = 0; q < p.gk.n && q < kMaxModes; ++q) span += (long long)(p.gk.dim[q] - 1) * std::llabs(p.gk.s0[q]);
     const int tab = (attr_err[dev] == cudaSuccess && p.K <= kTabMax && span < (1LL << 31)) ? 1 : 0;
     const size_t smem = tab ? (size_t)p.K * sizeof(int) : 0;
-    pack_kernel<<<(unsigned)blocks, threads, smem, st>>>(p, tab);
+    pack_kernel<SMAX><<<(unsigned)blocks, threads, smem, st>>>(p, tab);
   }
   count_launch();
   return cudaGetLastError();
+}
+
+cudaError_t launch_pack(const PackArgs& p, cudaStream_t st) {
+  if (p.nb < 1 || p.rows < 1 || p.rows_pad % (p.cplx ? 2 : 1) != 0 || p.rows * (p.cplx ? 2 : 1) > p.rows_pad ||
+      p.K_pad % 2 != 0 || p.K > p.K_pad)
+    return cudaErrorInvalidValue;
+  const long long blocks = (long long)p.nb * p.rows;
+  if (blocks > 0x7FFFFFFFLL) return cudaErrorInvalidConfiguration;
+  return p.S > TC_MAX_SLICES ? launch_pack_slices<TC_DEEP_SLICES>(p, blocks, st)
+                             : launch_pack_slices<TC_MAX_SLICES>(p, blocks, st);
 }
 
 template <class C>
@@ -1874,6 +1796,7 @@ static cudaError_t launch_persist(const TcArgs& a0, const void* packA, const voi
 
 cudaError_t launch_ozaki(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st) {
   if (a.nb < 1 || a.nsplit < 1 || (long long)a.nsplit * a.kb_per_split < a.kblocks) return cudaErrorInvalidValue;
+  if (a.variant == 4) return launch_deep(a, packA, packB, st);
   if (a.variant == 3) return launch_persist(a, packA, packB, st);
   if (a.variant == 2) return launch_tile128(a, packA, packB, st);
   return a.variant == 1 ? launch_variant<TcNarrow>(a, packA, packB, st) : launch_variant<TcWide>(a, packA, packB, st);

@@ -14,6 +14,7 @@ constexpr int TC_BK = 64;                    // K per TMA box (128 B of BF16)
 constexpr int TC_CHUNK_KB = 8;               // 512-wide K chunks (exact FP32 level sums)
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;
 constexpr int TC_MAX_SLICES = 6;
+constexpr int TC_DEEP_SLICES = 8;            // the FP64 form's tensor-core contractions
 
 // Kernel variants: tile width BN (UMMA N), ring depth, TMEM-drain warps and
 // CTAs per SM.  The ring must hold the S slices of one K block (STAGES >= S).
@@ -66,5 +67,20 @@ struct TcPersist {
 constexpr int tc_chunk_kblocks(int S) {
   return S <= 2 ? 16 : S == 3 ? (1 << 24) / (20480 * 64) : (1 << 24) / (24576 * 64);
 }
+
+// Deep form (gemm_deep.cu): 8 slices, 56 bits, 128 x 64 tile, the 8 level
+// accumulators of 64 columns filling TMEM; a ring of (A, B) slice pairs; int64
+// sums in the drain warps' registers across K chunks of at most 6 K blocks (a
+// level grows by at most 2 x 128 x 64 + 6 x 64 x 64 = 40960 per K index and
+// must stay within 2^24).
+struct TcDeep {
+  static constexpr int BN = 64, STAGES = 9, EPI = 16;
+  static constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
+  static constexpr int THREADS = 64 + 32 * EPI;
+  static constexpr int SMEM = 1024 + STAGES * (A_BYTES + B_BYTES) + 2560;
+  static constexpr int CHUNK_KB = (1 << 24) / (40960 * TC_BK);
+};
+
+cudaError_t launch_deep(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st);
 
 }  // namespace tdcc

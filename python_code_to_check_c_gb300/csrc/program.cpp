@@ -14,6 +14,8 @@
 
 namespace tdcc {
 
+static long long rup(long long x, long long m) { return (x + m - 1) / m * m; }
+
 Program::Program(Dims d, std::string nm) : dims(d), name(std::move(nm)) {
   const long long n = d.n, o = d.o, v = d.v;
   slots.resize(kNumFixedSlots);
@@ -753,6 +755,10 @@ cudaError_t Program::launch_op(const Op& op, const std::vector<void*>& bases, cu
     a.expB = reinterpret_cast<const int*>(pb + op.tc_expb_off);
     a.C = const_cast<void*>(at(bases, op.sc, op.oc, op.dtc));
     a.err = static_cast<int*>(bases[op.tc_err]);
+    if (op.tc_sa >= 0) {
+      a.srcA = at(bases, op.tc_sa, op.oa, op.dta);
+      a.srcB = at(bases, op.tc_sb, op.ob, op.dtb);
+    }
     e = launch_ozaki(a, pa, pb, st);
   }
   if (e != cudaSuccess) set_error("kernel launch failed in " + op.tag + ": " + cudaGetErrorString(e));
@@ -875,7 +881,6 @@ cudaError_t Program::run_dag(const std::vector<void*>& bases, cudaStream_t st, P
   return cudaSuccess;
 }
 
-static long long rup(long long x, long long m) { return (x + m - 1) / m * m; }
 
 // Merges neighbouring modes of a packing traversal whose strides (s0) make
 // them one run (s0[q] == dim[q+1] * s0[q+1]): the flat index maps to the
@@ -902,10 +907,58 @@ static void merge_pack_modes(ModeGroup& g) {
   g = m;
 }
 
+// K splits of a contraction of the FP64 form on the tensor cores (deep form),
+// 0 where the integer pipe is expected to be faster.  Model, in microseconds:
+// the fixed-point tiles reach 4.3 real multiply-adds per clock and SM; a deep
+// tile takes 6.5 per K block and 13 for its first loads and its drain, one per
+// SM; packing an operand that is not an integral block 3 and its traffic at 3
+// TB/s.  Measured at o=10, v=38: the ladder (1444 x 200 x 1444 real) 320 us
+// on the integer pipe, 75 deep.
+static int deep_splits(const Op& op) {
+  constexpr int BM = 128, BN = 64, BK = 64, kMinK = 32;
+  const GemmArgs& g = op.g;
+  const double K = g.K, nb = std::max(g.nb, 1);
+  const bool ac = op.dta == C64, bc = op.dtb == C64;
+  if (g.K < kMinK || (op.dtc != C64 && (ac || bc))) return 0;
+  const double ra = (double)g.M * (ac ? 2 : 1), rb = (double)g.N * (bc ? 2 : 1);
+  const double fx = 6.0 + ra * rb * K * nb / (152.0 * 4.3 * 2070.0);
+  const long long tiles = (long long)(std::ceil(ra / BM) * std::ceil(rb / BN) * nb), kb = (g.K + BK - 1) / BK;
+  double best = 1e300;
+  int splits = 0;
+  for (long long sp = 1; sp <= std::min<long long>(kb, 64); ++sp) {
+    const double per = (double)((kb + sp - 1) / sp);
+    const double t = std::ceil((double)(tiles * sp) / 152.0) * (per * 6.5 + 13.0) + (sp > 1 ? 2.0 : 0.0);
+    if (t < best * 0.999) {
+      best = t;
+      splits = (int)sp;
+    }
+  }
+  double deep = best + 4.0;
+  auto pack = [&](int slot, double rows, int dt) {
+    if (slot != S_TEI) deep += 3.0 + rows * K * ((double)elem_bytes(dt) + 2.0 * TC_DEEP_SLICES * (dt == C64 ? 2 : 1)) / 3e6;
+  };
+  pack(op.sa, (double)g.M * (g.bsA ? nb : 1), op.dta);
+  pack(op.sb, (double)g.N * (g.bsB ? nb : 1), op.dtb);
+  return deep < 0.85 * fx ? splits : 0;
+}
+
 void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k, int min_mn, int simt_max_k,
-                             long long simt_min_macs) {
-  if (prec_mode != 1) return;
-  if (S < 1 || S > 6) throw std::runtime_error("slices must be 1..6");
+                             long long simt_min_macs, long long deep_bytes) {
+  const bool deep = prec_mode == 0;
+  if (deep) {
+    S = TC_DEEP_SLICES;
+    // all of them or none: the packed operands have to fit
+    double need = 0.0;
+    for (const auto& op : ops)
+      if (op.kind == OP_GEMM && deep_splits(op) > 0) {
+        const double nb = std::max(op.g.nb, 1), kp = (double)rup(op.g.K, 64) * 2.0 * S;
+        need += kp * ((double)rup(op.g.M * (op.dta == C64 ? 2LL : 1LL), 128) * (op.g.bsA ? nb : 1.0) +
+                      (double)rup(op.g.N * (op.dtb == C64 ? 2LL : 1LL), 64) * (op.g.bsB ? nb : 1.0));
+      }
+    if (need == 0.0 || need > (double)deep_bytes) return;
+  } else if (S < 1 || S > 6) {
+    throw std::runtime_error("slices must be 1..6");
+  }
   constexpr int BM = 128, BN = 64, BK = 64;  // tensor-core tile (gemm_tc.h)
   std::vector<Op> out;
   out.reserve(ops.size() * 2);
@@ -938,7 +991,12 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
       continue;
     }
     const long long M = op.g.M, N = op.g.N, K = op.g.K;
-    if (M * N * K * std::max(op.g.nb, 1) < min_macs || K < min_k || std::min(M, N) < min_mn) {
+    const int dsplits = deep ? deep_splits(op) : 0;
+    if (deep && dsplits == 0) {
+      push_op(op);
+      continue;
+    }
+    if (!deep && (M * N * K * std::max(op.g.nb, 1) < min_macs || K < min_k || std::min(M, N) < min_mn)) {
       // short contractions: slice products on the FP32 pipe (the FP64 pipe
       // is the one the elementwise ops and the update need)
       const bool types_ok = op.dtc == C64 || (op.dta != C64 && op.dtb != C64);
@@ -1085,7 +1143,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     a.kblocks = (int)(Kp / BK);
     a.S = S;
     int cols = 32;
-    while (cols < (S + 2) * BN) cols *= 2;  // S level accumulators + int64 partial sums
+    while (cols < (deep ? S : S + 2) * BN) cols *= 2;  // S level accumulators (+ int64 partial sums)
     if (cols > 512) throw std::runtime_error("tensor-core tile needs more than 512 TMEM columns");
     a.tmem_cols = cols;
     a.ac = ac;
@@ -1134,15 +1192,32 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
         }
       }
     }
+    if (deep) splits = dsplits;
     a.kb_per_split = (int)((a.kblocks + splits - 1) / splits);
     splits = (a.kblocks + a.kb_per_split - 1) / a.kb_per_split;
     a.nsplit = (int)splits;
     a.atomic = splits > 1 ? 1 : 0;
     t.zeroed = a.acc || a.atomic;  // split K is allowed (a zero op precedes when not accumulating)
     // short K: the narrow variant (two CTAs per SM overlap their latencies)
-    a.variant = persist ? 3 : tile128 ? 2 : (a.kb_per_split == 1 && S <= 5) ? 1 : 0;
+    a.variant = deep ? 4 : persist ? 3 : tile128 ? 2 : (a.kb_per_split == 1 && S <= 5) ? 1 : 0;
     t.bytes = (long long)S * (nbA * rA + nbB * rB) * Kp * 2 + nbt * M * N * elem_bytes(op.dtc);
     t.reads = {pa.pk_dst, pb.pk_dst};
+    if (deep) {  // the drain reads the operands of rows that digits cannot hold
+      t.tc_sa = op.sa;
+      t.tc_sb = op.sb;
+      t.oa = op.oa;
+      t.ob = op.ob;
+      t.dta = op.dta;
+      t.dtb = op.dtb;
+      t.reads.push_back(op.sa);
+      t.reads.push_back(op.sb);
+      a.gmA = op.g.gm;
+      a.gnB = op.g.gn;
+      a.gkAB = op.g.gk;
+      a.bsA = op.g.bsA;
+      a.bsB = op.g.bsB;
+      a.K = (int)K;
+    }
     if (a.acc || a.atomic) t.reads.push_back(op.sc);
     t.write = op.sc;
     for (Op* pk : {&pa, &pb}) {

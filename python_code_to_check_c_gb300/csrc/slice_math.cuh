@@ -32,6 +32,7 @@ __device__ __forceinline__ void decomp_tc(const ModeGroup& g, int l, long long& 
 // Row exponents are stored biased (e + kExpBias; 0 = all-zero row) so that
 // zero-initialised memory and atomicMax give the maximum directly.
 constexpr int kExpBias = 4096;
+constexpr int kExpMarked = 1 << 30;  // a row that digits cannot hold (deep form)
 __device__ __forceinline__ int row_exp(int biased) { return biased > 0 ? biased - kExpBias : 0; }
 
 // floor(|x| 2^(nbits - e)) as an integer, from the bits of x (exact; no FP64
@@ -47,7 +48,19 @@ __device__ __forceinline__ unsigned long long fixed_point(double x, int e, int n
   return M >> (-sh);
 }
 
-// The digits of f < 2^(7S) in balanced form, least significant first:
+// The same rounded to nearest (ties away), at most 2^nbits.
+__device__ __forceinline__ unsigned long long fixed_point_rounded(double x, int e, int nbits) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  const int E = (int)(u >> 52);
+  if (E == 0) return 0ull;
+  const unsigned long long M = (u & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+  const int sh = E - 1075 - e + nbits;
+  if (sh >= 0) return M << sh;
+  if (sh < -54) return 0ull;
+  return ((M >> (-sh - 1)) + 1ull) >> 1;
+}
+
+// The digits of f <= 2^(7S) in balanced form, least significant first:
 // every digit below the top one in [-64, 63] (a digit >= 64 becomes d - 128
 // with a carry into the next), the top one in [0, 128].  The value is f
 // itself, sum_s q[s] 2^(7(S-1-s)), and products of digits stay within 2^14.
