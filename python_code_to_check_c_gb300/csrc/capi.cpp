@@ -1264,14 +1264,15 @@ int tdcc_autotune(tdcc_system s, int method, const void* t1, const void* t2, con
             op = best_op;
             ++tuned;
           }
-        } else if (op.kind == OP_TCGEMM && op.tc.variant != 4) {
+        } else if (op.kind == OP_TCGEMM && op.tc.S <= TC_MAX_SLICES) {
           const double t_cur = time_op(pi, op);
           double best = t_cur;
           TcArgs best_a = op.tc;
-          for (int variant = 0; variant < 4; ++variant) {
+          for (int variant = 0; variant < 5; ++variant) {
             if (variant == 1 && op.tc.S > TcNarrow::STAGES) continue;
             if (variant == 2 && (op.tc.S > TC_TILE128_MAX_S || op.tc.rowsB_pad % TcTile128::BN != 0)) continue;
             if (variant == 3 && op.tc.S > TC_TILE128_MAX_S) continue;
+            if (variant == 4 && op.tc.S != 4 && op.tc.S != 5) continue;
             for (int sp : {0, 1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {  // 0: the current split
               Op c = op;
               c.tc.variant = variant;

@@ -1,28 +1,35 @@
-// Contractions of the FP64 form on the tensor cores: exact BF16 slice products
-// (as gemm_tc.cu) with 8 slices of 7 bits a side, 56 bits under each row's
-// maximum, the last one rounded.
+// Exact BF16 slice products on tcgen05 with the sums over all of K in the drain
+// warps' registers: the FP64 form's contractions (8 slices of 7 bits a side,
+// 56 bits under each row's maximum, the last digit rounded) and the mixed
+// form's with 4 or 5 slices and K beyond what the persistent form takes.
 //
-// The 36 products A_s B_t with s + t <= 9 go to the accumulators of their
-// levels L = s + t, FP32 sums of integers that stay exact over a K chunk of 6
-// K blocks.  The 8 levels of a 128 x 64 tile fill TMEM, so the drain warps
-// keep the sums over all chunks in registers: two int64 per output, levels
-// 2..5 and 6..9, rounded to FP64 once at the end.  What is dropped (levels
-// above 9, the operands' rounding) is about 2^-58 of the product of the two
-// row maxima per term and of either sign.  Against extended precision the
-// four residuals at o=8, v=26 (amplitudes near an MP2 guess or normal) are off
-// by 0.61 to 1.02 times what FP64 multiply-add chains gave.
+// The products A_s B_t with s + t <= S + 1 go to the accumulators of their
+// levels L = s + t, FP32 sums of integers that stay exact over a K chunk
+// (TcDeep::CHUNK_KB).  The S levels of a 128 x BN tile fill TMEM (BN = 128, 96,
+// 64 for S = 4, 5, 8); after every chunk the drain warps add them to int64
+// sums (two per output for S = 8, levels 2..5 and 6..9), which are rounded to
+// FP64 once at the end.  With 8 slices what is dropped (levels above 9, the
+// operands' rounding) is about 2^-58 of the product of the two row maxima per
+// term and of either sign: against extended precision the four residuals at
+// o=8, v=26 (amplitudes near an MP2 guess or normal) are off by 0.61 to 1.02
+// times what FP64 multiply-add chains gave.
 //
-// Order of a K block: the slices arrive in pairs (A_j, B_j), j = 1..8, and
-// step j runs the products that pair j completes, (j, t <= min(j, 9 - j)) and
-// (s < j, j) with s <= 9 - j, so the tensor pipe starts with the first pair;
-// pairs j and 9 - j have their last use in step j >= 5.  Bound: shared memory.
-// A K block's 144 MMAs read their operands in 48 clocks each (6.9 k), its 192
-// KB arrive by TMA at 32 bytes a clock (6.1 k), and the two add up: 13.3 k
-// clocks (6.4 us) measured, of which the MMA queue is busy 10.2 k; then 13 us
-// of drain.  The 64-column tile is what 8 levels leave room for in TMEM.
+// Order of a K block: the slices arrive in pairs (A_j, B_j), j = 1..S, and
+// step j runs the products that pair j completes, (j, t <= min(j, S + 1 - j))
+// and (s < j, j) with s <= S + 1 - j, so the tensor pipe starts with the first
+// pair; a pair is released after its last product.  Bound: shared memory.  A K
+// block's MMAs read their operands at 128 bytes a clock (S = 8: 144 of 48
+// clocks, 6.9 k), its slices arrive by TMA at 32 (192 KB, 6.1 k), and the two
+// add up: 13.3 k clocks measured.  So the wider the tile the better (per
+// output column and K block 52, 82 and 204 clocks for S = 4, 5, 8).  Measured:
+// the 24-trajectory ladder at o=10, v=38 (S = 4, 1444 x 4800 x 1444 real) 210
+// us, 335 as single-chunk 128-column tiles over split K (TcTile128); the ladder
+// at o=18, v=82 (S = 5, 6724 x 648 x 6724 real) 829 us, 1842 as 64-column tiles
+// with int64 partial sums in TMEM (TcWide).
 //
 // A row whose maximum is not finite (or that holds subnormals only) is marked
-// by the packing; its outputs are done by FP64 dot products over the operands.
+// by the packing with 8 slices; its outputs are done by FP64 dot products over
+// the operands.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -41,13 +48,14 @@ CUtensorMap slice_map(const void* base, int S, int rows_pad, int K_pad, int box_
 
 namespace {
 
+template <class C>
 struct DeepShared {
-  uint64_t full[TcDeep::STAGES], empty[TcDeep::STAGES];
+  uint64_t full[C::STAGES], empty[C::STAGES];
   uint64_t accfull, accempty, done;
   uint32_t tmem;
   volatile int abort;
-  long long col_off[TcDeep::BN];  // output offset of each logical column (-1: outside)
-  int col_exp[TcDeep::BN];        // stored exponent of each packed column of B
+  long long col_off[C::BN];  // output offset of each logical column (-1: outside)
+  int col_exp[C::BN];        // stored exponent of each packed column of B
 };
 
 // sum over k in [k0, k1) of A[m, k] B[k, n] of batch z, operands as they are
@@ -75,17 +83,16 @@ __device__ __noinline__ double2 direct_dot(const TcArgs& g, int m, int n, int z,
   return s;
 }
 
-template <bool AC, bool BC>
-__global__ void __launch_bounds__(TcDeep::THREADS, 1)
+template <class C, bool AC, bool BC>
+__global__ void __launch_bounds__(C::THREADS, 1)
     ozaki_deep_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ TcArgs g) {
-  using C = TcDeep;
-  constexpr int S = TC_DEEP_SLICES;
+  constexpr int S = C::S;
   extern __shared__ uint8_t smraw[];
   uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
   uint8_t* stA = sm;                                // STAGES x 16 KB
-  uint8_t* stB = sm + C::STAGES * C::A_BYTES;       // STAGES x 8 KB
-  DeepShared* sh = (DeepShared*)(stB + C::STAGES * C::B_BYTES);
+  uint8_t* stB = sm + C::STAGES * C::A_BYTES;       // STAGES x BN x 128 B
+  DeepShared<C>* sh = (DeepShared<C>*)(stB + C::STAGES * C::B_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -171,7 +178,7 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
           if (ok) {
             auto product = [&](int s, int t) {
               // the first product of each level in a chunk starts its sum
-              const bool lead = (s == t || s == t + 1) && s <= 5;
+              const bool lead = s == t || s == t + 1;
 #pragma unroll
               for (int k = 0; k < TC_BK / 16; ++k)
                 umma_warp(tmem + (uint32_t)((s + t - 2) * C::BN), hi64 | (uint64_t)(la[s - 1] + 2 * k),
@@ -184,9 +191,9 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
 #pragma unroll
             for (int q = 1; q <= S; ++q)
               if (q < j && q <= last) product(q, j);
-            if (j > S / 2) {  // pairs j and S + 1 - j have had their last use
+            if (j >= last) {  // pairs j and S + 1 - j have had their last use
               umma_commit_warp(empty0 + 8 * slot[j - 1], on);
-              umma_commit_warp(empty0 + 8 * slot[last - 1], on);
+              if (j > last) umma_commit_warp(empty0 + 8 * slot[last - 1], on);
             }
           }
         }
@@ -204,8 +211,9 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
     umma_commit_warp(smem_u32(&sh->done), on);
     mbar_wait(smem_u32(&sh->done), 0, kWaitLimit);
   } else {
-    // ---------------- drain warps (2 .. 17): 16 packed columns each ----------------
-    const int q = warp & 3, j0 = ((warp - 2) >> 2) * 16;
+    // ---------------- drain warps (2 .. 17): NC packed columns each ----------------
+    constexpr int NC = C::BN / (C::EPI / 4), HL = S > 5 ? 2 : 1;
+    const int q = warp & 3, j0 = ((warp - 2) >> 2) * NC;
     const int row = q * 32 + lane;
     {
       const int t = threadIdx.x - 64;
@@ -216,13 +224,19 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
         if (n < g.N) decomp_tc(g.gnC, n, o);
         sh->col_off[t] = o;
       }
-      if (t < C::BN) sh->col_exp[t] = g.expB[rowB0 + nt * C::BN + t];
+      // the last tile may reach beyond the packed rows (its loads read zeros
+      // or the next batch there; those columns are not stored)
+      if (t < C::BN) sh->col_exp[t] = nt * C::BN + t < g.rowsB_pad ? g.expB[rowB0 + nt * C::BN + t] : 0;
       asm volatile("bar.sync 1, %0;" ::"n"(32 * C::EPI) : "memory");
     }
     const uint32_t tl = (uint32_t)(q * 32) << 16;
-    long long hi[16], lo[16];  // levels 2..5 in units of 2^-35, 6..9 in units of 2^-63
+    // exact sums in units of 2^-u: all levels (u = 7 (S + 1)), or with S = 8
+    // levels 2..5 (u = 35) and 6..9 (u = 63)
+    long long acc[HL][NC];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) hi[j] = lo[j] = 0;
+    for (int h = 0; h < HL; ++h)
+#pragma unroll
+      for (int j = 0; j < NC; ++j) acc[h][j] = 0;
     bool ok = true;
     for (int c = 0; c < nchunks; ++c) {
       if (__any_sync(0xffffffffu, sh->abort != 0)) {
@@ -236,20 +250,22 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
+      constexpr int SL = S / HL;  // levels per sum
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < HL; ++h)
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          uint32_t v0[16], v1[16];  // levels 2 + 4 h + 2 p and the next
-          tmem_ld16_nowait(tmem + tl + (uint32_t)((4 * h + 2 * p) * C::BN + j0), v0);
-          tmem_ld16_nowait(tmem + tl + (uint32_t)((4 * h + 2 * p + 1) * C::BN + j0), v1);
+        for (int w = 0; w < NC; w += 8) {
+          uint32_t v[SL][8];
+#pragma unroll
+          for (int p = 0; p < SL; ++p) tmem_ld8_nowait(tmem + tl + (uint32_t)((SL * h + p) * C::BN + j0 + w), v[p]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            // |v| <= 2^24: exact in 32 bits; two levels join in 64
-            const long long x = ((long long)__float2int_rn(__uint_as_float(v0[j])) << 7) +
-                                (long long)__float2int_rn(__uint_as_float(v1[j]));
-            (h ? lo : hi)[j] += p ? x : x << 14;
+          for (int j = 0; j < 8; ++j) {
+            // |v| <= 2^24: exact in 32 bits, Horner in 64
+            long long x = (long long)__float2int_rn(__uint_as_float(v[0][j]));
+#pragma unroll
+            for (int p = 1; p < SL; ++p) x = (x << 7) + (long long)__float2int_rn(__uint_as_float(v[p][j]));
+            acc[h][w + j] += x;
           }
         }
       asm volatile("tcgen05.fence::before_thread_sync;");
@@ -258,16 +274,18 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
     if (ok && __any_sync(0xffffffffu, sh->abort != 0)) ok = false;
     if (ok) {
       const bool odd = AC && (lane & 1);
-      constexpr int NJ = BC ? 8 : 16;          // logical columns of this warp
-      constexpr int rows_out = AC ? 16 : 32;    // logical rows
-      constexpr int RS = NJ + 1;
+      constexpr int GC = NC > 24 ? NC / 2 : NC;  // packed columns staged at a time
+      constexpr int NL = BC ? GC / 2 : GC;       // logical columns of them
+      constexpr int rows_out = AC ? 16 : 32;     // logical rows
+      constexpr int RS = NL + 1;
+      static_assert(C::EPI * 32 * RS * 16 <= C::STAGES * (C::A_BYTES + C::B_BYTES), "staging fits the ring");
       double2* stage = reinterpret_cast<double2*>(sm) + (size_t)(warp - 2) * (32 * RS);  // the ring is idle
       const int lr = AC ? (lane >> 1) : lane;
       const int prow = mt * TC_BM + row;
       const int m = AC ? (prow >> 1) : prow;
       const int ea = prow < g.rowsA_pad ? g.expA[rowA0 + prow] : 0;
       const bool neg = g.alpha_pow2 && g.alpha_neg;
-      const int ebase = row_exp(ea) - 63 + (g.alpha_pow2 ? g.alpha_e : 0);
+      const int ebase = row_exp(ea) - 7 * (S + 1) + (g.alpha_pow2 ? g.alpha_e : 0);
       long long coffm = 0;
       if (m < g.M) decomp_tc(g.gmC, m, coffm);
       double2* Cc = static_cast<double2*>(g.C) + (g.cc ? zb * g.bsC : 0);
@@ -276,79 +294,83 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
       const int nrows = min(rows_out, g.M - m0w);
       const bool red = g.acc || g.atomic;
 #pragma unroll
-      for (int k = 0; k < NJ; ++k) {
-        const int jj = (BC ? j0 / 2 : j0) + k;
-        long long rh, rl, ih = 0, il = 0;  // real and imaginary part, high and low sum
-        if constexpr (BC) {
-          const long long h0 = hi[2 * k], h1 = hi[2 * k + 1], l0 = lo[2 * k], l1 = lo[2 * k + 1];
-          if constexpr (AC) {
-            const long long p0 = __shfl_xor_sync(0xffffffffu, h0, 1), p1 = __shfl_xor_sync(0xffffffffu, h1, 1);
-            const long long s0 = __shfl_xor_sync(0xffffffffu, l0, 1), s1 = __shfl_xor_sync(0xffffffffu, l1, 1);
-            // even lane: (re re, re im) own, (im re, im im) the partner's
-            rh = odd ? p0 - h1 : h0 - p1;
-            ih = odd ? p1 + h0 : h1 + p0;
-            rl = odd ? s0 - l1 : l0 - s1;
-            il = odd ? s1 + l0 : l1 + s0;
-          } else {
-            rh = h0;
-            ih = h1;
-            rl = l0;
-            il = l1;
+      for (int g0 = 0; g0 < NC; g0 += GC) {
+        if (g0) __syncwarp();  // the previous group's stores have read the staging area
+#pragma unroll
+        for (int k = 0; k < NL; ++k) {
+          const int jj = (BC ? (j0 + g0) / 2 : j0 + g0) + k;  // logical column within the tile
+          long long re[HL], im[HL];
+#pragma unroll
+          for (int h = 0; h < HL; ++h) {
+            im[h] = 0;
+            if constexpr (BC) {
+              const long long x0 = acc[h][g0 + 2 * k], x1 = acc[h][g0 + 2 * k + 1];
+              if constexpr (AC) {
+                const long long p0 = __shfl_xor_sync(0xffffffffu, x0, 1), p1 = __shfl_xor_sync(0xffffffffu, x1, 1);
+                // even lane: (re re, re im) own, (im re, im im) the partner's
+                re[h] = odd ? p0 - x1 : x0 - p1;
+                im[h] = odd ? p1 + x0 : x1 + p0;
+              } else {
+                re[h] = x0;
+                im[h] = x1;
+              }
+            } else {
+              const long long x = acc[h][g0 + k];
+              if constexpr (AC) {
+                const long long p = __shfl_xor_sync(0xffffffffu, x, 1);
+                re[h] = odd ? p : x;
+                im[h] = odd ? x : p;
+              } else {
+                re[h] = x;
+              }
+            }
           }
-        } else if constexpr (AC) {
-          const long long p = __shfl_xor_sync(0xffffffffu, hi[k], 1), s = __shfl_xor_sync(0xffffffffu, lo[k], 1);
-          rh = odd ? p : hi[k];
-          ih = odd ? hi[k] : p;
-          rl = odd ? s : lo[k];
-          il = odd ? lo[k] : s;
-        } else {
-          rh = hi[k];
-          rl = lo[k];
-        }
-        // with complex A the two lanes of a pair hold the same output: split columns
-        if (AC && ((k & 1) != (lane & 1))) continue;
-        const int eb = sh->col_exp[BC ? 2 * jj : jj];
-        double2 v;
-        if (ea == kExpMarked || eb == kExpMarked) {
-          const int n = nt * (BC ? C::BN / 2 : C::BN) + jj;
-          v = make_double2(0.0, 0.0);
-          if (m < g.M && n < g.N)
-            v = direct_dot(g, m, n, zb, kb0 * TC_BK, min(g.K, kb1 * TC_BK));
-          if (g.alpha_pow2) {
-            v.x *= g.ar;
-            v.y *= g.ar;
-          }
-        } else {
+          // with complex A the two lanes of a pair hold the same output: split columns
+          if (AC && ((k & 1) != (lane & 1))) continue;
+          const int eb = sh->col_exp[BC ? 2 * jj : jj];
           const int E = ebase + row_exp(eb);
-          v.x = joined(neg ? -rh : rh, neg ? -rl : rl, E);
-          v.y = (AC || BC) ? joined(neg ? -ih : ih, neg ? -il : il, E) : 0.0;
-        }
-        if (!g.alpha_pow2) v = make_double2(g.ar * v.x - g.ai * v.y, g.ar * v.y + g.ai * v.x);
-        stage[lr * RS + k] = v;
-      }
-      __syncwarp();
-      constexpr int RPP = 32 / NJ, NPASS = rows_out / RPP;
-      const int lc = lane % NJ, lrw = lane / NJ;
-      const long long cn = sh->col_off[(BC ? j0 / 2 : j0) + lc];
-#pragma unroll 4
-      for (int p = 0; p < NPASS; ++p) {
-        const int r = p * RPP + lrw;
-        const long long cm = __shfl_sync(0xffffffffu, coffm, (AC ? 2 * r : r) & 31);
-        if (r >= nrows || cn < 0) continue;
-        const long long off = cm + cn;
-        const double2 v = stage[r * RS + lc];
-        if (g.cc) {
-          if (red) {
-            atomicAdd(&Cc[off].x, v.x);
-            atomicAdd(&Cc[off].y, v.y);
-          } else {
-            Cc[off] = v;
+          auto value = [&](const long long (&x)[HL]) {
+            if constexpr (HL == 2)
+              return joined(neg ? -x[0] : x[0], neg ? -x[1] : x[1], E);
+            else
+              return scaled_i64_to_double(neg ? -x[0] : x[0], E);
+          };
+          double2 v = make_double2(value(re), (AC || BC) ? value(im) : 0.0);
+          if (HL == 2 && (ea == kExpMarked || eb == kExpMarked)) {
+            const int n = nt * (BC ? C::BN / 2 : C::BN) + jj;
+            v = make_double2(0.0, 0.0);
+            if (m < g.M && n < g.N) v = direct_dot(g, m, n, zb, kb0 * TC_BK, min(g.K, kb1 * TC_BK));
+            if (g.alpha_pow2) {
+              v.x *= g.ar;
+              v.y *= g.ar;
+            }
           }
-        } else {
-          if (red)
-            atomicAdd(&Cr[off], v.x);
-          else
-            Cr[off] = v.x;
+          if (!g.alpha_pow2) v = make_double2(g.ar * v.x - g.ai * v.y, g.ar * v.y + g.ai * v.x);
+          stage[lr * RS + k] = v;
+        }
+        __syncwarp();
+        // every lane owns a (row, column) pair per pass
+#pragma unroll 4
+        for (int i = lane; i < rows_out * NL; i += 32) {
+          const int r = i / NL, lc = i - r * NL;
+          const long long cm = __shfl_sync(0xffffffffu, coffm, (AC ? 2 * r : r) & 31);
+          const long long cn = sh->col_off[(BC ? (j0 + g0) / 2 : j0 + g0) + lc];
+          if (r >= nrows || cn < 0) continue;
+          const long long off = cm + cn;
+          const double2 v = stage[r * RS + lc];
+          if (g.cc) {
+            if (red) {
+              atomicAdd(&Cc[off].x, v.x);
+              atomicAdd(&Cc[off].y, v.y);
+            } else {
+              Cc[off] = v;
+            }
+          } else {
+            if (red)
+              atomicAdd(&Cr[off], v.x);
+            else
+              Cr[off] = v.x;
+          }
         }
       }
     }
@@ -358,11 +380,9 @@ __global__ void __launch_bounds__(TcDeep::THREADS, 1)
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
-}  // namespace
-
-cudaError_t launch_deep(const TcArgs& a0, const void* packA, const void* packB, cudaStream_t st) {
-  using C = TcDeep;
-  static_assert(sizeof(DeepShared) <= 2560, "shared-memory tail");
+template <class C>
+cudaError_t launch_deep_form(const TcArgs& a0, const void* packA, const void* packB, cudaStream_t st) {
+  static_assert(sizeof(DeepShared<C>) <= C::TAIL && C::SMEM <= 232448, "shared memory");
   constexpr int kMaxDev = 64;
   static std::once_flag once[kMaxDev];
   static cudaError_t attr_err[kMaxDev] = {};
@@ -370,8 +390,8 @@ cudaError_t launch_deep(const TcArgs& a0, const void* packA, const void* packB, 
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
   std::call_once(once[dev], [dev] {
     cudaError_t e = cudaSuccess;
-    for (auto fn : {ozaki_deep_kernel<true, true>, ozaki_deep_kernel<true, false>, ozaki_deep_kernel<false, true>,
-                    ozaki_deep_kernel<false, false>}) {
+    for (auto fn : {ozaki_deep_kernel<C, true, true>, ozaki_deep_kernel<C, true, false>,
+                    ozaki_deep_kernel<C, false, true>, ozaki_deep_kernel<C, false, false>}) {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -380,25 +400,37 @@ cudaError_t launch_deep(const TcArgs& a0, const void* packA, const void* packB, 
   });
   if (attr_err[dev] != cudaSuccess) return attr_err[dev];
   TcArgs a = a0;
-  if (a.S != TC_DEEP_SLICES || a.rowsB_pad % C::BN != 0 || a.rowsA_pad % TC_BM != 0) return cudaErrorInvalidValue;
+  if (a.S != C::S || a.rowsB_pad < 1 || a.rowsA_pad % TC_BM != 0) return cudaErrorInvalidValue;
   a.tmem_cols = 512;
   const CUtensorMap ma = slice_map(packA, a.S, (a.bat_a ? a.nb : 1) * a.rowsA_pad, a.kblocks * TC_BK, TC_BM);
   const CUtensorMap mb = slice_map(packB, a.S, (a.bat_b ? a.nb : 1) * a.rowsB_pad, a.kblocks * TC_BK, C::BN);
   // the tiles of the smaller operand side vary fastest: that side stays in L2
-  const unsigned mtiles = (unsigned)(a.rowsA_pad / TC_BM), ntiles = (unsigned)(a.rowsB_pad / C::BN);
+  const unsigned mtiles = (unsigned)(a.rowsA_pad / TC_BM);
+  const unsigned ntiles = (unsigned)(((long long)a.N * (a.bc ? 2 : 1) + C::BN - 1) / C::BN);
   a.m_fast = (a.rowsA_pad < a.rowsB_pad && ntiles <= 65535u) ? 1 : 0;
   if ((a.m_fast ? ntiles : mtiles) > 65535u || (long long)a.nb * a.nsplit > 65535LL) return cudaErrorInvalidConfiguration;
   dim3 grid(a.m_fast ? mtiles : ntiles, a.m_fast ? ntiles : mtiles, (unsigned)((long long)a.nb * a.nsplit));
   if (a.ac && a.bc)
-    ozaki_deep_kernel<true, true><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
+    ozaki_deep_kernel<C, true, true><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
   else if (a.ac)
-    ozaki_deep_kernel<true, false><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
+    ozaki_deep_kernel<C, true, false><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
   else if (a.bc)
-    ozaki_deep_kernel<false, true><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
+    ozaki_deep_kernel<C, false, true><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
   else
-    ozaki_deep_kernel<false, false><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
+    ozaki_deep_kernel<C, false, false><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
   count_launch();
   return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_deep(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st) {
+  switch (a.S) {
+    case 4: return launch_deep_form<TcDeep<4, 128, 6>>(a, packA, packB, st);
+    case 5: return launch_deep_form<TcDeep<5, 96, 8>>(a, packA, packB, st);
+    case 8: return launch_deep_form<TcDeep<8, 64, 9>>(a, packA, packB, st);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 }  // namespace tdcc

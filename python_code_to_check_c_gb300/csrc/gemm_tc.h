@@ -68,17 +68,20 @@ constexpr int tc_chunk_kblocks(int S) {
   return S <= 2 ? 16 : S == 3 ? (1 << 24) / (20480 * 64) : (1 << 24) / (24576 * 64);
 }
 
-// Deep form (gemm_deep.cu): 8 slices, 56 bits, 128 x 64 tile, the 8 level
-// accumulators of 64 columns filling TMEM; a ring of (A, B) slice pairs; int64
-// sums in the drain warps' registers across K chunks of at most 6 K blocks (a
-// level grows by at most 2 x 128 x 64 + 6 x 64 x 64 = 40960 per K index and
-// must stay within 2^24).
+// Deep form (gemm_deep.cu): a 128 x BN tile whose S level accumulators fill
+// TMEM, a ring of (A, B) slice pairs, sums over K in the drain warps'
+// registers across exact chunks of CHUNK_KB K blocks: a level of p pairs grows
+// by at most 2 x 128 x 64 + (p - 2) x 64 x 64 per K index and must stay within
+// 2^24.
+template <int S_, int BN_, int STAGES_>
 struct TcDeep {
-  static constexpr int BN = 64, STAGES = 9, EPI = 16;
+  static constexpr int S = S_, BN = BN_, STAGES = STAGES_, EPI = 16;
   static constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
   static constexpr int THREADS = 64 + 32 * EPI;
-  static constexpr int SMEM = 1024 + STAGES * (A_BYTES + B_BYTES) + 2560;
-  static constexpr int CHUNK_KB = (1 << 24) / (40960 * TC_BK);
+  static constexpr int TAIL = 2048;
+  static constexpr int SMEM = 1024 + STAGES * (A_BYTES + B_BYTES) + TAIL;
+  static constexpr int CHUNK_KB = (1 << 24) / ((16384 + (S - 2) * 4096) * TC_BK);
+  static_assert(S * BN <= 512 && STAGES >= S, "TMEM columns, ring");
 };
 
 cudaError_t launch_deep(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st);

@@ -1167,17 +1167,26 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
       a.alpha_neg = op.g.ar < 0.0 ? 1 : 0;
     }
     a.acc = op.g.acc;
-    // split K so that few output tiles still occupy the SMs: one CTA per SM,
-    // cost = waves x (K blocks per CTA + fixed pipeline/epilogue overhead);
-    // the 128-column tile takes at most one exact K chunk per CTA
     // S <= 4 and at most two K blocks: the persistent 64-column form, whose
     // TMEM drain runs under the next tile's loads and MMAs (measured at o=10,
     // v=38 with 24 trajectories: 10-35 % faster than the 128-column tile for
     // one or two K blocks, 30-50 % slower for six or more, where the
     // 128-column tile's MMA rate and operand reuse count)
     const bool persist = S <= TC_TILE128_MAX_S && a.kblocks <= 2;
-    const long long ctas = (rB / (tile128 && !persist ? TcTile128::BN : BN)) * (rA / BM) * nbt;
-    const long long min_sp = (tile128 || persist) ? (a.kblocks + tc_chunk_kblocks(S) - 1) / tc_chunk_kblocks(S) : 1;
+    // S = 4, 5 and longer K: the deep form, which sums all of K in one CTA.
+    // Against the 128-column tile (S = 4, o=10, v=38, 24 trajectories) 210 us
+    // for 335 on the ladder (23 blocks), 174 for 222 on the ring terms (6); against
+    // the 64-column tile (S = 5, o=18, v=82) 829 for 1842 (106 blocks), 420 for
+    // 890 (24).  A B side of less than 3/4 of a tile keeps the narrower ones.
+    const int deepBN = S == 5 ? 96 : 128;
+    const bool long_k = !deep && (S == 4 || S == 5) && a.kblocks > 2 && nBrows >= deepBN * 3 / 4;
+    // split K so that few output tiles still occupy the SMs: one CTA per SM,
+    // cost = waves x (K blocks per CTA + fixed pipeline/epilogue overhead);
+    // the 128-column tile takes at most one exact K chunk per CTA
+    const int tileN = long_k ? deepBN : tile128 && !persist ? TcTile128::BN : BN;
+    const long long ctas = (((long_k ? nBrows : rB) + tileN - 1) / tileN) * (rA / BM) * nbt;
+    const long long min_sp =
+        !long_k && (tile128 || persist) ? (a.kblocks + tc_chunk_kblocks(S) - 1) / tc_chunk_kblocks(S) : 1;
     long long splits = min_sp;
     {
       double best = 1e300;
@@ -1185,7 +1194,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
       for (long long sp = min_sp; sp <= maxs; ++sp) {
         const long long waves = (ctas * sp + 151) / 152;
         const long long per = (a.kblocks + sp - 1) / sp;
-        const double cost = (double)waves * (double)(per * S + 6);
+        const double cost = (double)waves * (double)(per * S + (long_k ? 12 : 6));
         if (cost < best - 1e-9) {
           best = cost;
           splits = sp;
@@ -1199,7 +1208,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     a.atomic = splits > 1 ? 1 : 0;
     t.zeroed = a.acc || a.atomic;  // split K is allowed (a zero op precedes when not accumulating)
     // short K: the narrow variant (two CTAs per SM overlap their latencies)
-    a.variant = deep ? 4 : persist ? 3 : tile128 ? 2 : (a.kb_per_split == 1 && S <= 5) ? 1 : 0;
+    a.variant = deep || long_k ? 4 : persist ? 3 : tile128 ? 2 : (a.kb_per_split == 1 && S <= 5) ? 1 : 0;
     t.bytes = (long long)S * (nbA * rA + nbB * rB) * Kp * 2 + nbt * M * N * elem_bytes(op.dtc);
     t.reads = {pa.pk_dst, pb.pk_dst};
     if (deep) {  // the drain reads the operands of rows that digits cannot hold

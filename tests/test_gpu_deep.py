@@ -89,3 +89,28 @@ def test_amplitudes_of_unusual_size(scale):
     finally:
         eng.close()
     assert rel_err(got, CCOracle(s.tei(), 7).lam2eq_rhs(*[x[0] for x in st], F[0])) < 1e-12
+
+
+@pytest.mark.parametrize("S,tol", [(4, 1e-7), (5, 1e-9)])  # the mixed form's bars
+@pytest.mark.parametrize("o,v,nb", [(7, 31, 1), (5, 45, 2), (12, 26, 3), (4, 60, 1)])
+def test_long_contractions_of_the_mixed_form(o, v, nb, S, tol):
+    """K from 3 blocks of 64 (o v) over several exact chunks (v^2), tiles of 96
+    and 128 columns with ragged edges, batches, every operand type."""
+    from oracle.cc_oracle import CCOracle
+    from python_code_to_check_c_gb300.engine import CCEngine
+    assert o * v > 128
+    s, st, F = _case(o, v, nb)
+    orc = CCOracle(s.tei(), o)
+    eng = CCEngine.from_system(s, nb=nb, device_integrals=False)
+    try:
+        eng.set_precision("mixed", S)
+        eng.set_tc_policy(0, 1, 1)  # every contraction on the tensor cores
+        one = [x if nb > 1 else x[0] for x in st]
+        for b, name in enumerate(NAMES["CCSD"]):
+            got = eng.rhs("CCSD", b, *one, F if nb > 1 else F[0]).cpu().numpy().reshape((nb,) + st[b].shape[1:])
+            for z in range(nb):
+                a = [st[0][z], st[1][z]] + ([st[2][z], st[3][z]] if b > 1 else [])
+                assert rel_err(got[z], getattr(orc, name)(*a, F[z])) < tol, (name, z)
+        eng.check_errors()
+    finally:
+        eng.close()
