@@ -1,12 +1,12 @@
 // Exact BF16 slice products on tcgen05 with the sums over all of K in the drain
 // warps' registers: the FP64 form's contractions (8 slices of 7 bits a side,
 // 56 bits under each row's maximum, the last digit rounded) and the mixed
-// form's with 4 or 5 slices and K beyond what the persistent form takes.
+// form's with up to 5 slices and K beyond two blocks.
 //
 // The products A_s B_t with s + t <= S + 1 go to the accumulators of their
 // levels L = s + t, FP32 sums of integers that stay exact over a K chunk
 // (TcDeep::CHUNK_KB).  The S levels of a 128 x BN tile fill TMEM (BN = 128, 96,
-// 64 for S = 4, 5, 8); after every chunk the drain warps add them to int64
+// 64 for S <= 4, 5, 8); after every chunk the drain warps add them to int64
 // sums (two per output for S = 8, levels 2..5 and 6..9), which are rounded to
 // FP64 once at the end.  With 8 slices what is dropped (levels above 9, the
 // operands' rounding) is about 2^-58 of the product of the two row maxima per
@@ -23,7 +23,7 @@
 // add up: 13.3 k clocks measured.  So the wider the tile the better (per
 // output column and K block 52, 82 and 204 clocks for S = 4, 5, 8).  Measured:
 // the 24-trajectory ladder at o=10, v=38 (S = 4, 1444 x 4800 x 1444 real) 210
-// us, 335 as single-chunk 128-column tiles over split K (TcTile128); the ladder
+// us, 335 as single-chunk 128-column tiles over split K; the ladder
 // at o=18, v=82 (S = 5, 6724 x 648 x 6724 real) 829 us, 1842 as 64-column tiles
 // with int64 partial sums in TMEM (TcWide).
 //
@@ -147,11 +147,8 @@ __global__ void __launch_bounds__(C::THREADS, 1)
   } else if (warp == 1) {
     // ---------------- MMA issuer (the whole warp, one lane executing) ----------------
     constexpr uint32_t id = idesc_bf16(TC_BM, C::BN);
-    const uint64_t hi64 = sdesc(0);
-    const uint32_t a0 = (smem_u32(stA) & 0x3FFFF) >> 4, b0 = (smem_u32(stB) & 0x3FFFF) >> 4;
-    const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
     const uint32_t on = lane == 0 ? 1u : 0u;
-    uint32_t st0 = 0, ph = 0;  // ring slot and phase of the block's first pair
+    PairRing<C::STAGES, C::A_BYTES, C::B_BYTES> ring(stA, stB, &sh->full[0], &sh->empty[0]);
     bool ok = true;
     for (int c = 0; c < nchunks && ok; ++c) {
       if (c > 0 && !mbar_wait_warp(smem_u32(&sh->accempty), (uint32_t)((c - 1) & 1), kWaitLimit)) {
@@ -161,49 +158,8 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       asm volatile("tcgen05.fence::after_thread_sync;");
       const int kbs = kb0 + c * C::CHUNK_KB, kbe = min(kb1, kbs + C::CHUNK_KB);
 #pragma unroll 1
-      for (int kb = kbs; kb < kbe && ok; ++kb) {
-        const bool first = kb == kbs;
-        // what an MMA needs beside constants of the unrolled loops, once per slice
-        uint32_t la[S], lb[S], slot[S];  // descriptor low words and ring slots of the block's slices
-#pragma unroll
-        for (int j = 0; j < S; ++j) {
-          slot[j] = st0 + j < C::STAGES ? st0 + j : st0 + j - C::STAGES;
-          la[j] = a0 + slot[j] * (C::A_BYTES >> 4);
-          lb[j] = b0 + slot[j] * (C::B_BYTES >> 4);
-        }
-#pragma unroll
-        for (int j = 1; j <= S; ++j) {
-          if (ok) ok = mbar_wait_warp(full0 + 8 * slot[j - 1], st0 + j - 1 < C::STAGES ? ph : ph ^ 1u, kWaitLimit);
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          if (ok) {
-            auto product = [&](int s, int t) {
-              // the first product of each level in a chunk starts its sum
-              const bool lead = s == t || s == t + 1;
-#pragma unroll
-              for (int k = 0; k < TC_BK / 16; ++k)
-                umma_warp(tmem + (uint32_t)((s + t - 2) * C::BN), hi64 | (uint64_t)(la[s - 1] + 2 * k),
-                          hi64 | (uint64_t)(lb[t - 1] + 2 * k), id, (lead && k == 0 && first) ? 0u : 1u, on);
-            };
-            const int last = S + 1 - j;  // largest partner of slice j
-#pragma unroll
-            for (int t = 1; t <= S; ++t)
-              if (t <= j && t <= last) product(j, t);
-#pragma unroll
-            for (int q = 1; q <= S; ++q)
-              if (q < j && q <= last) product(q, j);
-            if (j >= last) {  // pairs j and S + 1 - j have had their last use
-              umma_commit_warp(empty0 + 8 * slot[j - 1], on);
-              if (j > last) umma_commit_warp(empty0 + 8 * slot[last - 1], on);
-            }
-          }
-        }
-        if (!ok) fail(sh, g.err, 3);
-        st0 += S;
-        if (st0 >= C::STAGES) {
-          st0 -= C::STAGES;
-          ph ^= 1u;
-        }
-      }
+      for (int kb = kbs; kb < kbe && ok; ++kb) ok = ring.template issue<S, C::BN>(tmem, id, kb == kbs, on);
+      if (!ok) fail(sh, g.err, 3);
       if (ok) umma_commit_warp(smem_u32(&sh->accfull), on);
       ok = __all_sync(0xffffffffu, ok && sh->abort == 0) != 0;
     }
@@ -426,6 +382,9 @@ cudaError_t launch_deep_form(const TcArgs& a0, const void* packA, const void* pa
 
 cudaError_t launch_deep(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st) {
   switch (a.S) {
+    case 1: return launch_deep_form<TcDeep<1, 128, 6>>(a, packA, packB, st);
+    case 2: return launch_deep_form<TcDeep<2, 128, 6>>(a, packA, packB, st);
+    case 3: return launch_deep_form<TcDeep<3, 128, 6>>(a, packA, packB, st);
     case 4: return launch_deep_form<TcDeep<4, 128, 6>>(a, packA, packB, st);
     case 5: return launch_deep_form<TcDeep<5, 96, 8>>(a, packA, packB, st);
     case 8: return launch_deep_form<TcDeep<8, 64, 9>>(a, packA, packB, st);

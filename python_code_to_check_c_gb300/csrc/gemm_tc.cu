@@ -357,58 +357,36 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
         mbar_wait(smem_u32(&sh->full[j % C::STAGES]), (uint32_t)((j / C::STAGES) & 1), kWaitLimit);
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t id = idesc_bf16(TC_BM, C::BN);
-      int it = 0;
-      for (int c = 0; c < nchunks && !sh->abort; ++c) {
-        if (c > 0 && !mbar_wait(smem_u32(&sh->accempty), (uint32_t)((c - 1) & 1), kWaitLimit)) {
-          fail(sh, g.err, 2);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const int kbs = kb0 + c * TC_CHUNK_KB, kbe = min(kb1, kbs + TC_CHUNK_KB);
-        bool first = true;
-        for (int kb = kbs; kb < kbe && !sh->abort; ++kb, it += S) {
-          bool ok = true;
-          for (int s = 0; s < S; ++s) {
-            const int j = it + s;
-            if (!mbar_wait(smem_u32(&sh->full[j % C::STAGES]), (uint32_t)((j / C::STAGES) & 1), kWaitLimit)) {
-              ok = false;
-              break;
-            }
-          }
-          if (!ok) {
-            fail(sh, g.err, 3);
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          for (int L = 2; L <= S + 1; ++L) {
-            const uint32_t dacc = tmem + (uint32_t)((L - 2) * C::BN);
-            int np = 0;
-            for (int s = 1; s < L; ++s) {
-              const int t = L - s;
-              if (s > S || t > S) continue;
-              const int sa = (it + s - 1) % C::STAGES, sb = (it + t - 1) % C::STAGES;
-              const uint64_t da = sdesc(smem_u32(stA + sa * TC_A_BYTES));
-              const uint64_t db = sdesc(smem_u32(stB + sb * C::B_BYTES));
-#pragma unroll
-              for (int k = 0; k < TC_BK / 16; ++k) {
-                const uint32_t accf = (first && np == 0 && k == 0) ? 0u : 1u;
-                umma(dacc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), id, accf);
-              }
-              ++np;
-            }
-          }
-          first = false;
-          for (int s = 0; s < S; ++s) umma_commit(smem_u32(&sh->empty[(it + s) % C::STAGES]));
-        }
-        umma_commit(smem_u32(&sh->accfull));
+    // ---------------- MMA issuer (the whole warp, one lane executing) ----------------
+    constexpr uint32_t id = idesc_bf16(TC_BM, C::BN);
+    const uint32_t on = lane == 0 ? 1u : 0u;
+    PairRing<C::STAGES, TC_A_BYTES, C::B_BYTES> ring(stA, stB, &sh->full[0], &sh->empty[0]);
+    bool ok = true;
+    for (int c = 0; c < nchunks && ok; ++c) {
+      if (c > 0 && !mbar_wait_warp(smem_u32(&sh->accempty), (uint32_t)((c - 1) & 1), kWaitLimit)) {
+        fail(sh, g.err, 2);
+        break;
       }
-      // all issued MMAs complete before TMEM is released
-      umma_commit(smem_u32(&sh->done));
-      mbar_wait(smem_u32(&sh->done), 0, kWaitLimit);
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const int kbs = kb0 + c * TC_CHUNK_KB, kbe = min(kb1, kbs + TC_CHUNK_KB);
+#pragma unroll 1
+      for (int kb = kbs; kb < kbe && ok; ++kb)
+        switch (S) {
+          case 1: ok = ring.template issue<1, C::BN>(tmem, id, kb == kbs, on); break;
+          case 2: ok = ring.template issue<2, C::BN>(tmem, id, kb == kbs, on); break;
+          case 3: ok = ring.template issue<3, C::BN>(tmem, id, kb == kbs, on); break;
+          case 4: ok = ring.template issue<4, C::BN>(tmem, id, kb == kbs, on); break;
+          case 5: ok = ring.template issue<5, C::BN>(tmem, id, kb == kbs, on); break;
+          default:
+            if constexpr (C::STAGES >= 6) ok = ring.template issue<6, C::BN>(tmem, id, kb == kbs, on);
+        }
+      if (!ok) fail(sh, g.err, 3);
+      if (ok) umma_commit_warp(smem_u32(&sh->accfull), on);
+      ok = __all_sync(0xffffffffu, ok && sh->abort == 0) != 0;
     }
+    // all issued MMAs complete before TMEM is released
+    umma_commit_warp(smem_u32(&sh->done), on);
+    mbar_wait(smem_u32(&sh->done), 0, kWaitLimit);
   } else {
     // ---------------- epilogue (warps 2 .. 2 + C::EPI - 1) ----------------
     // C::EPI / 4 warps per TMEM lane quarter, each owning a slice of the
@@ -627,304 +605,19 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 }
 
 // ---------------------------------------------------------------------------
-// 128-column tile for S <= 4 slices (TcTile128): one K range per CTA.
-//
-// A tcgen05.mma of 128 x N x 16 costs the same ~71 cycles for every N <= 128,
-// and the TMA unit of an SM delivers about 62 GB/s, so the 64-column tile
-// spends half of its MMA time and 1.5x the loaded bytes per output that a
-// 128-column tile does.  S level accumulators of 128 columns fill TMEM
-// (S <= 4), which leaves no room for int64 partial sums across K chunks:
-// each CTA therefore takes at most one exact chunk of K (the planner splits
-// longer K across CTAs, whose results meet in the output by L2 reductions)
-// and drains TMEM once.  Level sums per K index are at most
-// 2^13 + 2^12 + 2^12 + 2^13 = 24576 (S = 4), so 10 K blocks (640) stay
-// below 2^24 and exact in FP32 (tc_chunk_kblocks).  The ring holds single
-// slices (a 128 x 64 tile of A or of B) with their own barriers: the
-// products of a K block run row by row, (1,1) .. (1,S), (2,1) .., and each
-// slice is released right after its last product, so the TMA (the bound
-// of this tile: about 62 GB/s per SM) keeps loading the next block while
-// the current one finishes.  The drain takes 16 columns at a time per warp,
-// stages them in the idle operand ring (one area per warp) and writes them
-// at once, so the whole tile is never staged.
-// ---------------------------------------------------------------------------
-template <bool AC, bool BC>
-__global__ void __launch_bounds__(TcTile128::THREADS, 1)
-    ozaki_tile128_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                         const TcArgs g) {
-  using C = TcTile128;
-  extern __shared__ uint8_t smraw[];
-  uint8_t* sm = (uint8_t*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
-  uint8_t* ring = sm;  // STAGES slots of 16 KB: one slice of A or of B each
-  TcShared<C>* sh = (TcShared<C>*)(ring + C::STAGES * C::SLOT_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int S = g.S;
-  const int ncols = g.tmem_cols;
-
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < C::STAGES; ++i) {
-      mbar_init(smem_u32(&sh->full[i]), 1);
-      mbar_init(smem_u32(&sh->empty[i]), 1);
-    }
-    mbar_init(smem_u32(&sh->accfull), 1);
-    mbar_init(smem_u32(&sh->accempty), 32 * C::EPI);
-    mbar_init(smem_u32(&sh->done), 1);
-    sh->abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;");
-    asm volatile("fence.proxy.async.shared::cta;");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem)),
-                 "r"(ncols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = sh->tmem;
-
-  const int mt = g.m_fast ? blockIdx.x : blockIdx.y, nt = g.m_fast ? blockIdx.y : blockIdx.x;
-  const int zb = blockIdx.z / g.nsplit;  // batch
-  const int kb0 = (blockIdx.z - zb * g.nsplit) * g.kb_per_split;
-  const int rowA0 = (g.bat_a ? zb * g.rowsA_pad : 0);
-  const int rowB0 = (g.bat_b ? zb * g.rowsB_pad : 0);
-  const int kb1 = min(g.kblocks, kb0 + g.kb_per_split);
-  // Per K block the 2S slices enter the ring in the order A1, B1 .. BS,
-  // A2 .. AS, and the products run row by row, (1,1) .. (1,S), (2,1) ..
-  // (2,S-1), .., (S,1): products start once A1 and B1 have landed, and after
-  // row s both A_s and B_(S+1-s) have had their last use and are released.
-  // Position of a slice within its block: A1 -> 0, B_t -> t, A_s -> S + s - 1.
-  const int per = 2 * S;
-
-  if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int j = 0;
-      for (int kb = kb0; kb < kb1 && !sh->abort; ++kb)
-        for (int i = 0; i < per && !sh->abort; ++i, ++j) {
-          const int st = j % C::STAGES;
-          const uint32_t ph = (uint32_t)((j / C::STAGES) & 1);
-          if (!mbar_wait(smem_u32(&sh->empty[st]), ph ^ 1u, kWaitLimit)) {
-            fail(sh, g.err, 1);
-            break;
-          }
-          const uint32_t fb = smem_u32(&sh->full[st]);
-          mbar_expect_tx(fb, C::SLOT_BYTES);
-          if (i == 0 || i > S)  // A_1, then A_2 .. A_S
-            tma3d(smem_u32(ring + st * C::SLOT_BYTES), &tmA, kb * TC_BK, rowA0 + mt * TC_BM, i == 0 ? 0 : i - S, fb);
-          else  // B_1 .. B_S
-            tma3d(smem_u32(ring + st * C::SLOT_BYTES), &tmB, kb * TC_BK, rowB0 + nt * C::BN, i - 1, fb);
-        }
-      const int issued = j;
-      for (int q = (issued > C::STAGES ? issued - C::STAGES : 0); q < issued; ++q)
-        mbar_wait(smem_u32(&sh->full[q % C::STAGES]), (uint32_t)((q / C::STAGES) & 1), kWaitLimit);
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t id = idesc_bf16(TC_BM, C::BN);
-      int j0 = 0;
-      bool first = true;
-      for (int kb = kb0; kb < kb1 && !sh->abort; ++kb, j0 += per) {
-        bool ok = true;
-        for (int s = 1; s <= S && ok; ++s) {
-          const int ja = j0 + (s == 1 ? 0 : S + s - 1);  // A_s
-          if (!mbar_wait(smem_u32(&sh->full[ja % C::STAGES]), (uint32_t)((ja / C::STAGES) & 1), kWaitLimit)) {
-            ok = false;
-            break;
-          }
-          const uint64_t da = sdesc(smem_u32(ring + (ja % C::STAGES) * C::SLOT_BYTES));
-          for (int t = 1; t <= S + 1 - s; ++t) {
-            const int jb = j0 + t;  // B_t
-            if (s == 1 &&
-                !mbar_wait(smem_u32(&sh->full[jb % C::STAGES]), (uint32_t)((jb / C::STAGES) & 1), kWaitLimit)) {
-              ok = false;
-              break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint64_t db = sdesc(smem_u32(ring + (jb % C::STAGES) * C::SLOT_BYTES));
-            const uint32_t dacc = tmem + (uint32_t)((s + t - 2) * C::BN);
-#pragma unroll
-            for (int k = 0; k < TC_BK / 16; ++k) {
-              // the first product of each level (s = 1) in the first K block starts its accumulator
-              const uint32_t accf = (first && s == 1 && k == 0) ? 0u : 1u;
-              umma(dacc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), id, accf);
-            }
-          }
-          if (!ok) break;
-          // A_s and B_(S+1-s) have had their last use: free their slots
-          umma_commit(smem_u32(&sh->empty[ja % C::STAGES]));
-          umma_commit(smem_u32(&sh->empty[(j0 + S + 1 - s) % C::STAGES]));
-        }
-        if (!ok) {
-          fail(sh, g.err, 3);
-          break;
-        }
-        first = false;
-      }
-      umma_commit(smem_u32(&sh->accfull));
-      umma_commit(smem_u32(&sh->done));
-      mbar_wait(smem_u32(&sh->done), 0, kWaitLimit);
-    }
-  } else {
-    // ---------------- epilogue (warps 2 .. 17) ----------------
-    constexpr int kWq = C::EPI / 4;   // 4 warps per lane quarter
-    constexpr int kCw = C::BN / kWq;  // 32 packed columns per warp
-    const int q = warp & 3;
-    const int hcol = (warp - 2) >> 2;
-    const int row = q * 32 + lane;
-    const int u = 7 * (S + 1);  // S <= 4: sum_L v_L 2^(u - 7L) is exact in int64
-    {
-      const int t = threadIdx.x - 64;
-      constexpr int ncl = BC ? C::BN / 2 : C::BN;
-      if (t < ncl) {
-        const int n = nt * ncl + t;
-        long long o = -1;
-        if (n < g.N) decomp_tc(g.gnC, n, o);
-        sh->col_off[t] = o;
-      }
-      if (t < C::BN) sh->col_exp[t] = row_exp(g.expB[rowB0 + nt * C::BN + t]);
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * C::EPI) : "memory");
-    }
-    const int prow = mt * TC_BM + row;
-    const int m = AC ? (prow >> 1) : prow;
-    const bool odd = AC && (lane & 1);
-    constexpr int NJ = BC ? 8 : 16;          // logical columns per 16 packed columns
-    constexpr int rows_out = AC ? 16 : 32;    // logical rows of this warp
-    constexpr int RS = NJ + 1;                // staging row stride (double2), padded
-    double2* stage = reinterpret_cast<double2*>(sm) + (size_t)(warp - 2) * (32 * RS);
-    const int lr = AC ? (lane >> 1) : lane;
-    const uint32_t tl = (uint32_t)(q * 32) << 16;
-    bool ok = !__any_sync(0xffffffffu, sh->abort != 0);
-    if (ok) {
-      const bool got = mbar_wait(smem_u32(&sh->accfull), 0u, kWaitLimit);
-      if (!__all_sync(0xffffffffu, got)) {
-        fail(sh, g.err, 4);
-        ok = false;
-      }
-    }
-    if (ok && __any_sync(0xffffffffu, sh->abort != 0)) ok = false;
-    if (ok) {
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      const int ea = prow < g.rowsA_pad ? row_exp(g.expA[rowA0 + prow]) : 0;
-      const int ebase = ea - u + (g.alpha_pow2 ? g.alpha_e : 0);
-      const bool neg = g.alpha_pow2 && g.alpha_neg;
-      long long coffm = 0;
-      if (m < g.M) decomp_tc(g.gmC, m, coffm);
-      double2* Cc = static_cast<double2*>(g.C) + (g.cc ? zb * g.bsC : 0);
-      double* Cr = static_cast<double*>(g.C) + (g.cc ? 0 : zb * g.bsC);
-      const int m0w = AC ? ((mt * TC_BM + q * 32) >> 1) : (mt * TC_BM + q * 32);
-      const int nrows = min(rows_out, g.M - m0w);
-      const bool red = g.acc || g.atomic;
-      constexpr int RPP = 32 / NJ;  // rows per store pass
-      constexpr int NPASS = rows_out / RPP;
-      const int lc = lane % NJ, lrw = lane / NJ;
-#pragma unroll 1
-      for (int j0 = hcol * kCw; j0 < (hcol + 1) * kCw; j0 += 16) {
-        long long a16[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) a16[j] = 0;
-#pragma unroll
-        for (int L0 = 2; L0 <= 5; L0 += 2) {
-          if (L0 > S + 1) break;
-          uint32_t lv[2][16];
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-            if (L0 + i <= S + 1) tmem_ld16_nowait(tmem + tl + (uint32_t)((L0 + i - 2) * C::BN + j0), lv[i]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int L = L0 + i;
-            if (L > S + 1) break;
-            const int shl = u - 7 * L;  // >= 0 for L <= S + 1
-#pragma unroll
-            for (int j = 0; j < 16; ++j) a16[j] += (long long)__float2int_rn(__uint_as_float(lv[i][j])) << shl;
-          }
-        }
-        __syncwarp();  // the previous group's stores have read the staging area
-#pragma unroll
-        for (int k = 0; k < NJ; ++k) {
-          const int jj = (BC ? j0 / 2 : j0) + k;  // logical column within the tile
-          long long re, im;
-          if constexpr (BC) {
-            const long long x0 = a16[2 * k], x1 = a16[2 * k + 1];
-            if constexpr (AC) {
-              const long long p0 = __shfl_xor_sync(0xffffffffu, x0, 1);
-              const long long p1 = __shfl_xor_sync(0xffffffffu, x1, 1);
-              const long long rr = odd ? p0 : x0, ri = odd ? p1 : x1, ir = odd ? x0 : p0, ii = odd ? x1 : p1;
-              re = rr - ii;
-              im = ri + ir;
-            } else {
-              re = x0;
-              im = x1;
-            }
-          } else {
-            const long long x = a16[k];
-            if constexpr (AC) {
-              const long long p = __shfl_xor_sync(0xffffffffu, x, 1);
-              re = odd ? p : x;
-              im = odd ? x : p;
-            } else {
-              re = x;
-              im = 0;
-            }
-          }
-          if (AC && ((k & 1) != (lane & 1))) continue;
-          const int E = ebase + sh->col_exp[BC ? 2 * jj : jj];
-          double vr, vi;
-          if (g.alpha_pow2) {
-            vr = scaled_i64_to_double(neg ? -re : re, E);
-            vi = scaled_i64_to_double(neg ? -im : im, E);
-          } else {
-            const double dr = scaled_i64_to_double(re, E), di = scaled_i64_to_double(im, E);
-            vr = g.ar * dr - g.ai * di;
-            vi = g.ar * di + g.ai * dr;
-          }
-          stage[lr * RS + k] = make_double2(vr, vi);
-        }
-        __syncwarp();
-        // store the group: every lane owns a (row, column) pair per pass
-        const long long cn = sh->col_off[(BC ? j0 / 2 : j0) + lc];
-#pragma unroll 4
-        for (int p = 0; p < NPASS; ++p) {
-          const int r = p * RPP + lrw;
-          const long long cm = __shfl_sync(0xffffffffu, coffm, (AC ? 2 * r : r) & 31);
-          if (r >= nrows || cn < 0) continue;
-          const long long off = cm + cn;
-          const double2 v = stage[r * RS + lc];
-          if (g.cc) {
-            if (red) {
-              atomicAdd(&Cc[off].x, v.x);
-              atomicAdd(&Cc[off].y, v.y);
-            } else {
-              Cc[off] = v;
-            }
-          } else {
-            if (red)
-              atomicAdd(&Cr[off], v.x);
-            else
-              Cr[off] = v.x;
-          }
-        }
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
-}
-
-// ---------------------------------------------------------------------------
 // Persistent 64-column form for S <= 4 slices (TcPersist).  One CTA per SM
 // walks the output tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... (each
-// at most one exact K chunk, as in the 128-column form).  Two TMEM buffers of
+// at most one exact K chunk).  Two TMEM buffers of
 // S level accumulators: the MMA issuer fills buffer j & 1 for its j-th tile
 // once the drain warps have released it (accempty), the drain warps empty it
 // once its MMAs are complete (accfull) and release it as soon as the levels
 // are in registers, before they convert and store -- so a tile's drain runs
 // under the next tile's loads and MMAs.  A and B slices have rings of their
 // own (A1 .. AS and B1 .. BS per K block, products row by row, each slice
-// released after its last product).
+// released after its last product).  Bound: the drain, 11 k to 20 k clocks a
+// tile against 5 k a K block for loads and products; accumulated outputs are
+// reductions in L2 (as loads and stores the o=10, v=38 contractions of 24
+// trajectories took 180 us instead of 150).
 // ---------------------------------------------------------------------------
 struct PersistShared {
   uint64_t fullA[TcPersist::RA], emptyA[TcPersist::RA];
@@ -958,6 +651,87 @@ __device__ __forceinline__ TileCoord persist_tile(const TcArgs& g, int t, int mt
   c.rowA0 = g.bat_a ? c.zb * g.rowsA_pad : 0;
   c.rowB0 = g.bat_b ? c.zb * g.rowsB_pad : 0;
   return c;
+}
+
+// The MMA warp of the persistent form.  The ring slots and descriptor words of
+// a K block's slices are computed once per slice; with them worked out for
+// every product (a ring index, a modulo, a descriptor) the issue of 10
+// products took longer than the products.
+template <int S>
+__device__ __forceinline__ void persist_issue(const TcArgs& g, PersistShared* sh, const uint8_t* ringA,
+                                              const uint8_t* ringB, uint32_t tmem, int ntiles_total, int mtiles,
+                                              int ntiles, int lane) {
+  using C = TcPersist;
+  constexpr uint32_t id = idesc_bf16(TC_BM, C::BN);
+  const uint64_t hi64 = sdesc(0);
+  const uint32_t a0 = (smem_u32(ringA) & 0x3FFFF) >> 4, b0 = (smem_u32(ringB) & 0x3FFFF) >> 4;
+  const uint32_t fullA = smem_u32(&sh->fullA[0]), emptyA = smem_u32(&sh->emptyA[0]);
+  const uint32_t fullB = smem_u32(&sh->fullB[0]), emptyB = smem_u32(&sh->emptyB[0]);
+  const uint32_t on = lane == 0 ? 1u : 0u;
+  uint32_t sa0 = 0, pa = 0, sb0 = 0, pb = 0;  // ring slot and phase of the block's first slices
+  int jt = 0;
+  bool ok = true;
+  for (int t = blockIdx.x; t < ntiles_total && ok; t += gridDim.x, ++jt) {
+    const TileCoord c = persist_tile(g, t, mtiles, ntiles);
+    const int b = jt & 1, use = jt >> 1;
+    if (use > 0 && !mbar_wait_warp(smem_u32(&sh->accempty[b]), (uint32_t)((use - 1) & 1), kWaitLimit)) {
+      fail(sh, g.err, 2);
+      break;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t dbuf = tmem + (uint32_t)(b * S * C::BN);
+#pragma unroll 1
+    for (int kb = c.kb0; kb < c.kb1 && ok; ++kb) {
+      const bool first = kb == c.kb0;
+      uint32_t la[S], lb[S], qa[S], qb[S];
+#pragma unroll
+      for (int j = 0; j < S; ++j) {
+        qa[j] = sa0 + j < C::RA ? sa0 + j : sa0 + j - C::RA;
+        qb[j] = sb0 + j < C::RB ? sb0 + j : sb0 + j - C::RB;
+        la[j] = a0 + qa[j] * (C::A_SLOT >> 4);
+        lb[j] = b0 + qb[j] * (C::B_SLOT >> 4);
+      }
+#pragma unroll
+      for (int s = 1; s <= S; ++s) {
+        if (ok) ok = mbar_wait_warp(fullA + 8 * qa[s - 1], sa0 + s - 1 < C::RA ? pa : pa ^ 1u, kWaitLimit);
+#pragma unroll
+        for (int tt = 1; tt <= S; ++tt) {
+          if (tt > S + 1 - s) continue;
+          if (s == 1 && ok) ok = mbar_wait_warp(fullB + 8 * qb[tt - 1], sb0 + tt - 1 < C::RB ? pb : pb ^ 1u, kWaitLimit);
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          if (ok) {
+#pragma unroll
+            for (int k = 0; k < TC_BK / 16; ++k)
+              umma_warp(dbuf + (uint32_t)((s + tt - 2) * C::BN), hi64 | (uint64_t)(la[s - 1] + 2 * k),
+                        hi64 | (uint64_t)(lb[tt - 1] + 2 * k), id, (first && s == 1 && k == 0) ? 0u : 1u, on);
+          }
+        }
+        if (ok) {  // A_s and B_(S+1-s) have had their last use in this K block
+          umma_commit_warp(emptyA + 8 * qa[s - 1], on);
+          umma_commit_warp(emptyB + 8 * qb[S - s], on);
+        }
+      }
+      sa0 += S;
+      if (sa0 >= C::RA) {
+        sa0 -= C::RA;
+        pa ^= 1u;
+      }
+      sb0 += S;
+      if (sb0 >= C::RB) {
+        sb0 -= C::RB;
+        pb ^= 1u;
+      }
+    }
+    if (!ok) {
+      fail(sh, g.err, 3);
+      break;
+    }
+    umma_commit_warp(smem_u32(&sh->accfull[b]), on);
+    ok = __all_sync(0xffffffffu, sh->abort == 0) != 0;
+  }
+  // all issued MMAs complete before TMEM is released
+  umma_commit_warp(smem_u32(&sh->done), on);
+  mbar_wait(smem_u32(&sh->done), 0, kWaitLimit);
 }
 
 template <bool AC, bool BC>
@@ -1045,60 +819,12 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
         mbar_wait(smem_u32(&sh->fullB[q % C::RB]), (uint32_t)((q / C::RB) & 1), kWaitLimit);
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t id = idesc_bf16(TC_BM, C::BN);
-      int ja = 0, jb = 0, jt = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < ntiles_total && ok && !sh->abort; t += gridDim.x, ++jt) {
-        const TileCoord c = persist_tile(g, t, mtiles, ntiles);
-        const int b = jt & 1, use = jt >> 1;
-        if (use > 0 && !mbar_wait(smem_u32(&sh->accempty[b]), (uint32_t)((use - 1) & 1), kWaitLimit)) {
-          fail(sh, g.err, 2);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t dbuf = tmem + (uint32_t)b * buf_cols;
-        bool first = true;
-        for (int kb = c.kb0; kb < c.kb1 && ok; ++kb, ja += S, jb += S) {
-          for (int s = 1; s <= S && ok; ++s) {
-            const int qa = ja + s - 1;  // A_s
-            if (!mbar_wait(smem_u32(&sh->fullA[qa % C::RA]), (uint32_t)((qa / C::RA) & 1), kWaitLimit)) {
-              ok = false;
-              break;
-            }
-            const uint64_t da = sdesc(smem_u32(ringA + (qa % C::RA) * C::A_SLOT));
-            for (int tt = 1; tt <= S + 1 - s; ++tt) {
-              const int qb = jb + tt - 1;  // B_tt
-              if (s == 1 &&
-                  !mbar_wait(smem_u32(&sh->fullB[qb % C::RB]), (uint32_t)((qb / C::RB) & 1), kWaitLimit)) {
-                ok = false;
-                break;
-              }
-              asm volatile("tcgen05.fence::after_thread_sync;");
-              const uint64_t db = sdesc(smem_u32(ringB + (qb % C::RB) * C::B_SLOT));
-              const uint32_t dacc = dbuf + (uint32_t)((s + tt - 2) * C::BN);
-#pragma unroll
-              for (int k = 0; k < TC_BK / 16; ++k) {
-                const uint32_t accf = (first && s == 1 && k == 0) ? 0u : 1u;
-                umma(dacc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), id, accf);
-              }
-            }
-            if (!ok) break;
-            // A_s and B_(S+1-s) have had their last use in this K block
-            umma_commit(smem_u32(&sh->emptyA[qa % C::RA]));
-            umma_commit(smem_u32(&sh->emptyB[(jb + S - s) % C::RB]));
-          }
-          first = false;
-        }
-        if (!ok) {
-          fail(sh, g.err, 3);
-          break;
-        }
-        umma_commit(smem_u32(&sh->accfull[b]));
-      }
-      umma_commit(smem_u32(&sh->done));
-      mbar_wait(smem_u32(&sh->done), 0, kWaitLimit);
+    // ---------------- MMA issuer (the whole warp, one lane executing) ----------------
+    switch (S) {
+      case 1: persist_issue<1>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
+      case 2: persist_issue<2>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
+      case 3: persist_issue<3>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
+      default: persist_issue<4>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
     }
   } else {
     // ---------------- drain warps (2 .. 17): 16 columns each ----------------
@@ -1146,27 +872,32 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
         continue;  // the next tile's decision stops every drain warp
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-      long long a16[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) a16[j] = 0;
+      // Level sums of at most two K blocks stay below 2^22 (24576 x 128), so
+      // adding 1.5 x 2^23 leaves the integer in the low bits of the float,
+      // and two levels (2^7 apart) meet in 32 bits.
+      static_assert(24576LL * C::MAX_KB * TC_BK <= (1 << 22), "level sums of a persistent tile");
+      int p01[16], p23[16];
 #pragma unroll
       for (int L0 = 2; L0 <= 5; L0 += 2) {
-        if (L0 > S + 1) break;
-        uint32_t lv[2][16];
+        int* p = L0 == 2 ? p01 : p23;
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-          if (L0 + i <= S + 1)
-            tmem_ld16_nowait(tmem + tl + (uint32_t)b * buf_cols + (uint32_t)((L0 + i - 2) * C::BN + j0), lv[i]);
+        for (int j = 0; j < 16; ++j) p[j] = 0;
+        if (L0 > S + 1) continue;
+        uint32_t lv[2][16];
+        tmem_ld16_nowait(tmem + tl + (uint32_t)b * buf_cols + (uint32_t)((L0 - 2) * C::BN + j0), lv[0]);
+        if (L0 < S + 1) tmem_ld16_nowait(tmem + tl + (uint32_t)b * buf_cols + (uint32_t)((L0 - 1) * C::BN + j0), lv[1]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int L = L0 + i;
-          if (L > S + 1) break;
-          const int shl = u - 7 * L;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) a16[j] += (long long)__float2int_rn(__uint_as_float(lv[i][j])) << shl;
+        for (int j = 0; j < 16; ++j) {
+          p[j] = (int)(__float_as_uint(__fadd_rn(__uint_as_float(lv[0][j]), 12582912.f)) - 0x4B400000u);
+          if (L0 < S + 1)
+            p[j] = (p[j] << 7) + (int)(__float_as_uint(__fadd_rn(__uint_as_float(lv[1][j]), 12582912.f)) - 0x4B400000u);
         }
       }
+      // units of 2^-u: level L weighs 2^(u - 7 L), u = 7 (S + 1)
+      long long a16[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) a16[j] = S <= 2 ? p01[j] : ((long long)p01[j] << (7 * (S - 2))) + p23[j];
       // the levels are in registers: the MMAs of a later tile may refill this buffer
       asm volatile("tcgen05.fence::before_thread_sync;");
       mbar_arrive(smem_u32(&sh->accempty[b]));
@@ -1274,8 +1005,12 @@ constexpr int kSimtMaxK = 64;
 // Tile BM x BN (32 x 32, 16 x 64 or 64 x 16), 256 threads on a 16 x 16 grid,
 // 4 outputs each: rows ty + 16 i, columns tx + 16 j.  Digits in shared memory
 // per K index and row: S x (2 if complex) floats, contiguous, read as float2.
+// Three blocks per SM: a block's exponents, digits and stores are chains of
+// loads that the others' multiply-adds cover (the K = 10 contractions at o=10,
+// v=38 with 24 trajectories: 198 us with two, 181 with three; K = 18 at o=18,
+// v=82: 258, 228).
 template <bool AC, bool BC, bool CC, int S, int BM, int BN>
-__global__ void __launch_bounds__(256, 2) simt_slices_kernel(const GemmArgs g, int alpha_pow2, int alpha_e,
+__global__ void __launch_bounds__(256, 3) simt_slices_kernel(const GemmArgs g, int alpha_pow2, int alpha_e,
                                                              int alpha_neg) {
   constexpr int PA = AC ? 2 : 1, PB = BC ? 2 : 1;
   constexpr int SPA = (S * PA + 1) / 2 * 2, SPB = (S * PB + 1) / 2 * 2;  // floats per row, even
@@ -1705,50 +1440,6 @@ static cudaError_t launch_variant(const TcArgs& a0, const void* packA, const voi
   return cudaGetLastError();
 }
 
-static cudaError_t launch_tile128(const TcArgs& a0, const void* packA, const void* packB, cudaStream_t st) {
-  using C = TcTile128;
-  constexpr int kMaxDev = 64;
-  static std::once_flag once[kMaxDev];
-  static cudaError_t attr_err[kMaxDev] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
-  std::call_once(once[dev], [dev] {
-    cudaError_t e = cudaSuccess;
-    for (auto fn : {ozaki_tile128_kernel<true, true>, ozaki_tile128_kernel<true, false>,
-                    ozaki_tile128_kernel<false, true>, ozaki_tile128_kernel<false, false>}) {
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    }
-    attr_err[dev] = e;
-  });
-  if (attr_err[dev] != cudaSuccess) return attr_err[dev];
-  TcArgs a = a0;
-  // one exact K chunk per CTA, S level accumulators of 128 columns
-  if (a.S < 1 || a.S > TC_TILE128_MAX_S || 2 * a.S > C::STAGES || a.kb_per_split > tc_chunk_kblocks(a.S))
-    return cudaErrorInvalidValue;
-  int cols = 32;
-  while (cols < a.S * C::BN) cols *= 2;
-  a.tmem_cols = cols;
-  if (a.rowsB_pad % C::BN != 0 || a.rowsA_pad % TC_BM != 0) return cudaErrorInvalidValue;
-  const CUtensorMap ma = slice_map(packA, a.S, (a.bat_a ? a.nb : 1) * a.rowsA_pad, a.kblocks * TC_BK, TC_BM);
-  const CUtensorMap mb = slice_map(packB, a.S, (a.bat_b ? a.nb : 1) * a.rowsB_pad, a.kblocks * TC_BK, C::BN);
-  const unsigned mtiles = (unsigned)(a.rowsA_pad / TC_BM), ntiles = (unsigned)(a.rowsB_pad / C::BN);
-  a.m_fast = (a.rowsA_pad < a.rowsB_pad && ntiles <= 65535u) ? 1 : 0;
-  if ((a.m_fast ? ntiles : mtiles) > 65535u || (long long)a.nb * a.nsplit > 65535LL) return cudaErrorInvalidConfiguration;
-  dim3 grid(a.m_fast ? mtiles : ntiles, a.m_fast ? ntiles : mtiles, (unsigned)((long long)a.nb * a.nsplit));
-  if (a.ac && a.bc)
-    ozaki_tile128_kernel<true, true><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
-  else if (a.ac)
-    ozaki_tile128_kernel<true, false><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
-  else if (a.bc)
-    ozaki_tile128_kernel<false, true><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
-  else
-    ozaki_tile128_kernel<false, false><<<grid, C::THREADS, C::SMEM, st>>>(ma, mb, a);
-  count_launch();
-  return cudaGetLastError();
-}
-
 static cudaError_t launch_persist(const TcArgs& a0, const void* packA, const void* packB, cudaStream_t st) {
   using C = TcPersist;
   constexpr int kMaxDev = 64;
@@ -1769,8 +1460,8 @@ static cudaError_t launch_persist(const TcArgs& a0, const void* packA, const voi
   });
   if (attr_err[dev] != cudaSuccess) return attr_err[dev];
   TcArgs a = a0;
-  // two TMEM buffers of S levels, one exact K chunk per tile
-  if (a.S < 1 || a.S > TC_TILE128_MAX_S || a.kb_per_split > tc_chunk_kblocks(a.S)) return cudaErrorInvalidValue;
+  // two TMEM buffers of S levels, short K per tile
+  if (a.S < 1 || a.S > TC_PERSIST_MAX_S || a.kb_per_split > C::MAX_KB) return cudaErrorInvalidValue;
   int cols = 32;
   while (cols < 2 * a.S * C::BN) cols *= 2;
   a.tmem_cols = cols;
@@ -1796,9 +1487,8 @@ static cudaError_t launch_persist(const TcArgs& a0, const void* packA, const voi
 
 cudaError_t launch_ozaki(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st) {
   if (a.nb < 1 || a.nsplit < 1 || (long long)a.nsplit * a.kb_per_split < a.kblocks) return cudaErrorInvalidValue;
-  if (a.variant == 4) return launch_deep(a, packA, packB, st);
-  if (a.variant == 3) return launch_persist(a, packA, packB, st);
-  if (a.variant == 2) return launch_tile128(a, packA, packB, st);
+  if (a.variant == 3) return launch_deep(a, packA, packB, st);
+  if (a.variant == 2) return launch_persist(a, packA, packB, st);
   return a.variant == 1 ? launch_variant<TcNarrow>(a, packA, packB, st) : launch_variant<TcWide>(a, packA, packB, st);
 }
 

@@ -30,19 +30,7 @@ using TcWide = TcCfg<64, 8, 16, 1>;
 // two CTAs per SM (one's drain overlaps the other's MMAs): 32-wide tile, 5
 // stages, 8 drain warps; TMEM (S + 2) x 32 <= 256 columns, so S <= 5
 using TcNarrow = TcCfg<32, 5, 8, 2>;
-// 128-wide tile, one K chunk per CTA (no int64 partial sums): S x 128 <= 512
-// TMEM columns, so S <= 4.  Its ring holds single slices (one 128 x 64 tile
-// of A or of B, 16 KB, SWIZZLE_128B) in 12 slots, each with its own
-// barriers, so that a slice is released after its last product rather than
-// with the whole K block; 16 drain warps; one CTA per SM.
-struct TcTile128 {
-  static constexpr int BN = 128, STAGES = 12, EPI = 16, MINB = 1;
-  static constexpr int SLOT_BYTES = TC_BM * TC_BK * 2;  // 16 KB (A: 128 rows, B: BN = 128 rows)
-  static constexpr int THREADS = 64 + 32 * EPI;
-  // + 1 KB alignment and the barrier block
-  static constexpr int SMEM = 1024 + STAGES * SLOT_BYTES + 2048;
-};
-constexpr int TC_TILE128_MAX_S = 4;
+constexpr int TC_PERSIST_MAX_S = 4;
 
 // Persistent 64-column form for S <= 4 slices: one CTA per SM walks a list
 // of output tiles; S level accumulators of 64 columns make one TMEM buffer
@@ -53,6 +41,7 @@ constexpr int TC_TILE128_MAX_S = 4;
 // loading the next tile meanwhile).
 struct TcPersist {
   static constexpr int BN = 64, EPI = 16, MINB = 1;
+  static constexpr int MAX_KB = 2;                   // K blocks per tile
   static constexpr int RA = 5, RB = 6;               // ring slots of A and B slices
   static constexpr int A_SLOT = TC_BM * TC_BK * 2;   // 16 KB
   static constexpr int B_SLOT = BN * TC_BK * 2;      // 8 KB
@@ -60,13 +49,6 @@ struct TcPersist {
   static constexpr int THREADS = 64 + 32 * EPI;
   static constexpr int SMEM = 1024 + RA * A_SLOT + RB * B_SLOT + EPI * STAGE_WARP + 2048;
 };
-
-// K blocks one CTA of the 128-wide tile may accumulate exactly: the FP32
-// level sums grow by at most sum_{s+t=L} |q_s| |q_t| per K index (|q_1| <=
-// 128, |q_s| <= 64 for s >= 2) and must stay within 2^24.
-constexpr int tc_chunk_kblocks(int S) {
-  return S <= 2 ? 16 : S == 3 ? (1 << 24) / (20480 * 64) : (1 << 24) / (24576 * 64);
-}
 
 // Deep form (gemm_deep.cu): a 128 x BN tile whose S level accumulators fill
 // TMEM, a ring of (A, B) slice pairs, sums over K in the drain warps'
@@ -80,7 +62,7 @@ struct TcDeep {
   static constexpr int THREADS = 64 + 32 * EPI;
   static constexpr int TAIL = 2048;
   static constexpr int SMEM = 1024 + STAGES * (A_BYTES + B_BYTES) + TAIL;
-  static constexpr int CHUNK_KB = (1 << 24) / ((16384 + (S - 2) * 4096) * TC_BK);
+  static constexpr int CHUNK_KB = (1 << 24) / ((16384 + (S > 2 ? S - 2 : 0) * 4096) * TC_BK);
   static_assert(S * BN <= 512 && STAGES >= S, "TMEM columns, ring");
 };
 

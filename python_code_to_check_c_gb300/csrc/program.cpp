@@ -1027,12 +1027,8 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
       err_slot = e.slot;
     }
     const bool ac = op.dta == C64, bc = op.dtb == C64;
-    // S <= 4: the 128-column tile (one K chunk per CTA, K split across CTAs
-    // beyond it) when B has rows enough to fill it
     const long long nBrows = N * (bc ? 2 : 1);
-    const bool tile128 = S <= TC_TILE128_MAX_S && nBrows >= 96;
-    const long long rA = rup(M * (ac ? 2 : 1), BM), rB = rup(nBrows, tile128 ? TcTile128::BN : BN),
-                    Kp = rup(K, BK);
+    const long long rA = rup(M * (ac ? 2 : 1), BM), rB = rup(nBrows, BN), Kp = rup(K, BK);
     // batched products: an operand with a batch stride is packed per batch
     const int nbt = std::max(op.g.nb, 1);
     const int nbA = (nbt > 1 && op.g.bsA != 0) ? nbt : 1, nbB = (nbt > 1 && op.g.bsB != 0) ? nbt : 1;
@@ -1168,30 +1164,25 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     }
     a.acc = op.g.acc;
     // S <= 4 and at most two K blocks: the persistent 64-column form, whose
-    // TMEM drain runs under the next tile's loads and MMAs (measured at o=10,
-    // v=38 with 24 trajectories: 10-35 % faster than the 128-column tile for
-    // one or two K blocks, 30-50 % slower for six or more, where the
-    // 128-column tile's MMA rate and operand reuse count)
-    const bool persist = S <= TC_TILE128_MAX_S && a.kblocks <= 2;
-    // S = 4, 5 and longer K: the deep form, which sums all of K in one CTA.
-    // Against the 128-column tile (S = 4, o=10, v=38, 24 trajectories) 210 us
-    // for 335 on the ladder (23 blocks), 174 for 222 on the ring terms (6); against
-    // the 64-column tile (S = 5, o=18, v=82) 829 for 1842 (106 blocks), 420 for
-    // 890 (24).  A B side of less than 3/4 of a tile keeps the narrower ones.
+    // TMEM drain runs under the next tile's loads and MMAs
+    const bool persist = S <= TC_PERSIST_MAX_S && a.kblocks <= TcPersist::MAX_KB;
+    // S <= 5 and longer K: the deep form, which sums all of K in one CTA.
+    // Against 128-column tiles over split K (S = 4, o=10, v=38, 24
+    // trajectories) 210 us for 335 on the ladder (23 blocks), 174 for 190 on
+    // the ring terms (6); against the 64-column tile (S = 5, o=18, v=82) 829
+    // for 1842 (106 blocks), 420 for 892 (24).  A B side of less than 3/4 of a
+    // tile keeps the 64-column tile.
     const int deepBN = S == 5 ? 96 : 128;
-    const bool long_k = !deep && (S == 4 || S == 5) && a.kblocks > 2 && nBrows >= deepBN * 3 / 4;
+    const bool long_k = !deep && S <= 5 && a.kblocks > 2 && nBrows >= deepBN * 3 / 4;
     // split K so that few output tiles still occupy the SMs: one CTA per SM,
-    // cost = waves x (K blocks per CTA + fixed pipeline/epilogue overhead);
-    // the 128-column tile takes at most one exact K chunk per CTA
-    const int tileN = long_k ? deepBN : tile128 && !persist ? TcTile128::BN : BN;
+    // cost = waves x (K blocks per CTA + fixed pipeline/epilogue overhead)
+    const int tileN = long_k ? deepBN : BN;
     const long long ctas = (((long_k ? nBrows : rB) + tileN - 1) / tileN) * (rA / BM) * nbt;
-    const long long min_sp =
-        !long_k && (tile128 || persist) ? (a.kblocks + tc_chunk_kblocks(S) - 1) / tc_chunk_kblocks(S) : 1;
-    long long splits = min_sp;
+    long long splits = 1;
     {
       double best = 1e300;
-      const long long maxs = std::max<long long>(min_sp, std::min<long long>(a.kblocks, 64));
-      for (long long sp = min_sp; sp <= maxs; ++sp) {
+      const long long maxs = std::min<long long>(a.kblocks, 64);
+      for (long long sp = 1; sp <= maxs; ++sp) {
         const long long waves = (ctas * sp + 151) / 152;
         const long long per = (a.kblocks + sp - 1) / sp;
         const double cost = (double)waves * (double)(per * S + (long_k ? 12 : 6));
@@ -1208,7 +1199,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     a.atomic = splits > 1 ? 1 : 0;
     t.zeroed = a.acc || a.atomic;  // split K is allowed (a zero op precedes when not accumulating)
     // short K: the narrow variant (two CTAs per SM overlap their latencies)
-    a.variant = deep || long_k ? 4 : persist ? 3 : tile128 ? 2 : (a.kb_per_split == 1 && S <= 5) ? 1 : 0;
+    a.variant = deep || long_k ? 3 : persist ? 2 : (a.kb_per_split == 1 && S <= 5) ? 1 : 0;
     t.bytes = (long long)S * (nbA * rA + nbB * rB) * Kp * 2 + nbt * M * N * elem_bytes(op.dtc);
     t.reads = {pa.pk_dst, pb.pk_dst};
     if (deep) {  // the drain reads the operands of rows that digits cannot hold

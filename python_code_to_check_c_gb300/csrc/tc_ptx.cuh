@@ -6,6 +6,8 @@
 
 #include <cstdint>
 
+#include "gemm_tc.h"
+
 namespace tdcc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -128,6 +130,69 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 }
 
 constexpr int kWaitLimit = 1 << 22;
+
+// The MMA warp's side of a ring of slice pairs (A_j, B_j): the products of one
+// K block with s + t <= S + 1 into the accumulators of their levels, BN columns
+// each.  Step j runs the products that pair j completes; a pair is released
+// after its last product.  Slots and descriptor words are computed once per
+// slice (per product they cost more than the products: the FP64 form's ladder
+// at o=10, v=38 took 90 us so, 75 with them hoisted).
+template <int STAGES, int A_BYTES, int B_BYTES>
+struct PairRing {
+  uint64_t hi64;
+  uint32_t a0, b0, full0, empty0;
+  uint32_t st0 = 0, ph = 0;  // ring slot and phase of the block's first pair
+  __device__ __forceinline__ PairRing(const uint8_t* stA, const uint8_t* stB, const uint64_t* full, const uint64_t* empty)
+      : hi64(sdesc(0)),
+        a0((smem_u32(stA) & 0x3FFFF) >> 4),
+        b0((smem_u32(stB) & 0x3FFFF) >> 4),
+        full0(smem_u32(full)),
+        empty0(smem_u32(empty)) {}
+  // `first`: the block starts the sums.  False when a wait expired.
+  template <int S, int BN>
+  __device__ __forceinline__ bool issue(uint32_t tmem, uint32_t id, bool first, uint32_t on) {
+    static_assert(S <= STAGES, "the ring holds one K block's slices");
+    uint32_t la[S], lb[S], slot[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      slot[j] = st0 + j < STAGES ? st0 + j : st0 + j - STAGES;
+      la[j] = a0 + slot[j] * (A_BYTES >> 4);
+      lb[j] = b0 + slot[j] * (B_BYTES >> 4);
+    }
+    bool ok = true;
+#pragma unroll
+    for (int j = 1; j <= S; ++j) {
+      if (ok) ok = mbar_wait_warp(full0 + 8 * slot[j - 1], st0 + j - 1 < STAGES ? ph : ph ^ 1u, kWaitLimit);
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      if (ok) {
+        auto product = [&](int s, int t) {
+          const bool lead = s == t || s == t + 1;  // the first product of its level in a block
+#pragma unroll
+          for (int k = 0; k < TC_BK / 16; ++k)
+            umma_warp(tmem + (uint32_t)((s + t - 2) * BN), hi64 | (uint64_t)(la[s - 1] + 2 * k),
+                      hi64 | (uint64_t)(lb[t - 1] + 2 * k), id, (lead && k == 0 && first) ? 0u : 1u, on);
+        };
+        const int last = S + 1 - j;  // largest partner of slice j
+#pragma unroll
+        for (int t = 1; t <= S; ++t)
+          if (t <= j && t <= last) product(j, t);
+#pragma unroll
+        for (int q = 1; q <= S; ++q)
+          if (q < j && q <= last) product(q, j);
+        if (j >= last) {  // pairs j and S + 1 - j have had their last use
+          umma_commit_warp(empty0 + 8 * slot[j - 1], on);
+          if (j > last) umma_commit_warp(empty0 + 8 * slot[last - 1], on);
+        }
+      }
+    }
+    st0 += S;
+    if (st0 >= STAGES) {
+      st0 -= STAGES;
+      ph ^= 1u;
+    }
+    return ok;
+  }
+};
 
 // records an expired wait: every role of the CTA stops
 template <class SH>
