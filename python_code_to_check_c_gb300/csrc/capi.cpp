@@ -2,7 +2,9 @@
 #include <cmath>
 #include <cstring>
 #include <initializer_list>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -233,6 +235,49 @@ long long deep_budget() {
   }
   return (long long)(fr / 6);
 }
+
+// Scratch of a call without a system, from a pool of the library's own per
+// device.  The device's default pool gives everything back at each
+// synchronisation, so a call paid for mapping its memory anew (300 of the 370 us
+// of a 2000-step spectrum); this one keeps up to 64 MB.  Stream-ordered: several
+// threads and streams may use it; `p` stays null where there is no memory.
+struct Scratch {
+  void* p = nullptr;
+  cudaStream_t st = nullptr;
+  void get(size_t bytes, cudaStream_t stream) {
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    st = stream;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    cudaMemPool_t pool = nullptr;
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      auto it = pools.find(dev);
+      if (it == pools.end()) {
+        cudaMemPoolProps pr{};
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = dev;
+        unsigned long long keep = 64ull << 20;
+        if (cudaMemPoolCreate(&pool, &pr) != cudaSuccess) {
+          cudaGetLastError();
+          return;
+        }
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        it = pools.emplace(dev, pool).first;
+      }
+      pool = it->second;
+    }
+    if (cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~Scratch() {
+    if (p) cudaFreeAsync(p, st);
+  }
+};
 
 ProgInst& get_rhs(tdcc_system s, int method, int block) {
   auto& slot = s->rhs[method][block];
@@ -1697,9 +1742,68 @@ int tdcc_tei_from_df(const double* B, int n, int nq, double* tei, void* stream) 
     g.ai = 0.0;
     g.acc = 0;
     g.nb = 1;
-    Program::plan_gemm(op, false);
-    CK(launch_gemm(op, B, B, tei, st));
-    CK(launch_tei_antisym(tei, n, st));
+    // The two operands are one matrix of n^2 rows: packed once, and the product
+    // is symmetric, so the tensor cores do the tiles on and above its diagonal
+    // (5 us to pack, 32 us a wave of 152 tiles at K = 144; the fixed-point tiles
+    // do 4.3 multiply-adds a clock and SM).  n = 48, K = 144: 526 -> 146 us in
+    // all.  Short of scratch, or inside a capture, the fixed-point tiles.
+    const double kb = std::ceil(nq / 64.0), half = 0.5 * std::ceil(n2 / 128.0) * (std::ceil(n2 / 64.0) + 1.0);
+    const double t_deep = 12.0 + std::ceil(half / 152.0) * (kb * 6.5 + 13.0);
+    const double t_fx = 6.0 + (double)n2 * n2 * nq / (152.0 * 4.3 * 2070.0);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cap));
+    const long long rows = (n2 + 127) / 128 * 128, kpad = (nq + 63) / 64 * 64LL;
+    const long long exp_off = (long long)TC_DEEP_SLICES * rows * kpad * 2, need = exp_off + rows * 4 + 256;
+    Scratch w;
+    if (nq >= 32 && t_deep < 0.85 * t_fx && cap == cudaStreamCaptureStatusNone && need <= deep_budget()) w.get((size_t)need, st);
+    if (w.p) {
+      char* base = static_cast<char*>(w.p);
+      int* err = reinterpret_cast<int*>(base + exp_off + rows * 4);
+      CK(cudaMemsetAsync(base + exp_off, 0, (size_t)(rows * 4 + 256), st));
+      PackArgs pk{};
+      pk.src = B;
+      pk.gr = g.gm;
+      pk.gk = g.gk;
+      pk.rows = g.M;
+      pk.K = nq;
+      pk.rows_pad = (int)rows;
+      pk.K_pad = (int)kpad;
+      pk.S = TC_DEEP_SLICES;
+      pk.nb = 1;
+      pk.out = base;
+      pk.exps = reinterpret_cast<int*>(base + exp_off);
+      TcArgs a{};
+      a.M = a.N = g.M;
+      a.rowsA_pad = a.rowsB_pad = (int)rows;
+      a.nb = a.nsplit = 1;
+      a.variant = 3;
+      a.kblocks = a.kb_per_split = (int)(kpad / 64);
+      a.S = TC_DEEP_SLICES;
+      a.expA = a.expB = pk.exps;
+      a.gmC = g.gm;
+      a.gnC = g.gn;
+      for (int i = 0; i < 2; ++i) {
+        a.gmC.s0[i] = g.gm.s1[i];
+        a.gnC.s0[i] = g.gn.s1[i];
+      }
+      a.C = tei;
+      a.ar = 1.0;
+      a.alpha_pow2 = 1;
+      a.err = err;
+      a.srcA = a.srcB = B;
+      a.gmA = g.gm;
+      a.gnB = g.gn;
+      a.gkAB = g.gk;
+      a.K = nq;
+      a.sym = 1;
+      CK(launch_pack(pk, st));
+      CK(launch_ozaki(a, base, base, st));
+      CK(launch_tei_antisym(tei, n, err, st));
+    } else {
+      Program::plan_gemm(op, false);
+      CK(launch_gemm(op, B, B, tei, st));
+      CK(launch_tei_antisym(tei, n, nullptr, st));
+    }
   } catch (const std::exception& ex) {
     return fail(TDCC_ERR_CUDA, ex.what());
   }

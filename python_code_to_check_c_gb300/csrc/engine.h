@@ -176,6 +176,7 @@ struct TcArgs {
   ModeGroup gmA, gnB, gkAB;  // offsets in s0 (A / B); gkAB: A in s0, B in s1
   long long bsA, bsB;
   int K;
+  int sym;  // deep form, real, B is A: tiles on and above the diagonal only, each stored both ways
 };
 
 // GB_SIMT: exact BF16-digit slice products on the FP32 pipe for short

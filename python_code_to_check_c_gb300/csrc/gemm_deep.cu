@@ -56,6 +56,7 @@ struct DeepShared {
   volatile int abort;
   long long col_off[C::BN];  // output offset of each logical column (-1: outside)
   int col_exp[C::BN];        // stored exponent of each packed column of B
+  long long col_offT[C::S > 5 ? C::BN : 1];  // offset of each column as a row (symmetric products)
 };
 
 // sum over k in [k0, k1) of A[m, k] B[k, n] of batch z, operands as they are
@@ -118,9 +119,12 @@ __global__ void __launch_bounds__(C::THREADS, 1)
   const uint32_t tmem = sh->tmem;
 
   const int mt = g.m_fast ? blockIdx.x : blockIdx.y, nt = g.m_fast ? blockIdx.y : blockIdx.x;
+  constexpr bool SYM = !AC && !BC && S > 5;
+  // a symmetric product's tile below the diagonal comes from its mirror image
+  const bool skip = SYM && g.sym && (nt + 1) * C::BN <= mt * TC_BM;
   const int zb = blockIdx.z / g.nsplit;
   const int kb0 = (blockIdx.z - zb * g.nsplit) * g.kb_per_split;
-  const int kb1 = min(g.kblocks, kb0 + g.kb_per_split);
+  const int kb1 = skip ? kb0 : min(g.kblocks, kb0 + g.kb_per_split);
   const int rowA0 = g.bat_a ? zb * g.rowsA_pad : 0, rowB0 = g.bat_b ? zb * g.rowsB_pad : 0;
   const int nchunks = (kb1 - kb0 + C::CHUNK_KB - 1) / C::CHUNK_KB;
 
@@ -179,6 +183,10 @@ __global__ void __launch_bounds__(C::THREADS, 1)
         long long o = -1;
         if (n < g.N) decomp_tc(g.gnC, n, o);
         sh->col_off[t] = o;
+        if constexpr (SYM) {
+          if (g.sym && n < g.N) decomp_tc(g.gmC, n, o);
+          sh->col_offT[t] = o;
+        }
       }
       // the last tile may reach beyond the packed rows (its loads read zeros
       // or the next batch there; those columns are not stored)
@@ -227,7 +235,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       asm volatile("tcgen05.fence::before_thread_sync;");
       mbar_arrive(smem_u32(&sh->accempty));
     }
-    if (ok && __any_sync(0xffffffffu, sh->abort != 0)) ok = false;
+    if (skip || (ok && __any_sync(0xffffffffu, sh->abort != 0))) ok = false;
     if (ok) {
       const bool odd = AC && (lane & 1);
       constexpr int GC = NC > 24 ? NC / 2 : NC;  // packed columns staged at a time
@@ -244,6 +252,8 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       const int ebase = row_exp(ea) - 7 * (S + 1) + (g.alpha_pow2 ? g.alpha_e : 0);
       long long coffm = 0;
       if (m < g.M) decomp_tc(g.gmC, m, coffm);
+      long long coffT = 0;  // this row as a column
+      if (SYM && g.sym && m < g.M) decomp_tc(g.gnC, m, coffT);
       double2* Cc = static_cast<double2*>(g.C) + (g.cc ? zb * g.bsC : 0);
       double* Cr = static_cast<double*>(g.C) + (g.cc ? 0 : zb * g.bsC);
       const int m0w = AC ? ((mt * TC_BM + q * 32) >> 1) : (mt * TC_BM + q * 32);
@@ -305,6 +315,14 @@ __global__ void __launch_bounds__(C::THREADS, 1)
           stage[lr * RS + k] = v;
         }
         __syncwarp();
+        if constexpr (SYM) {  // the mirror image: lanes along the rows, which are its columns
+          if (g.sym && lane < nrows)
+#pragma unroll 4
+            for (int k = 0; k < NL; ++k) {
+              const long long cT = sh->col_offT[j0 + g0 + k];
+              if (cT >= 0) Cr[cT + coffT] = stage[lane * RS + k].x;
+            }
+        }
         // every lane owns a (row, column) pair per pass
 #pragma unroll 4
         for (int i = lane; i < rows_out * NL; i += 32) {
@@ -356,6 +374,8 @@ cudaError_t launch_deep_form(const TcArgs& a0, const void* packA, const void* pa
   });
   if (attr_err[dev] != cudaSuccess) return attr_err[dev];
   TcArgs a = a0;
+  if (a.sym && (C::S <= 5 || a.ac || a.bc || a.cc || a.acc || a.atomic || a.nb != 1 || a.M != a.N || packA != packB))
+    return cudaErrorInvalidValue;
   if (a.S != C::S || a.rowsB_pad < 1 || a.rowsA_pad % TC_BM != 0) return cudaErrorInvalidValue;
   a.tmem_cols = 512;
   const CUtensorMap ma = slice_map(packA, a.S, (a.bat_a ? a.nb : 1) * a.rowsA_pad, a.kblocks * TC_BK, TC_BM);

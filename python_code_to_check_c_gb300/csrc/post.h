@@ -4,8 +4,9 @@
 
 namespace tdcc {
 
-// X[p,q,r,s] (= (pr|qs)) <- X[p,q,r,s] - X[p,q,s,r], in place, n^4 doubles
-cudaError_t launch_tei_antisym(double* X, int n, cudaStream_t st);
+// X[p,q,r,s] (= (pr|qs)) <- X[p,q,r,s] - X[p,q,s,r], in place, n^4 doubles;
+// all NaN where *err (may be null) is set
+cudaError_t launch_tei_antisym(double* X, int n, const int* err, cudaStream_t st);
 
 // shifted DFTs of Re mu and Im mu (mu[n * stride], n < N); tw: N scratch
 // entries (the twiddles exp(-2 pi i r / N))

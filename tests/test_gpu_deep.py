@@ -115,3 +115,38 @@ def test_long_contractions_of_the_mixed_form(o, v, nb, S, tol):
         eng.check_errors()
     finally:
         eng.close()
+
+
+def _plain_integrals(B):
+    x = np.einsum("Qpr,Qqs->pqrs", B.astype(np.longdouble), B.astype(np.longdouble), optimize=False)
+    return x - x.transpose(0, 1, 3, 2)
+
+
+@pytest.mark.parametrize("n,nq,bad", [(30, 200, None), (33, 100, None), (40, 65, None), (33, 70, np.inf), (32, 130, 5e-324)])
+def test_integrals_from_one_packing(n, nq, bad):
+    """The symmetric product of the integrals: ragged tiles, the diagonal tiles,
+    rows that digits cannot hold; eager and captured (fixed-point tiles) alike."""
+    import torch
+
+    from python_code_to_check_c_gb300.engine import tei_from_df_device
+    B = np.random.default_rng(n * 1000 + nq).standard_normal((nq, n, n))
+    # per product 2^-56 of either maximum for the operands' digits and the levels left out, 2^-53 of the sum
+    m = np.abs(B).max()
+    tol = 2 * (nq * 3 * 2.0**-56 * m * m + (1 + nq // 60) * 2.0**-53 * nq * m * m)
+    if bad is not None:
+        B[:, 3, 5] = 0.0
+        B[1, 3, 5] = bad
+    with np.errstate(all="ignore"):
+        ref = _plain_integrals(B)
+    ref[..., np.arange(n), np.arange(n)] = 0.0
+    Bd = torch.as_tensor(B, device="cuda")
+    got = tei_from_df_device(Bd).cpu().numpy()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = tei_from_df_device(Bd)
+    g.replay()
+    for x in (got, out.cpu().numpy()):
+        ok = np.isfinite(ref)
+        assert np.array_equal(np.isfinite(x), ok)
+        assert np.abs(x[ok] - ref[ok]).max() <= tol
+        assert np.array_equal(x[ok], -x.transpose(0, 1, 3, 2)[ok])
