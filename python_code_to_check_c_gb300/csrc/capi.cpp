@@ -1817,13 +1817,16 @@ int tdcc_spectrum(const void* mu, long long nsteps, long long stride, double dt,
   if (!(dt > 0.0)) return fail(TDCC_ERR_ARG, "dt must be > 0");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   try {
-    void* tw = nullptr;
-    CK(cudaMallocAsync(&tw, (size_t)nsteps * 16, st));
-    const cudaError_t e = launch_spectrum(static_cast<const double2*>(mu), nsteps, stride,
-                                          static_cast<double2*>(tw), static_cast<double2*>(Yr),
-                                          static_cast<double2*>(Yi), st);
-    cudaFreeAsync(tw, st);
-    CK(e);
+    Scratch w;  // the twiddles
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cap));
+    if (cap == cudaStreamCaptureStatusNone) w.get((size_t)nsteps * 16, st);
+    if (!w.p) {  // a node of the graph's own, or the last resort
+      CK(cudaMallocAsync(&w.p, (size_t)nsteps * 16, st));
+      w.st = st;
+    }
+    CK(launch_spectrum(static_cast<const double2*>(mu), nsteps, stride, static_cast<double2*>(w.p),
+                       static_cast<double2*>(Yr), static_cast<double2*>(Yi), st));
     if (energy_ev)
       for (long long j = 0; j < nsteps; ++j)
         energy_ev[j] = (double)(j - nsteps / 2) / ((double)nsteps * dt) * (2.0 * M_PI) * 27.211;

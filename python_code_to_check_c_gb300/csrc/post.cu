@@ -64,66 +64,76 @@ __global__ void twiddle_kernel(double2* __restrict__ tw, long long N) {
   }
 }
 
-// One block per output position j of the shifted spectra: frequency index
-// k = (j + N - N/2) mod N; Yr[j] = sum_n Re mu[n] tw[k n mod N], Yi likewise
-// with Im mu.
+// Frequencies k = 0 .. N/2 of the transforms of the two real sequences Re mu and
+// Im mu; those of N - k are their conjugates.  64 threads per frequency, each
+// with four partial sums of every 256th term.  Bound: the FP64 pipe (8 N^2/2
+// operations, 14 us at N = 2000) and the table's reads.  A block of 256 threads
+// per frequency, all N of them, spent 160 of its 416 FP64 instructions per
+// warp-column on shuffle sums: 58 us; this form adds in the same depth with a
+// sixth of them and does half the frequencies (a call of 7934 samples 835 ->
+// 333 us, one of 2000, with its scratch no longer mapped anew, 376 -> 108).
+constexpr int kSpecLanes = 64;
 __global__ void __launch_bounds__(256) spectrum_kernel(const double2* __restrict__ mu, long long N, long long stride,
                                                        const double2* __restrict__ tw, double2* __restrict__ Yr,
                                                        double2* __restrict__ Yi) {
-  const long long j = blockIdx.x;
-  const long long k = (j + N - N / 2) % N;
-  const long long step = (k * (long long)blockDim.x) % N;
-  long long r = (k * (long long)threadIdx.x) % N;
-  double rr = 0.0, ri = 0.0, ir = 0.0, ii = 0.0;
-  for (long long nn = threadIdx.x; nn < N; nn += blockDim.x) {
-    const double2 m = mu[nn * stride];
-    const double2 w = tw[r];
-    rr = fma(m.x, w.x, rr);
-    ri = fma(m.x, w.y, ri);
-    ir = fma(m.y, w.x, ir);
-    ii = fma(m.y, w.y, ii);
-    r += step;
-    if (r >= N) r -= N;
+  constexpr int L = kSpecLanes, Q = 256 / L;
+  const int t = threadIdx.x % L, q = threadIdx.x / L;
+  const long long k = (long long)blockIdx.x * Q + q;
+  double rr[4] = {}, ri[4] = {}, ir[4] = {}, ii[4] = {};
+  if (k <= N / 2) {
+    const long long step = (k * L) % N;
+    long long r = (k * t) % N;
+    for (long long n0 = t; n0 < N; n0 += 4 * L)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const long long n = n0 + u * L;
+        if (n < N) {
+          const double2 m = mu[n * stride];
+          const double2 w = tw[r];
+          rr[u] = fma(m.x, w.x, rr[u]);
+          ri[u] = fma(m.x, w.y, ri[u]);
+          ir[u] = fma(m.y, w.x, ir[u]);
+          ii[u] = fma(m.y, w.y, ii[u]);
+          r += step;
+          if (r >= N) r -= N;
+        }
+      }
   }
-  for (int d = 16; d > 0; d >>= 1) {
-    rr += __shfl_down_sync(0xffffffffu, rr, d);
-    ri += __shfl_down_sync(0xffffffffu, ri, d);
-    ir += __shfl_down_sync(0xffffffffu, ir, d);
-    ii += __shfl_down_sync(0xffffffffu, ii, d);
-  }
-  __shared__ double red[4][8];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) {
-    red[0][w] = rr;
-    red[1][w] = ri;
-    red[2][w] = ir;
-    red[3][w] = ii;
+  double v[4] = {(rr[0] + rr[1]) + (rr[2] + rr[3]), (ri[0] + ri[1]) + (ri[2] + ri[3]),
+                 (ir[0] + ir[1]) + (ir[2] + ir[3]), (ii[0] + ii[1]) + (ii[2] + ii[3])};
+  __shared__ double red[256 / 32][4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    for (int d = 16; d > 0; d >>= 1) v[p] += __shfl_down_sync(0xffffffffu, v[p], d);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][p] = v[p];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-      a += red[0][q];
-      b += red[1][q];
-      c += red[2][q];
-      d += red[3][q];
+  if (t == 0 && k <= N / 2) {
+    const int w = threadIdx.x >> 5;
+    const double2 a = make_double2(red[w][0] + red[w + 1][0], red[w][1] + red[w + 1][1]);
+    const double2 b = make_double2(red[w][2] + red[w + 1][2], red[w][3] + red[w + 1][3]);
+    const long long j = (k + N / 2) % N, j2 = (N - k + N / 2) % N;  // shifted positions of k and N - k
+    Yr[j] = a;
+    Yi[j] = b;
+    if (j2 != j) {
+      Yr[j2] = make_double2(a.x, -a.y);
+      Yi[j2] = make_double2(b.x, -b.y);
     }
-    Yr[j] = make_double2(a, b);
-    Yi[j] = make_double2(c, d);
   }
 }
 
 cudaError_t launch_spectrum(const double2* mu, long long N, long long stride, double2* tw, double2* Yr, double2* Yi,
                             cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
-  long long tb = (N + 255) / 256;
-  if (tb > 152LL * 8) tb = 152LL * 8;
-  twiddle_kernel<<<(unsigned)tb, 256, 0, st>>>(tw, N);
+  if (N > 0x7fffffffLL) return cudaErrorInvalidValue;
+  long long tb = (N + 63) / 64;
+  if (tb > 152LL * 16) tb = 152LL * 16;
+  twiddle_kernel<<<(unsigned)tb, 64, 0, st>>>(tw, N);
   count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (N > 0x7fffffffLL) return cudaErrorInvalidValue;
-  spectrum_kernel<<<(unsigned)N, 256, 0, st>>>(mu, N, stride, tw, Yr, Yi);
+  constexpr int Q = 256 / kSpecLanes;
+  spectrum_kernel<<<(unsigned)((N / 2 + 1 + Q - 1) / Q), 256, 0, st>>>(mu, N, stride, tw, Yr, Yi);
   count_launch();
   return cudaGetLastError();
 }

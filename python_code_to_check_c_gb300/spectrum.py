@@ -29,12 +29,12 @@ def spectrum(mu, dt: float):
     if mu.dim() != 1:
         raise ValueError("mu must be one-dimensional (one entry per step)")
     n = int(mu.shape[0])
-    Yr = torch.empty(n, dtype=torch.complex128, device=mu.device)
-    Yi = torch.empty_like(Yr)
+    Y = torch.empty((2, n), dtype=torch.complex128, device=mu.device)
     e = np.zeros(n)
-    check(lib.tdcc_spectrum(_ptr(mu), n, int(mu.stride(0)), float(dt), _ptr(Yr), _ptr(Yi),
+    check(lib.tdcc_spectrum(_ptr(mu), n, int(mu.stride(0)), float(dt), _ptr(Y[0]), _ptr(Y[1]),
                             e.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), _stream()), "tdcc_spectrum")
-    return e, Yr.cpu().numpy(), Yi.cpu().numpy()
+    Yr, Yi = Y.cpu().numpy()  # one copy for both
+    return e, Yr, Yi
 
 
 def read_trajectory(path: str = "H2O.csv"):
