@@ -817,10 +817,18 @@ int tdcc_ground_state(tdcc_system s, int method, int mode, void* t1, void* t2, v
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int o = s->dims.o, v = s->dims.v, n = s->dims.n;
     const long long n1 = (long long)o * v, n2 = n1 * n1;
+    const int ns = maxsize + 2, ne = maxsize + 1;
+    constexpr int kEn = 2 * kSumParts;  // an energy's parts, then the dot products' parts
+    // one allocation for all vectors (one each cost 50 of them, and as many frees)
+    auto pad = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t b1 = pad((size_t)n1 * sizeof(double2)), b2 = pad((size_t)n2 * sizeof(double2));
+    char* next = nullptr;
+    CK(cudaMalloc(&next, pad((size_t)n * sizeof(double)) + pad((size_t)n * n * sizeof(double2)) +
+                             (3 + ns + ne) * (b1 + b2) + pad((size_t)(kEn + 64 * kSumParts) * sizeof(double2))));
+    mem.push_back(next);
     auto alloc = [&](size_t bytes) {
-      void* p = nullptr;
-      CK(cudaMalloc(&p, bytes));
-      mem.push_back(p);
+      void* p = next;
+      next += pad(bytes);
       return p;
     };
     auto c2 = [&](long long cnt) { return static_cast<double2*>(alloc((size_t)cnt * sizeof(double2))); };
@@ -829,8 +837,7 @@ int tdcc_ground_state(tdcc_system s, int method, int mode, void* t1, void* t2, v
     double2* Fc = c2((long long)n * n);
     CK(g_to_complex(Fc, s->fock, (long long)n * n, st));
     double2 *r1 = c2(n1), *r2 = c2(n2), *x1 = c2(n1), *x2 = c2(n2), *o1 = c2(n1), *o2 = c2(n2);
-    double2* res = c2(64);
-    const int ns = maxsize + 2, ne = maxsize + 1;
+    double2* res = c2(kEn + 64 * kSumParts);
     std::vector<double2*> S1(ns), S2(ns), E1(ne), E2(ne);
     for (int k = 0; k < ns; ++k) {
       S1[k] = c2(n1);
@@ -864,21 +871,30 @@ int tdcc_ground_state(tdcc_system s, int method, int mode, void* t1, void* t2, v
       rhs(P1, r1);
       rhs(P2, r2);
       if (r_tol > 0.0) {
-        double2 h;
-        CK(g_maxabs(r1, n1, r2, n2, res + 63, st));
-        CK(cudaMemcpyAsync(&h, res + 63, sizeof(h), cudaMemcpyDeviceToHost, st));
+        double2 h[kSumParts];
+        CK(g_maxabs(r1, n1, r2, n2, res, st));
+        CK(cudaMemcpyAsync(h, res, sizeof(h), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        last_res = h.x;
+        last_res = 0.0;
+        for (const double2& x : h) last_res = std::fmax(last_res, x.x);
       }
       CK(g_jacobi(x1, r1, eps, o, v, 2, n1, st));
       CK(g_jacobi(x2, r2, eps, o, v, 4, n2, st));
     };
+    auto energy_sum = [&](const double2* h) {
+      double a = 0.0, b = 0.0;
+      for (int p = 0; p < kSumParts; ++p) {
+        a += h[2 * p].x;
+        b += h[2 * p + 1].x;
+      }
+      return a + b;
+    };
     auto energy_of = [&]() {
-      double2 h[2];
+      double2 h[kEn];
       CK(g_energy(s->tei, s->fock, x1, x2, o, v, mode, res, st));
       CK(cudaMemcpyAsync(h, res, sizeof(h), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
-      return h[0].x + h[1].x;
+      return energy_sum(h);
     };
     // buffer bookkeeping for the rolling stores (front = oldest)
     std::vector<int> s1q, s2q, e1q, e2q, s1free, s2free, efree;
@@ -925,7 +941,8 @@ int tdcc_ground_state(tdcc_system s, int method, int mode, void* t1, void* t2, v
     double E = 0.0;
     int it = 0;
     for (int z = 1; z < maxiter; ++z) {
-      const double e_old = energy_of();
+      double e_old = 0.0;  // read back with the first dot products
+      CK(g_energy(s->tei, s->fock, x1, x2, o, v, mode, res, st));
       // B[a][b] = <e_b, e_a> (t1 part + t2 part), symmetric
       std::vector<std::pair<int, int>> pairs;
       for (int a = 0; a < maxsize; ++a)
@@ -943,13 +960,19 @@ int tdcc_ground_state(tdcc_system s, int method, int mode, void* t1, void* t2, v
           dp.n[2 * q + 1] = n2;
         }
         dp.count = (int)(2 * cnt);
-        CK(g_dots(dp, res, st));
-        std::vector<double2> h(2 * cnt);
+        CK(g_dots(dp, res + kEn, st));
+        std::vector<double2> h(kEn + 2 * cnt * kSumParts);
         CK(cudaMemcpyAsync(h.data(), res, h.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (p0 == 0) e_old = energy_sum(h.data());
+        auto dot = [&](size_t q) {
+          double x = 0.0;
+          for (int p = 0; p < kSumParts; ++p) x += h[kEn + q * kSumParts + p].x;
+          return x;
+        };
         for (size_t q = 0; q < cnt; ++q) {
           const int a = pairs[p0 + q].first, b = pairs[p0 + q].second;
-          const double val = h[2 * q].x + h[2 * q + 1].x;
+          const double val = dot(2 * q) + dot(2 * q + 1);
           Bm[a * m1 + b] = val;
           Bm[b * m1 + a] = val;
         }
