@@ -614,10 +614,12 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 // are in registers, before they convert and store -- so a tile's drain runs
 // under the next tile's loads and MMAs.  A and B slices have rings of their
 // own (A1 .. AS and B1 .. BS per K block, products row by row, each slice
-// released after its last product).  Bound: the drain, 11 k to 20 k clocks a
-// tile against 5 k a K block for loads and products; accumulated outputs are
-// reductions in L2 (as loads and stores the o=10, v=38 contractions of 24
-// trajectories took 180 us instead of 150).
+// released after its last product).  Bound: the drain; as one group of 16 warps,
+// all in the same phase of it, it took 11 k to 20 k clocks a tile against 5 k a
+// K block for loads and products.  Two groups of eight, a buffer each: the o=10,
+// v=38 contractions of 24 trajectories with mnij 160 -> 119 us, with the 38 x 38
+// intermediates 158 -> 98.  Accumulated outputs are reductions in L2: as loads
+// and stores the former took 180 us.
 // ---------------------------------------------------------------------------
 struct PersistShared {
   uint64_t fullA[TcPersist::RA], emptyA[TcPersist::RA];
@@ -625,10 +627,12 @@ struct PersistShared {
   uint64_t accfull[2], accempty[2], done;
   uint32_t tmem;
   volatile int abort;
-  int stop;                                 // the drain warps' common decision for a tile
-  long long col_off[TcPersist::BN / 1];     // output offset of each logical column (-1: outside)
-  int col_exp[TcPersist::BN];
+  int stop[2];                              // each drain group's common decision for a tile
+  long long col_off[2][TcPersist::BN];      // output offset of each logical column (-1: outside)
+  int col_exp[2][TcPersist::BN];
 };
+
+static_assert(sizeof(PersistShared) <= 2048, "fits behind the staging areas");
 
 struct TileCoord {
   int mt, nt, zb, kb0, kb1, rowA0, rowB0;
@@ -762,11 +766,11 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&sh->accfull[b]), 1);
-      mbar_init(smem_u32(&sh->accempty[b]), 32 * C::EPI);
+      mbar_init(smem_u32(&sh->accempty[b]), 32 * C::EPI / 2);
     }
     mbar_init(smem_u32(&sh->done), 1);
     sh->abort = 0;
-    sh->stop = 0;
+    sh->stop[0] = sh->stop[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
     asm volatile("fence.proxy.async.shared::cta;");
   }
@@ -827,12 +831,14 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
       default: persist_issue<4>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
     }
   } else {
-    // ---------------- drain warps (2 .. 17): 16 columns each ----------------
-    const int q = warp & 3;
-    const int j0 = ((warp - 2) >> 2) * 16;  // this warp's packed columns
+    // ---------------- drain warps (2 .. 17): two groups of eight ----------------
+    // Group b empties buffer b, so one group's chain of loads, conversions and
+    // stores runs under the other's; a warp owns 32 columns, 16 at a time.
+    const int grp = (warp - 2) >> 3, q = warp & 3;
+    const int j00 = (((warp - 2) >> 2) & 1) * 32;  // this warp's packed columns
     const int row = q * 32 + lane;
     const bool odd = AC && (lane & 1);
-    constexpr int NJ = BC ? 8 : 16;        // logical columns of the group
+    constexpr int NJ = BC ? 8 : 16;        // logical columns of 16 packed ones
     constexpr int rows_out = AC ? 16 : 32;  // logical rows of this warp
     constexpr int RS = NJ + 1;              // staging row stride, padded
     constexpr bool REAL_ONLY = !AC && !BC;  // real operands: stage the real part only
@@ -846,61 +852,24 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
     constexpr int RPP = 32 / NJ;
     constexpr int NPASS = rows_out / RPP;
     const int lc = lane % NJ, lrw = lane / NJ;
-    int jt = 0;
-    for (int t = blockIdx.x; t < ntiles_total; t += gridDim.x, ++jt) {
+    const int td = threadIdx.x - 64 - 32 * (C::EPI / 2) * grp;
+    auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(32 * (C::EPI / 2)) : "memory"); };
+    int use = 0;
+    for (int t = blockIdx.x + grp * gridDim.x; t < ntiles_total; t += 2 * gridDim.x, ++use) {
       const TileCoord c = persist_tile(g, t, mtiles, ntiles);
-      const int b = jt & 1, use = jt >> 1;
-      // one decision for all drain warps, and the tile's column data
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * C::EPI) : "memory");
-      const int td = threadIdx.x - 64;
-      if (td == 0) sh->stop = sh->abort;
+      // one decision for the group, and the tile's column data
+      group_sync();
+      if (td == 0) sh->stop[grp] = sh->abort;
       {
         constexpr int ncl = BC ? C::BN / 2 : C::BN;
         if (td < ncl) {
           const int n = c.nt * ncl + td;
           long long o = -1;
           if (n < g.N) decomp_tc(g.gnC, n, o);
-          sh->col_off[td] = o;
+          sh->col_off[grp][td] = o;
         }
-        if (td < C::BN) sh->col_exp[td] = row_exp(g.expB[c.rowB0 + c.nt * C::BN + td]);
+        if (td < C::BN) sh->col_exp[grp][td] = row_exp(g.expB[c.rowB0 + c.nt * C::BN + td]);
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * C::EPI) : "memory");
-      if (sh->stop) break;  // the same value for every drain warp
-      const bool got = mbar_wait(smem_u32(&sh->accfull[b]), (uint32_t)(use & 1), kWaitLimit);
-      if (!__all_sync(0xffffffffu, got)) {
-        fail(sh, g.err, 4);
-        continue;  // the next tile's decision stops every drain warp
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      // Level sums of at most two K blocks stay below 2^22 (24576 x 128), so
-      // adding 1.5 x 2^23 leaves the integer in the low bits of the float,
-      // and two levels (2^7 apart) meet in 32 bits.
-      static_assert(24576LL * C::MAX_KB * TC_BK <= (1 << 22), "level sums of a persistent tile");
-      int p01[16], p23[16];
-#pragma unroll
-      for (int L0 = 2; L0 <= 5; L0 += 2) {
-        int* p = L0 == 2 ? p01 : p23;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) p[j] = 0;
-        if (L0 > S + 1) continue;
-        uint32_t lv[2][16];
-        tmem_ld16_nowait(tmem + tl + (uint32_t)b * buf_cols + (uint32_t)((L0 - 2) * C::BN + j0), lv[0]);
-        if (L0 < S + 1) tmem_ld16_nowait(tmem + tl + (uint32_t)b * buf_cols + (uint32_t)((L0 - 1) * C::BN + j0), lv[1]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          p[j] = (int)(__float_as_uint(__fadd_rn(__uint_as_float(lv[0][j]), 12582912.f)) - 0x4B400000u);
-          if (L0 < S + 1)
-            p[j] = (p[j] << 7) + (int)(__float_as_uint(__fadd_rn(__uint_as_float(lv[1][j]), 12582912.f)) - 0x4B400000u);
-        }
-      }
-      // units of 2^-u: level L weighs 2^(u - 7 L), u = 7 (S + 1)
-      long long a16[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) a16[j] = S <= 2 ? p01[j] : ((long long)p01[j] << (7 * (S - 2))) + p23[j];
-      // the levels are in registers: the MMAs of a later tile may refill this buffer
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      mbar_arrive(smem_u32(&sh->accempty[b]));
       const int prow = c.mt * TC_BM + row;
       const int m = AC ? (prow >> 1) : prow;
       const int ea = prow < g.rowsA_pad ? row_exp(g.expA[c.rowA0 + prow]) : 0;
@@ -911,71 +880,113 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
       double* Cr = static_cast<double*>(g.C) + (g.cc ? 0 : c.zb * g.bsC);
       const int m0w = AC ? ((c.mt * TC_BM + q * 32) >> 1) : (c.mt * TC_BM + q * 32);
       const int nrows = min(rows_out, g.M - m0w);
-      __syncwarp();  // the previous tile's stores have read the staging area
-#pragma unroll
-      for (int k = 0; k < NJ; ++k) {
-        const int jj = (BC ? j0 / 2 : j0) + k;
-        long long re, im;
-        if constexpr (BC) {
-          const long long x0 = a16[2 * k], x1 = a16[2 * k + 1];
-          if constexpr (AC) {
-            const long long p0 = __shfl_xor_sync(0xffffffffu, x0, 1);
-            const long long p1 = __shfl_xor_sync(0xffffffffu, x1, 1);
-            const long long rr = odd ? p0 : x0, ri = odd ? p1 : x1, ir = odd ? x0 : p0, ii = odd ? x1 : p1;
-            re = rr - ii;
-            im = ri + ir;
-          } else {
-            re = x0;
-            im = x1;
-          }
-        } else {
-          const long long x = a16[k];
-          if constexpr (AC) {
-            const long long p = __shfl_xor_sync(0xffffffffu, x, 1);
-            re = odd ? p : x;
-            im = odd ? x : p;
-          } else {
-            re = x;
-            im = 0;
-          }
-        }
-        if (AC && ((k & 1) != (lane & 1))) continue;
-        const int E = ebase + sh->col_exp[BC ? 2 * jj : jj];
-        double vr, vi;
-        if (g.alpha_pow2) {
-          vr = scaled_i64_to_double(neg ? -re : re, E);
-          vi = scaled_i64_to_double(neg ? -im : im, E);
-        } else {
-          const double dr = scaled_i64_to_double(re, E), di = scaled_i64_to_double(im, E);
-          vr = g.ar * dr - g.ai * di;
-          vi = g.ar * di + g.ai * dr;
-        }
-        if constexpr (REAL_ONLY)
-          stage1[lr * RS + k] = vr;
-        else
-          stage2[lr * RS + k] = make_double2(vr, vi);
+      group_sync();
+      if (sh->stop[grp]) break;  // the same value for every warp of the group
+      const bool got = mbar_wait(smem_u32(&sh->accfull[grp]), (uint32_t)(use & 1), kWaitLimit);
+      if (!__all_sync(0xffffffffu, got)) {
+        fail(sh, g.err, 4);
+        continue;  // the next tile's decision stops the group
       }
-      __syncwarp();
-      const long long cn = sh->col_off[(BC ? j0 / 2 : j0) + lc];
-#pragma unroll 4
-      for (int p = 0; p < NPASS; ++p) {
-        const int r = p * RPP + lrw;
-        const long long cm = __shfl_sync(0xffffffffu, coffm, (AC ? 2 * r : r) & 31);
-        if (r >= nrows || cn < 0) continue;
-        const long long off = cm + cn;
-        const double2 v = REAL_ONLY ? make_double2(stage1[r * RS + lc], 0.0) : stage2[r * RS + lc];
-        if (g.cc) {
-          if (red) {
-            atomicAdd(&Cc[off].x, v.x);
-            if (!REAL_ONLY) atomicAdd(&Cc[off].y, v.y);
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      if (nrows <= 0) {  // rows of padding only
+        mbar_arrive(smem_u32(&sh->accempty[grp]));
+        continue;
+      }
+#pragma unroll 1
+      for (int j0 = j00; j0 < j00 + 32; j0 += 16) {
+        // Level sums of at most two K blocks stay below 2^22 (24576 x 128), so
+        // adding 1.5 x 2^23 leaves the integer in the low bits of the float,
+        // and two levels (2^7 apart) meet in 32 bits.
+        static_assert(24576LL * C::MAX_KB * TC_BK <= (1 << 22), "level sums of a persistent tile");
+        int p01[16], p23[16];
+#pragma unroll
+        for (int L0 = 2; L0 <= 5; L0 += 2) {
+          int* p = L0 == 2 ? p01 : p23;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) p[j] = 0;
+          if (L0 > S + 1) continue;
+          uint32_t lv[2][16];
+          const uint32_t ta = tmem + tl + (uint32_t)grp * buf_cols + (uint32_t)((L0 - 2) * C::BN + j0);
+          tmem_ld16_nowait(ta, lv[0]);
+          if (L0 < S + 1) tmem_ld16_nowait(ta + C::BN, lv[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            p[j] = (int)(__float_as_uint(__fadd_rn(__uint_as_float(lv[0][j]), 12582912.f)) - 0x4B400000u);
+            if (L0 < S + 1)
+              p[j] = (p[j] << 7) + (int)(__float_as_uint(__fadd_rn(__uint_as_float(lv[1][j]), 12582912.f)) - 0x4B400000u);
+          }
+        }
+        if (j0 != j00) {  // all levels read: the MMAs of a later tile may refill this buffer
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          mbar_arrive(smem_u32(&sh->accempty[grp]));
+        }
+        // units of 2^-u: level L weighs 2^(u - 7 L), u = 7 (S + 1)
+        long long a16[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) a16[j] = S <= 2 ? p01[j] : ((long long)p01[j] << (7 * (S - 2))) + p23[j];
+        __syncwarp();  // the previous stores have read the staging area
+        auto put = [&](int k, long long re, long long im) {
+          const int jj = (BC ? j0 / 2 : j0) + k;
+          const int E = ebase + sh->col_exp[grp][BC ? 2 * jj : jj];
+          double vr, vi;
+          if (g.alpha_pow2) {
+            vr = scaled_i64_to_double(neg ? -re : re, E);
+            vi = scaled_i64_to_double(neg ? -im : im, E);
           } else {
-            Cc[off] = v;
+            const double dr = scaled_i64_to_double(re, E), di = scaled_i64_to_double(im, E);
+            vr = g.ar * dr - g.ai * di;
+            vi = g.ar * di + g.ai * dr;
+          }
+          if constexpr (REAL_ONLY)
+            stage1[lr * RS + k] = vr;
+          else
+            stage2[lr * RS + k] = make_double2(vr, vi);
+        };
+        if constexpr (AC) {
+          // a row's real and imaginary parts lie in neighbouring lanes: the even
+          // one finishes column k, the odd one k + 1, each with what the other
+          // holds of it
+#pragma unroll
+          for (int k = 0; k < NJ; k += 2) {
+            if constexpr (BC) {
+              const long long p0 = __shfl_xor_sync(0xffffffffu, odd ? a16[2 * k] : a16[2 * k + 2], 1);
+              const long long p1 = __shfl_xor_sync(0xffffffffu, odd ? a16[2 * k + 1] : a16[2 * k + 3], 1);
+              const long long x0 = odd ? a16[2 * k + 2] : a16[2 * k], x1 = odd ? a16[2 * k + 3] : a16[2 * k + 1];
+              // even: (re re, re im) own, (im re, im im) the partner's
+              put(k + (odd ? 1 : 0), odd ? p0 - x1 : x0 - p1, odd ? p1 + x0 : x1 + p0);
+            } else {
+              const long long p = __shfl_xor_sync(0xffffffffu, odd ? a16[k] : a16[k + 1], 1);
+              const long long x = odd ? a16[k + 1] : a16[k];
+              put(k + (odd ? 1 : 0), odd ? p : x, odd ? x : p);
+            }
           }
         } else {
-          if (red)
-            atomicAdd(&Cr[off], v.x);
-          else
-            Cr[off] = v.x;
+#pragma unroll
+          for (int k = 0; k < NJ; ++k) put(k, BC ? a16[2 * k] : a16[k], BC ? a16[2 * k + 1] : 0);
+        }
+        __syncwarp();
+        const long long cn = sh->col_off[grp][(BC ? j0 / 2 : j0) + lc];
+#pragma unroll 4
+        for (int p = 0; p < NPASS; ++p) {
+          const int r = p * RPP + lrw;
+          const long long cm = __shfl_sync(0xffffffffu, coffm, (AC ? 2 * r : r) & 31);
+          if (r >= nrows || cn < 0) continue;
+          const long long off = cm + cn;
+          const double2 v = REAL_ONLY ? make_double2(stage1[r * RS + lc], 0.0) : stage2[r * RS + lc];
+          if (g.cc) {
+            if (red) {
+              atomicAdd(&Cc[off].x, v.x);
+              if (!REAL_ONLY) atomicAdd(&Cc[off].y, v.y);
+            } else {
+              Cc[off] = v;
+            }
+          } else {
+            if (red)
+              atomicAdd(&Cr[off], v.x);
+            else
+              Cr[off] = v.x;
+          }
         }
       }
     }
