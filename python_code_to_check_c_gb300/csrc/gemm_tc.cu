@@ -34,6 +34,7 @@
 // Every wait has an iteration limit: on expiry the kernel records an error
 // code, stops issuing work, waits (bounded) for its own operations and frees
 // TMEM before returning.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -71,22 +72,27 @@ __device__ __forceinline__ int packed_exponent(unsigned long long mx, int E) {
 // Digits of two neighbouring elements of a packed row (same exponent e), one
 // BF16 pair per slice: out is the packed buffer as BF16 pairs, plane2 the
 // pairs per slice, idx2 the pair's index within a slice.
-// SMAX > TC_MAX_SLICES (the deep form): the last digit is rounded, not cut.
 template <int SMAX>
 __device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, size_t idx2, double x0, double x1,
-                                                 int e, int nbits, int S) {
-  int q0[SMAX], q1[SMAX];
-  if constexpr (SMAX > TC_MAX_SLICES) {
-    balanced_digits(fixed_point_rounded(x0, e, nbits), S, q0);
-    balanced_digits(fixed_point_rounded(x1, e, nbits), S, q1);
-  } else {
-    balanced_digits(fixed_point(x0, e, nbits), S, q0);
-    balanced_digits(fixed_point(x1, e, nbits), S, q1);
+                                                 int e, int S) {
+  uint32_t h0, l0, h1, l1;
+  cut_digits<SMAX>(x0, e, S, h0, l0);
+  cut_digits<SMAX>(x1, e, S, h1, l1);
+  const uint32_t sgn = (((uint32_t)__double2hiint(x0) >> 16) & 0x8000u) | ((uint32_t)__double2hiint(x1) & 0x80000000u);
+  out += idx2;
+  out[0] = digit_pair<21, true>(h0, h1, sgn);
+  if (S > 1) out[plane2] = digit_pair<14, false>(h0, h1, sgn);
+  if (S > 2) out[2 * plane2] = digit_pair<7, false>(h0, h1, sgn);
+  if (S > 3) out[3 * plane2] = digit_pair<0, false>(h0, h1, sgn);
+  if constexpr (SMAX == 8) {
+    out[4 * plane2] = digit_pair<21, false>(l0, l1, sgn);
+    out[5 * plane2] = digit_pair<14, false>(l0, l1, sgn);
+    out[6 * plane2] = digit_pair<7, false>(l0, l1, sgn);
+    out[7 * plane2] = digit_pair<0, false>(l0, l1, sgn);
+  } else if constexpr (SMAX == 6) {
+    if (S > 4) out[4 * plane2] = digit_pair<7, false>(l0, l1, sgn);
+    if (S > 5) out[5 * plane2] = digit_pair<0, false>(l0, l1, sgn);
   }
-  const bool n0 = __double_as_longlong(x0) < 0, n1 = __double_as_longlong(x1) < 0;  // sign bits
-#pragma unroll
-  for (int s = 0; s < SMAX; ++s)
-    if (s < S) out[s * plane2 + idx2] = digit_pair_bf16x2(n0 ? -q0[s] : q0[s], n1 ? -q1[s] : q1[s]);
 }
 
 // One block per logical row (per batch; the real and imaginary rows of a
@@ -105,24 +111,32 @@ __device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, s
 // With tab set, the K offsets (the same for every row) are decoded once per
 // block into shared memory as 32-bit integers (K of them) and both passes
 // read them there.
-template <int SMAX>
+//
+// CL = 8: a cluster of eight blocks per row, a segment of K each; the segments'
+// maxima meet through distributed shared memory.  For few long rows (K = o v^2
+// with 36 rows at o=18, v=82: 190 us as a block per row, 41 so).
+template <int SMAX, int CL>
 __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
   extern __shared__ int kofs[];
   const int per = p.cplx ? 2 : 1;
-  const int z = blockIdx.x / p.rows, m = blockIdx.x - z * p.rows;  // one block per live row
+  const int br = blockIdx.x / CL, part_k = CL > 1 ? blockIdx.x % CL : 0;
+  const int z = br / p.rows, m = br - z * p.rows;  // one block or cluster per live row
+  // this block's K indices: [kb, ke) of the row, [kb, kpe) with its padding
+  const int seg = (p.K_pad / 2 + CL - 1) / CL * 2;
+  const int kb = min(part_k * seg, p.K_pad), kpe = min(kb + seg, p.K_pad), ke = min(p.K, kpe);
   long long ro = 0;
   decomp_tc(p.gr, m, ro);
   ro += z * p.bs;
   if (tab) {
-    for (int k = threadIdx.x; k < p.K; k += blockDim.x) {
+    for (int k = kb + threadIdx.x; k < ke; k += blockDim.x) {
       long long ko;
       decomp_tc(p.gk, k, ko);
-      kofs[k] = (int)ko;
+      kofs[k - kb] = (int)ko;
     }
     __syncthreads();
   }
   auto koff = [&](int k) -> long long {
-    if (tab) return kofs[k];
+    if (tab) return kofs[k - kb];
     long long ko;
     decomp_tc(p.gk, k, ko);
     return ko;
@@ -133,13 +147,13 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
   unsigned long long mx = 0;
   // four independent loads in flight per thread (complex elements as one 16-byte load)
   constexpr int U = 4;
-  for (int k0 = threadIdx.x; k0 < p.K; k0 += U * blockDim.x) {
+  for (int k0 = kb + threadIdx.x; k0 < ke; k0 += U * blockDim.x) {
     unsigned long long v[U][2];
 #pragma unroll
     for (int j = 0; j < U; ++j) {
       const int k = k0 + j * blockDim.x;
       v[j][0] = v[j][1] = 0ull;
-      if (k < p.K) {
+      if (k < ke) {
         const long long e = ro + koff(k);
         if (p.cplx) {
           const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(bits + 2 * e);
@@ -159,21 +173,29 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
   __syncthreads();
   mx = 0;
   for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx = max(mx, wmax[w]);
+  if constexpr (CL > 1) {
+    namespace cg = cooperative_groups;
+    __shared__ unsigned long long cmax;
+    cg::cluster_group cl = cg::this_cluster();
+    if (threadIdx.x == 0) cmax = mx;
+    cl.sync();
+    for (int r = 0; r < CL; ++r) mx = max(mx, *cl.map_shared_rank(&cmax, r));
+    cl.sync();  // every block has read the others'
+  }
   const int E = (int)(mx >> 52);
   const int eb = packed_exponent<SMAX>(mx, E);
   const size_t prow = (size_t)z * p.rows_pad + (size_t)m * per;  // first packed row
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && part_k == 0) {
     p.exps[prow] = eb;
     if (p.cplx) p.exps[prow + 1] = eb;
   }
   const int e = row_exp(eb);
-  const int nbits = 7 * p.S;
   uint32_t* out = static_cast<uint32_t*>(p.out);  // BF16 pairs (K_pad is even)
   const size_t plane2 = (size_t)p.nb * p.rows_pad * (p.K_pad / 2);
   // pass 2 over pairs of neighbouring K indices (one 4-byte store per slice
   // and part), two pairs per thread: four loads in flight
   constexpr int U2 = 2;
-  for (int k0 = 2 * threadIdx.x; k0 < p.K_pad; k0 += 2 * U2 * blockDim.x) {
+  for (int k0 = kb + 2 * threadIdx.x; k0 < kpe; k0 += 2 * U2 * blockDim.x) {
     double x[U2][2][2];  // [pair][element][part]
 #pragma unroll
     for (int j = 0; j < U2; ++j)
@@ -181,7 +203,7 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
       for (int h = 0; h < 2; ++h) {
         const int k = k0 + 2 * j * blockDim.x + h;
         x[j][h][0] = x[j][h][1] = 0.0;
-        if (k < p.K) {
+        if (k < ke) {
           const long long el = ro + koff(k);
           if (p.cplx) {
             const double2 w = *reinterpret_cast<const double2*>(src + 2 * el);
@@ -195,10 +217,9 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
 #pragma unroll
     for (int j = 0; j < U2; ++j) {
       const int k = k0 + 2 * j * blockDim.x;
-      if (k >= p.K_pad) break;
+      if (k >= kpe) break;
       for (int part = 0; part < per; ++part)
-        store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, nbits,
-                         p.S);
+        store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, p.S);
     }
   }
 }
@@ -265,7 +286,6 @@ __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
     if (p.cplx) p.exps[prow + 1] = eb;
   }
   const int e = row_exp(eb);
-  const int nbits = 7 * p.S;
   uint32_t* out = static_cast<uint32_t*>(p.out);  // BF16 pairs (K_pad is even)
   const size_t plane2 = (size_t)p.nb * p.rows_pad * (p.K_pad / 2);
 #pragma unroll
@@ -273,7 +293,7 @@ __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
     const int k = 2 * (32 * wr + lane + 32 * W * j);
     if (k >= p.K_pad) break;
     for (int part = 0; part < per; ++part)
-      store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, nbits, p.S);
+      store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, p.S);
   }
 }
 
@@ -1355,9 +1375,11 @@ static cudaError_t launch_pack_slices(const PackArgs& p, long long blocks, cudaS
     else
       go(pack_rows_regs_kernel<4, 8, SMAX>, 1);
   } else {
-    // long rows: a block per row; few long rows (the K = o v^2 operands)
-    // take more threads per row so that the SMs still fill
-    const int threads = (p.K_pad >= 4096 && blocks < 4 * 152) ? 1024 : 256;
+    // long rows: a block per row, of more threads where there are few; fewer than
+    // the SMs, a cluster of eight blocks per row
+    constexpr int CL = 8;
+    const bool cluster = blocks <= 152 && p.K_pad >= 8192;
+    const int threads = cluster ? 512 : (p.K_pad >= 4096 && blocks < 4 * 152) ? 1024 : 256;
     // the K offsets as a shared-memory table when they fit (64 KB, 32 bits)
     constexpr int kTabMax = 16384;
     constexpr int kMaxDev = 64;
@@ -1366,14 +1388,34 @@ static cudaError_t launch_pack_slices(const PackArgs& p, long long blocks, cudaS
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
     std::call_once(once[dev], [dev] {
-      attr_err[dev] = cudaFuncSetAttribute(pack_kernel<SMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      attr_err[dev] = cudaFuncSetAttribute(pack_kernel<SMAX, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            kTabMax * (int)sizeof(int));
+      if (attr_err[dev] == cudaSuccess)
+        attr_err[dev] = cudaFuncSetAttribute(pack_kernel<SMAX, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             kTabMax * (int)sizeof(int));
     });
     long long span = 0;  // largest K offset
     for (int q = 0; q < p.gk.n && q < kMaxModes; ++q) span += (long long)(p.gk.dim[q] - 1) * std::llabs(p.gk.s0[q]);
-    const int tab = (attr_err[dev] == cudaSuccess && p.K <= kTabMax && span < (1LL << 31)) ? 1 : 0;
-    const size_t smem = tab ? (size_t)p.K * sizeof(int) : 0;
-    pack_kernel<SMAX><<<(unsigned)blocks, threads, smem, st>>>(p, tab);
+    const int seg = cluster ? (p.K_pad / 2 + CL - 1) / CL * 2 : p.K;
+    const int tab = (attr_err[dev] == cudaSuccess && seg <= kTabMax && span < (1LL << 31)) ? 1 : 0;
+    const size_t smem = tab ? (size_t)seg * sizeof(int) : 0;
+    if (cluster) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(blocks * CL));
+      cfg.blockDim = dim3(threads);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cudaLaunchAttribute at[1] = {};
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = CL;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, pack_kernel<SMAX, CL>, p, tab);
+      if (e != cudaSuccess) return e;
+    } else {
+      pack_kernel<SMAX, 1><<<(unsigned)blocks, threads, smem, st>>>(p, tab);
+    }
   }
   count_launch();
   return cudaGetLastError();
@@ -1385,8 +1427,10 @@ cudaError_t launch_pack(const PackArgs& p, cudaStream_t st) {
     return cudaErrorInvalidValue;
   const long long blocks = (long long)p.nb * p.rows;
   if (blocks > 0x7FFFFFFFLL) return cudaErrorInvalidConfiguration;
+  if (p.S < 1 || (p.S > TC_MAX_SLICES && p.S != TC_DEEP_SLICES)) return cudaErrorInvalidValue;
   return p.S > TC_MAX_SLICES ? launch_pack_slices<TC_DEEP_SLICES>(p, blocks, st)
-                             : launch_pack_slices<TC_MAX_SLICES>(p, blocks, st);
+         : p.S > 4           ? launch_pack_slices<TC_MAX_SLICES>(p, blocks, st)
+                             : launch_pack_slices<4>(p, blocks, st);
 }
 
 template <class C>
