@@ -1033,13 +1033,21 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
 // ---------------------------------------------------------------------------
 constexpr int kSimtMaxK = 64;
 
+// d += a * b on two FP32 pairs: one instruction, each half rounded as fmaf does
+__device__ __forceinline__ void fma_f32x2(float2& d, float2 a, float2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+      : "+l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+}
+
 // Tile BM x BN (32 x 32, 16 x 64 or 64 x 16), 256 threads on a 16 x 16 grid,
 // 4 outputs each: rows ty + 16 i, columns tx + 16 j.  Digits in shared memory
 // per K index and row: S x (2 if complex) floats, contiguous, read as float2.
 // Three blocks per SM: a block's exponents, digits and stores are chains of
 // loads that the others' multiply-adds cover (the K = 10 contractions at o=10,
-// v=38 with 24 trajectories: 198 us with two, 181 with three; K = 18 at o=18,
-// v=82: 258, 228).
+// v=38 with 24 trajectories: 198 us with two, 181 with three, 166 with a chunk's
+// loads all in flight and kept for its digits; K = 18 at o=18, v=82: 258, 228,
+// 207).
 template <bool AC, bool BC, bool CC, int S, int BM, int BN>
 __global__ void __launch_bounds__(256, 3) simt_slices_kernel(const GemmArgs g, int alpha_pow2, int alpha_e,
                                                              int alpha_neg) {
@@ -1088,31 +1096,65 @@ __global__ void __launch_bounds__(256, 3) simt_slices_kernel(const GemmArgs g, i
     dec(g.gk, k, kofa[k], kofb[k]);
   }
   __syncthreads();
-  // exponents of the tile's rows of A and columns of B over all of K: every
-  // thread takes elements (row, k) with independent loads, the maxima of the
-  // bit patterns (the order of |x| for finite doubles) meet in shared memory
-  constexpr unsigned long long kAbs = 0x7FFFFFFFFFFFFFFFull;
-  __shared__ unsigned long long rmax[BM + BN];
-  if (tid < BM + BN) rmax[tid] = 0ull;
+  // a chunk's elements of A (BM x KC) and B (KC x BN), E to a thread, all loads
+  // in flight
+  constexpr int E = ((BM + BN) * KC + 255) / 256;
+  double x[E][2];
+  auto place = [&](int i, bool& isA, int& r, int& kk) {
+    const int idx = tid + 256 * i;
+    isA = idx < BM * KC;
+    const int id2 = isA ? idx : idx - BM * KC, nr = isA ? BM : BN;
+    r = id2 % nr;
+    kk = id2 / nr;
+    return idx < (BM + BN) * KC;
+  };
+  auto load_chunk = [&](int kc) {
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      bool isA;
+      int r, kk;
+      const bool in = place(i, isA, r, kk);
+      const int k = kc + kk;
+      x[i][0] = x[i][1] = 0.0;
+      const long long base = !in ? -1 : isA ? aoff[r] : boff[r];
+      if (base >= 0 && k < g.K) {
+        const double* src = isA ? A : B;
+        const long long el = base + (isA ? kofa[k] : kofb[k]);
+        if ((isA ? PA : PB) == 2) {
+          const double2 v = *reinterpret_cast<const double2*>(src + 2 * el);
+          x[i][0] = v.x;
+          x[i][1] = v.y;
+        } else {
+          x[i][0] = src[el];
+        }
+      }
+    }
+  };
+  // exponents of the tile's rows of A and columns of B over all of K, as twice
+  // the biased exponent of the largest |x| plus one where there is a nonzero
+  __shared__ unsigned rmax[BM + BN];
+  if (tid < BM + BN) rmax[tid] = 0u;
   __syncthreads();
-  for (int idx = tid; idx < (BM + BN) * g.K; idx += blockDim.x) {
-    const int r = idx % (BM + BN), k = idx / (BM + BN);
-    const bool isA = r < BM;
-    const long long base = isA ? aoff[r] : boff[r - BM];
-    if (base < 0) continue;
-    const unsigned long long* bits =
-        reinterpret_cast<const unsigned long long*>(isA ? static_cast<const void*>(A) : static_cast<const void*>(B));
-    const int per = isA ? PA : PB;
-    const long long el = base + (isA ? kofa[k] : kofb[k]);
-    unsigned long long v = bits[per * el] & kAbs;
-    if (per == 2) v = max(v, bits[2 * el + 1] & kAbs);
-    if (v) atomicMax(&rmax[r], v);
+  for (int kc = 0; kc < g.K; kc += KC) {
+    load_chunk(kc);
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      bool isA;
+      int r, kk;
+      if (!place(i, isA, r, kk)) continue;
+      unsigned v = 0u;
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        const unsigned h = (unsigned)__double2hiint(x[i][part]) & 0x7FFFFFFFu;
+        if (h | (unsigned)__double2loint(x[i][part])) v = max(v, 2u * (h >> 20) + 1u);
+      }
+      if (v) atomicMax(&rmax[isA ? r : BM + r], v);
+    }
   }
   __syncthreads();
   if (tid < BM + BN) {
-    const unsigned long long mx = rmax[tid];
-    const int E = (int)(mx >> 52);
-    const int e = mx != 0 ? (E > 0 ? E - 1022 : -1022) : 0;
+    const int E2 = (int)(rmax[tid] >> 1);
+    const int e = rmax[tid] != 0u ? (E2 > 0 ? E2 - 1022 : -1022) : 0;
     if (tid < BM)
       ea[tid] = e;
     else
@@ -1120,86 +1162,79 @@ __global__ void __launch_bounds__(256, 3) simt_slices_kernel(const GemmArgs g, i
   }
   __syncthreads();
   const int tx = tid % 16, ty = tid / 16;
-  float acc[MI][NJ][S][2];
+  float2 acc[MI][NJ][S];  // levels, (re, im)
 #pragma unroll
   for (int i = 0; i < MI; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int L = 0; L < S; ++L) acc[i][j][L][0] = acc[i][j][L][1] = 0.f;
-  constexpr int nbits = 7 * S;
+      for (int L = 0; L < S; ++L) acc[i][j][L] = make_float2(0.f, 0.f);
   for (int kc = 0; kc < g.K; kc += KC) {
-    // digits of the chunk: BM rows x KC of A, KC x BN columns of B
-    for (int idx = tid; idx < (BM + BN) * KC; idx += blockDim.x) {
-      const bool isA = idx < BM * KC;
-      const int id2 = isA ? idx : idx - BM * KC;
-      const int nr = isA ? BM : BN;
-      const int r = id2 % nr, kk = id2 / nr, k = kc + kk;
-      const long long base = isA ? aoff[r] : boff[r];
-      const int per = isA ? PA : PB;
-      double x[2] = {0.0, 0.0};
-      if (base >= 0 && k < g.K) {
-        const double* src = isA ? A : B;
-        const long long el = base + (isA ? kofa[k] : kofb[k]);
-        x[0] = src[per * el];
-        if (per == 2) x[1] = src[2 * el + 1];
-      }
-      const int e = isA ? ea[r] : eb[r];
-      float* dst = isA ? &sa[kk][r][0] : &sb[kk][r][0];
-      for (int part = 0; part < per; ++part) {
-        const unsigned long long f = fixed_point(x[part], e, nbits);
-        const bool neg = __double_as_longlong(x[part]) < 0;  // sign bit: no FP64 compare
-        int qd[S];
-        balanced_digits(f, S, qd);
+    if (g.K > KC) load_chunk(kc);  // one chunk: as loaded for the exponents
 #pragma unroll
-        for (int s = 0; s < S; ++s) dst[s * per + part] = small_int_to_float(neg ? -qd[s] : qd[s]);
+    for (int i = 0; i < E; ++i) {
+      bool isA;
+      int r, kk;
+      if (!place(i, isA, r, kk)) continue;
+      const int per = isA ? PA : PB, e = isA ? ea[r] : eb[r];
+      float* dst = isA ? &sa[kk][r][0] : &sb[kk][r][0];
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        if (part >= per) continue;
+        uint32_t hi, lo;
+        cut_digits<(S <= 4 ? 4 : 6)>(x[i][part], e, S, hi, lo);
+        const uint32_t sgn = (uint32_t)__double2hiint(x[i][part]) & 0x80000000u;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          // 2^23 + u is the float 0x4B000000 + u; digits after the first are biased by 64
+          const uint32_t w = s < 4 ? hi : lo, bit = s < 4 ? 21 - 7 * s : 7 * (5 - s);
+          const uint32_t uf = ((w >> bit) & (s == 0 ? 0xFFu : 0x7Fu)) | 0x4B000000u;
+          const float d = __uint_as_float(uf) - (s == 0 ? 8388608.f : 8388672.f);
+          dst[s * per + part] = __uint_as_float(__float_as_uint(d) ^ sgn);
+        }
       }
     }
     __syncthreads();
     const int kn = min(KC, g.K - kc);
     for (int kk = 0; kk < kn; ++kk) {
-      float a[MI][SPA], b[NJ][SPB];
-#pragma unroll
-      for (int i = 0; i < MI; ++i)
-#pragma unroll
-        for (int q = 0; q < SPA / 2; ++q) {
-          const float2 v = *reinterpret_cast<const float2*>(&sa[kk][ty + 16 * i][2 * q]);
-          a[i][2 * q] = v.x;
-          a[i][2 * q + 1] = v.y;
-        }
+      // real times complex: re and im share a packed FP32 multiply-add (97 -> 73 us
+      // on a K = 10 contraction; complex times complex, which needs B's digits
+      // swapped as well: 176 us so, 166 with single ones)
+      float2 b[NJ][S];  // B's digits (re, im), or the real one twice
 #pragma unroll
       for (int j = 0; j < NJ; ++j)
 #pragma unroll
-        for (int q = 0; q < SPB / 2; ++q) {
-          const float2 v = *reinterpret_cast<const float2*>(&sb[kk][tx + 16 * j][2 * q]);
-          b[j][2 * q] = v.x;
-          b[j][2 * q + 1] = v.y;
+        for (int t = 0; t < S; ++t) {
+          const float* p = &sb[kk][tx + 16 * j][t * PB];
+          if constexpr (BC) {
+            b[j][t] = *reinterpret_cast<const float2*>(p);
+          } else {
+            b[j][t] = make_float2(p[0], p[0]);
+          }
         }
 #pragma unroll
       for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < NJ; ++j)
+        for (int s = 0; s < S; ++s) {
+          const float* p = &sa[kk][ty + 16 * i][s * PA];
+          const float2 a = AC ? *reinterpret_cast<const float2*>(p) : make_float2(p[0], p[0]);
 #pragma unroll
-          for (int s = 0; s < S; ++s)
+          for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int t = 0; t < S - s; ++t) {  // level s + t (0-based), s + t <= S - 1
-              float& re = acc[i][j][s + t][0];
-              float& im = acc[i][j][s + t][1];
+              float2& c = acc[i][j][s + t];
               if constexpr (AC && BC) {
-                re = fmaf(a[i][2 * s], b[j][2 * t], re);
-                re = fmaf(-a[i][2 * s + 1], b[j][2 * t + 1], re);
-                im = fmaf(a[i][2 * s], b[j][2 * t + 1], im);
-                im = fmaf(a[i][2 * s + 1], b[j][2 * t], im);
-              } else if constexpr (AC) {
-                re = fmaf(a[i][2 * s], b[j][t], re);
-                im = fmaf(a[i][2 * s + 1], b[j][t], im);
-              } else if constexpr (BC) {
-                re = fmaf(a[i][s], b[j][2 * t], re);
-                im = fmaf(a[i][s], b[j][2 * t + 1], im);
+                c.x = fmaf(a.x, b[j][t].x, c.x);
+                c.x = fmaf(-a.y, b[j][t].y, c.x);
+                c.y = fmaf(a.x, b[j][t].y, c.y);
+                c.y = fmaf(a.y, b[j][t].x, c.y);
+              } else if constexpr (AC || BC) {
+                fma_f32x2(c, a, b[j][t]);
               } else {
-                re = fmaf(a[i][s], b[j][t], re);
+                c.x = fmaf(a.x, b[j][t].x, c.x);
               }
             }
+        }
     }
     __syncthreads();
   }
@@ -1217,7 +1252,7 @@ __global__ void __launch_bounds__(256, 3) simt_slices_kernel(const GemmArgs g, i
         const int sh = u - 7 * (L + 2);
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-          const long long v = (long long)__float2int_rn(acc[i][j][L][p]);
+          const long long v = (long long)__float2int_rn(p ? acc[i][j][L].y : acc[i][j][L].x);
           X[p] += sh >= 0 ? (v << sh) : (v >> (-sh));
         }
       }

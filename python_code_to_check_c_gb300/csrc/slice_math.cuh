@@ -37,20 +37,8 @@ constexpr int kExpBias = 4096;
 constexpr int kExpMarked = 1 << 30;  // a row that digits cannot hold (deep form)
 __device__ __forceinline__ int row_exp(int biased) { return biased > 0 ? biased - kExpBias : 0; }
 
-// floor(|x| 2^(nbits - e)) as an integer, from the bits of x (exact; no FP64
-// arithmetic).  Requires |x| < 2^e and nbits <= 56, so the result < 2^nbits.
-__device__ __forceinline__ unsigned long long fixed_point(double x, int e, int nbits) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
-  const int E = (int)(u >> 52);
-  if (E == 0) return 0ull;  // zero or subnormal: below every slice
-  const unsigned long long M = (u & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-  const int sh = E - 1075 - e + nbits;  // |x| = M 2^(E-1075)
-  if (sh >= 0) return M << sh;
-  if (sh <= -64) return 0ull;
-  return M >> (-sh);
-}
-
-// The same rounded to nearest (ties away), at most 2^nbits.
+// |x| 2^(nbits - e) rounded to the nearest integer (ties away) from the bits of x
+// (no FP64 arithmetic).  Requires |x| < 2^e and nbits <= 56: at most 2^nbits.
 __device__ __forceinline__ unsigned long long fixed_point_rounded(double x, int e, int nbits) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
   const int E = (int)(u >> 52);
@@ -62,42 +50,13 @@ __device__ __forceinline__ unsigned long long fixed_point_rounded(double x, int 
   return ((M >> (-sh - 1)) + 1ull) >> 1;
 }
 
-// The digits of f <= 2^(7S) in balanced form, least significant first:
-// every digit below the top one in [-64, 63] (a digit >= 64 becomes d - 128
-// with a carry into the next), the top one in [0, 128].  The value is f
-// itself, sum_s q[s] 2^(7(S-1-s)), and products of digits stay within 2^14.
-template <int SMAX>
-__device__ __forceinline__ void balanced_digits(unsigned long long f, int S, int (&q)[SMAX]) {
-#pragma unroll
-  for (int i = SMAX - 1; i >= 1; --i)
-    if (i < S) {
-      int d = (int)(f & 127ull);
-      f >>= 7;
-      if (d >= 64) {
-        d -= 128;
-        ++f;
-      }
-      q[i] = d;
-    }
-  q[0] = (int)f;
-}
-
-// (float)d for |d| < 2^22 with one integer and one FP32 addition, both on
-// full-rate pipes (an int-to-float conversion runs at a quarter of that):
-// 0x4B400000 is the float 1.5 * 2^23, whose neighbours are 1 apart, so its
-// bits + d are the float 1.5 * 2^23 + d, and the subtraction is exact.  d = 0
-// gives +0, as the conversion does.
-__device__ __forceinline__ float small_int_to_float(int d) {
-  return __int_as_float(0x4B400000 + d) - 12582912.0f;
-}
-
 // |x| 2^-e cut into SMAX balanced digits of 7 bits (the packing keeps the first S),
 // in two words: hi holds digits 1 .. 4, the first in [0, 128] at bit 21, lo the
 // others.  The digits after the first are biased by 64: f plus 64 at each of their
 // places has them in its 7-bit fields, carries included.  SMAX = 4 and 6 cut after
 // 7 S bits, 8 rounds to 56.  |x| < 2^e; integer operations only, of 32 bits for
-// SMAX = 4 (6.9 M numbers at o=10, v=38 with
-// 24 trajectories: 51 us with 64-bit digits one by one, 38 so, 16 for their bytes).
+// SMAX = 4.  (Packing 6.9 M numbers, o=10, v=38 with 24 trajectories: 51 us with
+// digits cut one by one in 64 bits, 38 so, 16 for their bytes.)
 template <int SMAX>
 __device__ __forceinline__ void cut_digits(double x, int e, int S, uint32_t& hi, uint32_t& lo) {
   constexpr uint32_t kB3 = 64u * (1u + (1u << 7) + (1u << 14)), kB2 = 64u * (1u + (1u << 7));
