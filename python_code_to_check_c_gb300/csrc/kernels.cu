@@ -24,9 +24,146 @@ __global__ void __launch_bounds__(256) add_kernel(const AddArgs a) {
     add_element<IDX>(a, st, idx);
 }
 
+// The sums that make up a step (one to four tensors with real coefficients, fewer
+// than 2^31 elements, offsets of 32 bits): divisions by the extents as
+// multiplications (Granlund and Montgomery, PLDI 1994: n < 2^31, sh = ceil log2 d,
+// mul = floor(2^32 (2^sh - d) / d) + 1, n / d = (mulhi(n, mul) + n) >> sh), all
+// loads of an element's terms in flight, nothing 64 bits wide but the data.
+// Bound: the memory system, the L2 reductions and the FP64 pipe (two operations an
+// element and term after the first).  3.5 M elements: three terms 98 us through
+// add_kernel, 72 here (two elements a thread); two terms accumulated 56, 46 (one
+// element a thread: with two, 58; as loads and stores instead of reductions, whose
+// additions the FP64 pipe would do, 70).
+constexpr int kFastTerms = 4;
+struct AddFast {
+  void* C;
+  unsigned total;
+  int nd, cc, acc;
+  unsigned d[kAddDims], mul[kAddDims], sh[kAddDims];
+  int sC[kAddDims];
+  const void* A[kFastTerms];
+  double cr[kFastTerms];
+  int ac[kFastTerms];
+  int sA[kFastTerms][kAddDims];
+};
+
+template <int NT, int U>
+__global__ void __launch_bounds__(256) add_fast_kernel(const __grid_constant__ AddFast a) {
+  const unsigned long long cb = (unsigned long long)__double_as_longlong(a.cr[0]);
+  const int ce = (int)((cb >> 52) & 0x7FF);
+  const bool p2 = (cb & 0x000FFFFFFFFFFFFFull) == 0ull && ce > 0 && ce < 2047;
+  double2 x[U][NT];
+  int oc[U];
+  bool in[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const unsigned idx = (blockIdx.x * U + u) * 256u + threadIdx.x;
+    in[u] = idx < a.total;
+    unsigned l = in[u] ? idx : 0u;
+    int oa[NT];
+    oc[u] = 0;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) oa[t] = 0;
+#pragma unroll
+    for (int q = kAddDims - 1; q >= 0; --q)
+      if (q < a.nd) {
+        const unsigned quo = q > 0 ? (__umulhi(l, a.mul[q]) + l) >> a.sh[q] : 0u;
+        const int r = (int)(l - quo * a.d[q]);
+        l = quo;
+        oc[u] += r * a.sC[q];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) oa[t] += r * a.sA[t][q];
+      }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) x[u][t] = ld(a.A[t], oa[t], a.ac[t]);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (!in[u]) continue;
+    double2 s = cz();
+    if (p2)
+      s = make_double2(scale_pow2(x[u][0].x, a.cr[0], cb & 0x8000000000000000ull, ce - 1023),
+                       scale_pow2(x[u][0].y, a.cr[0], cb & 0x8000000000000000ull, ce - 1023));
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+      if (t > 0 || !p2) {
+        s.x = fma(a.cr[t], x[u][t].x, s.x);
+        s.y = fma(a.cr[t], x[u][t].y, s.y);
+      }
+    if (a.cc) {
+      double2* C = static_cast<double2*>(a.C) + oc[u];
+      if (a.acc) {
+        atomicAdd(&C->x, s.x);
+        atomicAdd(&C->y, s.y);
+      } else {
+        *C = s;
+      }
+    } else {
+      double* C = static_cast<double*>(a.C) + oc[u];
+      if (a.acc)
+        atomicAdd(C, s.x);
+      else
+        *C = s.x;
+    }
+  }
+}
+
+// false where the general kernel has to run
+static bool fast_add(const AddArgs& a, AddFast& f) {
+  constexpr long long kMax = 0x7FFFFFFFLL;
+  if (a.nt < 1 || a.nt > kFastTerms || a.total >= kMax - 512) return false;
+  auto spans = [&](const long long* s) {  // every offset fits 32 bits
+    long long lo = 0, hi = 0;
+    for (int q = 0; q < a.nd; ++q) (s[q] < 0 ? lo : hi) += (long long)(a.d[q] - 1) * s[q];
+    return lo >= -kMax && hi <= kMax;
+  };
+  if (!spans(a.sC)) return false;
+  for (int t = 0; t < a.nt; ++t)
+    if (a.t[t].B || a.t[t].ci != 0.0 || !spans(a.t[t].sA)) return false;
+  f.C = a.C;
+  f.total = (unsigned)a.total;
+  f.nd = a.nd;
+  f.cc = a.cc;
+  f.acc = a.acc;
+  for (int q = 0; q < a.nd; ++q) {
+    const unsigned long long d = (unsigned long long)a.d[q];
+    if (d < 1) return false;
+    unsigned sh = 0;
+    while ((1ull << sh) < d) ++sh;
+    f.d[q] = (unsigned)d;
+    f.sh[q] = sh;
+    f.mul[q] = (unsigned)(((1ull << 32) * ((1ull << sh) - d)) / d + 1);
+    f.sC[q] = a.d[q] > 1 ? (int)a.sC[q] : 0;
+    for (int t = 0; t < a.nt; ++t) f.sA[t][q] = a.d[q] > 1 ? (int)a.t[t].sA[q] : 0;
+  }
+  for (int t = 0; t < a.nt; ++t) {
+    f.A[t] = a.t[t].A;
+    f.cr[t] = a.t[t].cr;
+    f.ac[t] = a.t[t].ac;
+  }
+  return true;
+}
+
 cudaError_t launch_add(const AddArgs& a, cudaStream_t st) {
   if (a.total <= 0) return cudaSuccess;
   if (a.nd < 1 || a.nd > kAddDims) return cudaErrorInvalidValue;
+  AddFast f{};
+  if (fast_add(a, f)) {
+    auto go = [&](auto one, auto two) {
+      if (a.acc)
+        one<<<(unsigned)((a.total + 255) / 256), 256, 0, st>>>(f);
+      else
+        two<<<(unsigned)((a.total + 511) / 512), 256, 0, st>>>(f);
+    };
+    switch (a.nt) {
+      case 1: go(add_fast_kernel<1, 1>, add_fast_kernel<1, 2>); break;
+      case 2: go(add_fast_kernel<2, 1>, add_fast_kernel<2, 2>); break;
+      case 3: go(add_fast_kernel<3, 1>, add_fast_kernel<3, 2>); break;
+      default: go(add_fast_kernel<4, 1>, add_fast_kernel<4, 2>); break;
+    }
+    count_launch();
+    return cudaGetLastError();
+  }
   long long blocks = (a.total + 255) / 256;
   if (blocks > 152 * 16) blocks = 152 * 16;
   // 32-bit index arithmetic unless the index space needs 64 bits
