@@ -25,7 +25,8 @@
 // the 24-trajectory ladder at o=10, v=38 (S = 4, 1444 x 4800 x 1444 real) 210
 // us, 335 as single-chunk 128-column tiles over split K; the ladder
 // at o=18, v=82 (S = 5, 6724 x 648 x 6724 real) 829 us, 1842 as 64-column tiles
-// with int64 partial sums in TMEM (TcWide).
+// with int64 partial sums in TMEM (TcWide).  With complex rows the two lanes of a
+// row finish a column each (the ring terms of the former, K = 380: 174 -> 139 us).
 //
 // A row whose maximum is not finite (or that holds subnormals only) is marked
 // by the packing with 8 slices; its outputs are done by FP64 dot products over
@@ -193,6 +194,8 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       if (t < C::BN) sh->col_exp[t] = nt * C::BN + t < g.rowsB_pad ? g.expB[rowB0 + nt * C::BN + t] : 0;
       asm volatile("bar.sync 1, %0;" ::"n"(32 * C::EPI) : "memory");
     }
+    const int prow = mt * TC_BM + row;
+    const int ea = prow < g.rowsA_pad ? g.expA[rowA0 + prow] : 0;
     const uint32_t tl = (uint32_t)(q * 32) << 16;
     // exact sums in units of 2^-u: all levels (u = 7 (S + 1)), or with S = 8
     // levels 2..5 (u = 35) and 6..9 (u = 63)
@@ -245,9 +248,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       static_assert(C::EPI * 32 * RS * 16 <= C::STAGES * (C::A_BYTES + C::B_BYTES), "staging fits the ring");
       double2* stage = reinterpret_cast<double2*>(sm) + (size_t)(warp - 2) * (32 * RS);  // the ring is idle
       const int lr = AC ? (lane >> 1) : lane;
-      const int prow = mt * TC_BM + row;
       const int m = AC ? (prow >> 1) : prow;
-      const int ea = prow < g.rowsA_pad ? g.expA[rowA0 + prow] : 0;
       const bool neg = g.alpha_pow2 && g.alpha_neg;
       const int ebase = row_exp(ea) - 7 * (S + 1) + (g.alpha_pow2 ? g.alpha_e : 0);
       long long coffm = 0;
@@ -262,37 +263,9 @@ __global__ void __launch_bounds__(C::THREADS, 1)
 #pragma unroll
       for (int g0 = 0; g0 < NC; g0 += GC) {
         if (g0) __syncwarp();  // the previous group's stores have read the staging area
-#pragma unroll
-        for (int k = 0; k < NL; ++k) {
+        // value of the staged column k from its exact sums
+        auto put = [&](int k, const long long (&re)[HL], const long long (&im)[HL]) {
           const int jj = (BC ? (j0 + g0) / 2 : j0 + g0) + k;  // logical column within the tile
-          long long re[HL], im[HL];
-#pragma unroll
-          for (int h = 0; h < HL; ++h) {
-            im[h] = 0;
-            if constexpr (BC) {
-              const long long x0 = acc[h][g0 + 2 * k], x1 = acc[h][g0 + 2 * k + 1];
-              if constexpr (AC) {
-                const long long p0 = __shfl_xor_sync(0xffffffffu, x0, 1), p1 = __shfl_xor_sync(0xffffffffu, x1, 1);
-                // even lane: (re re, re im) own, (im re, im im) the partner's
-                re[h] = odd ? p0 - x1 : x0 - p1;
-                im[h] = odd ? p1 + x0 : x1 + p0;
-              } else {
-                re[h] = x0;
-                im[h] = x1;
-              }
-            } else {
-              const long long x = acc[h][g0 + k];
-              if constexpr (AC) {
-                const long long p = __shfl_xor_sync(0xffffffffu, x, 1);
-                re[h] = odd ? p : x;
-                im[h] = odd ? x : p;
-              } else {
-                re[h] = x;
-              }
-            }
-          }
-          // with complex A the two lanes of a pair hold the same output: split columns
-          if (AC && ((k & 1) != (lane & 1))) continue;
           const int eb = sh->col_exp[BC ? 2 * jj : jj];
           const int E = ebase + row_exp(eb);
           auto value = [&](const long long (&x)[HL]) {
@@ -313,6 +286,46 @@ __global__ void __launch_bounds__(C::THREADS, 1)
           }
           if (!g.alpha_pow2) v = make_double2(g.ar * v.x - g.ai * v.y, g.ar * v.y + g.ai * v.x);
           stage[lr * RS + k] = v;
+        };
+        if constexpr (AC) {
+          // a row's real and imaginary parts lie in neighbouring lanes: the even
+          // one finishes column k, the odd one k + 1, each with what the other
+          // holds of it
+          static_assert(NL % 2 == 0, "columns in pairs");
+#pragma unroll
+          for (int k = 0; k < NL; k += 2) {
+            long long re[HL], im[HL];
+#pragma unroll
+            for (int h = 0; h < HL; ++h) {
+              if constexpr (BC) {
+                const long long* c = &acc[h][g0 + 2 * k];
+                const long long p0 = __shfl_xor_sync(0xffffffffu, odd ? c[0] : c[2], 1);
+                const long long p1 = __shfl_xor_sync(0xffffffffu, odd ? c[1] : c[3], 1);
+                const long long x0 = odd ? c[2] : c[0], x1 = odd ? c[3] : c[1];
+                // even: (re re, re im) own, (im re, im im) the partner's
+                re[h] = odd ? p0 - x1 : x0 - p1;
+                im[h] = odd ? p1 + x0 : x1 + p0;
+              } else {
+                const long long* c = &acc[h][g0 + k];
+                const long long p = __shfl_xor_sync(0xffffffffu, odd ? c[0] : c[1], 1);
+                const long long x = odd ? c[1] : c[0];
+                re[h] = odd ? p : x;
+                im[h] = odd ? x : p;
+              }
+            }
+            put(k + (odd ? 1 : 0), re, im);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < NL; ++k) {
+            long long re[HL], im[HL];
+#pragma unroll
+            for (int h = 0; h < HL; ++h) {
+              re[h] = BC ? acc[h][g0 + 2 * k] : acc[h][g0 + k];
+              im[h] = BC ? acc[h][g0 + 2 * k + 1] : 0;
+            }
+            put(k, re, im);
+          }
         }
         __syncwarp();
         if constexpr (SYM) {  // the mirror image: lanes along the rows, which are its columns

@@ -524,37 +524,8 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
         // final chunk: combine, scale back, stage (lanes own rows here)
         const bool neg = g.alpha_pow2 && g.alpha_neg;
         constexpr int NJ = BC ? 8 : 16;  // logical columns in this group
-#pragma unroll
-        for (int k = 0; k < NJ; ++k) {
+        auto put = [&](int k, long long re, long long im) {
           const int jj = (BC ? j0 / 2 : j0) + k;
-          // integer combine: the pair exponents are shared, so these are exact
-          long long re, im;
-          if constexpr (BC) {
-            const long long x0 = a16[2 * k], x1 = a16[2 * k + 1];
-            if constexpr (AC) {
-              const long long p0 = __shfl_xor_sync(0xffffffffu, x0, 1);
-              const long long p1 = __shfl_xor_sync(0xffffffffu, x1, 1);
-              // even lane: (rr, ri) own, (ir, ii) partner; odd lane the reverse
-              const long long rr = odd ? p0 : x0, ri = odd ? p1 : x1, ir = odd ? x0 : p0, ii = odd ? x1 : p1;
-              re = rr - ii;
-              im = ri + ir;
-            } else {
-              re = x0;
-              im = x1;
-            }
-          } else {
-            const long long x = a16[k];
-            if constexpr (AC) {
-              const long long p = __shfl_xor_sync(0xffffffffu, x, 1);
-              re = odd ? p : x;
-              im = odd ? x : p;
-            } else {
-              re = x;
-              im = 0;
-            }
-          }
-          // with complex A the two lanes of a pair hold the same output: split columns
-          if (AC && ((jj & 1) != (lane & 1))) continue;
           const int E = ebase + sh->col_exp[BC ? 2 * jj : jj];
           double vr, vi;
           if (g.alpha_pow2) {
@@ -566,6 +537,29 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
             vi = g.ar * di + g.ai * dr;
           }
           stage[lr * RS + jj] = make_double2(vr, vi);
+        };
+        // integer combine: the pair exponents are shared, so these are exact
+        if constexpr (AC) {
+          // a row's real and imaginary parts lie in neighbouring lanes: the even
+          // one finishes column k, the odd one k + 1, each with what the other
+          // holds of it
+#pragma unroll
+          for (int k = 0; k < NJ; k += 2) {
+            if constexpr (BC) {
+              const long long p0 = __shfl_xor_sync(0xffffffffu, odd ? a16[2 * k] : a16[2 * k + 2], 1);
+              const long long p1 = __shfl_xor_sync(0xffffffffu, odd ? a16[2 * k + 1] : a16[2 * k + 3], 1);
+              const long long x0 = odd ? a16[2 * k + 2] : a16[2 * k], x1 = odd ? a16[2 * k + 3] : a16[2 * k + 1];
+              // even: (re re, re im) own, (im re, im im) the partner's
+              put(k + (odd ? 1 : 0), odd ? p0 - x1 : x0 - p1, odd ? p1 + x0 : x1 + p0);
+            } else {
+              const long long p = __shfl_xor_sync(0xffffffffu, odd ? a16[k] : a16[k + 1], 1);
+              const long long x = odd ? a16[k + 1] : a16[k];
+              put(k + (odd ? 1 : 0), odd ? p : x, odd ? x : p);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < NJ; ++k) put(k, BC ? a16[2 * k] : a16[k], BC ? a16[2 * k + 1] : 0);
         }
       }
       if (!last) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

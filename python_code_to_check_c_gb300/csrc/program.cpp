@@ -1169,8 +1169,9 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     // S <= 5 and longer K: the deep form, which sums all of K in one CTA.
     // Against 128-column tiles over split K (S = 4, o=10, v=38, 24
     // trajectories) 210 us for 335 on the ladder (23 blocks), 174 for 190 on
-    // the ring terms (6); against the 64-column tile (S = 5, o=18, v=82) 829
-    // for 1842 (106 blocks), 420 for 892 (24).  A B side of less than 3/4 of a
+    // the ring terms (6; both forms' drains were quickened later); against the
+    // 64-column tile (S = 5, o=18, v=82) 829 for 1842 (106 blocks), 420 for 892
+    // (24).  A B side of less than 3/4 of a
     // tile keeps the 64-column tile.
     const int deepBN = S == 5 ? 96 : 128;
     const bool long_k = !deep && S <= 5 && a.kblocks > 2 && nBrows >= deepBN * 3 / 4;
