@@ -768,11 +768,12 @@ void PhaseKernel::build(const Program& p, Program::Phase ph, std::vector<void*>&
     recs[at.first].pslot[at.second] = -2;
     recs[at.first].pbyte[at.second] += (long long)(uintptr_t)(d + rb + tb + 256);
   }
-  if (cudaMemcpy(d, recs.data(), rb, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(d + rb, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-      (!tables.empty() && cudaMemcpy(d + rb + tb + 256, tables.data(), tables.size() * sizeof(int2),
-                                     cudaMemcpyHostToDevice) != cudaSuccess) ||
-      cudaMemset(d + rb + tb, 0, 256) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+  std::vector<char> host(rb + tb + 256 + ob, 0);  // one copy, the barrier's words zero
+  memcpy(host.data(), recs.data(), rb);
+  memcpy(host.data() + rb, tab.data(), tab.size() * sizeof(int));
+  if (!tables.empty()) memcpy(host.data() + rb + tb + 256, tables.data(), tables.size() * sizeof(int2));
+  if (cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaDeviceSynchronize() != cudaSuccess)
     throw std::runtime_error("uploading the phase records failed");
   ops_ = d;
   tab_ = reinterpret_cast<int*>(d + rb);
