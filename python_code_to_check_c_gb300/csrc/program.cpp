@@ -909,11 +909,15 @@ static void merge_pack_modes(ModeGroup& g) {
 
 // K splits of a contraction of the FP64 form on the tensor cores (deep form),
 // 0 where the integer pipe is expected to be faster.  Model, in microseconds:
-// the fixed-point tiles reach 4.3 real multiply-adds per clock and SM; a deep
+// the fixed-point tiles reach 4.3 real multiply-adds per clock and SM in large
+// grids, 3.0 at the sizes where the choice lies; a deep
 // tile takes 6.5 per K block and 13 for its first loads and its drain, one per
 // SM; packing an operand that is not an integral block 3 and its traffic at 3
 // TB/s.  Measured at o=10, v=38: the ladder (1444 x 200 x 1444 real) 320 us
-// on the integer pipe, 75 deep.
+// on the integer pipe, 70 deep; residuals T2, L1, L2 of one trajectory in us with
+// 4.3, 3.0, 2.2 here: 842 852 704, 764 794 630, 783 787 610; at o=9, v=31 570 539
+// 445, 557 525 436, 566 537 456; at o=14, v=20 627 554 473, 573 504 449, 573 503
+// 445.
 static int deep_splits(const Op& op) {
   constexpr int BM = 128, BN = 64, BK = 64, kMinK = 32;
   const GemmArgs& g = op.g;
@@ -921,7 +925,7 @@ static int deep_splits(const Op& op) {
   const bool ac = op.dta == C64, bc = op.dtb == C64;
   if (g.K < kMinK || (op.dtc != C64 && (ac || bc))) return 0;
   const double ra = (double)g.M * (ac ? 2 : 1), rb = (double)g.N * (bc ? 2 : 1);
-  const double fx = 6.0 + ra * rb * K * nb / (152.0 * 4.3 * 2070.0);
+  const double fx = 6.0 + ra * rb * K * nb / (152.0 * 3.0 * 2070.0);
   const long long tiles = (long long)(std::ceil(ra / BM) * std::ceil(rb / BN) * nb), kb = (g.K + BK - 1) / BK;
   double best = 1e300;
   int splits = 0;
