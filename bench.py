@@ -49,14 +49,14 @@ W0S = (0.5, 0.923)
 POLS = (0, 1, 2)
 REF_TRAJ = (2, 0.002, 0.923)  # the single-trajectory configuration (z, A, w0)
 # DRAM traffic of the slice-product kernels against their algorithmic bytes (packed operands
-# read once, output written once): 460.9 MB over 403.8 MB for four launches of the T2 program
+# read once, output written once): 424 MB over 402 MB for four launches of the T2 program
 # (ladder, 24 batched products, two long-K products), a one-pass ncu capture (dram__bytes_read.sum,
 # dram__bytes_write.sum) of `bench_cases/profile_case.py --block T2 --precision mixed --slices 4
 # --nb 24`; the roofline's traffic per launch is this ratio times the step's algorithmic bytes per
 # slice-product launch.
-TRAFFIC_RATIO = {"ozaki_kernel": 460.9 / 403.8}
+TRAFFIC_RATIO = {"ozaki_kernel": 424.3 / 402.0}
 TRAFFIC_SOURCE = ("ncu DRAM bytes / algorithmic bytes of four slice-product launches of the T2 program "
-                  "(1.14), times the step's algorithmic bytes per launch")
+                  "(1.06), times the step's algorithmic bytes per launch")
 
 
 def parse():
@@ -518,7 +518,7 @@ def run_ours(args, rank, world, local_rank):
 
     def kernel_of(r):
         if r["kind"] == 0:
-            return {1: "ozaki_kernel", 2: "simt_slices_kernel"}.get(r["backend"], "gemm_f64_kernel")
+            return {1: "ozaki_kernel", 2: "simt_slices_kernel"}.get(r["backend"], "gemm_fx_kernel")
         if r["tag"].endswith(":packA") or r["tag"].endswith(":packB"):
             return "pack_kernel"
         return "add_kernel" if r["kind"] == 1 else "rk4/trace kernels"
@@ -546,7 +546,7 @@ def run_ours(args, rank, world, local_rank):
                 "peak_source": "measured bf16 burst (MEASURED_PEAKS.json)" if "bf16_tflops" in peaks else "fallback",
                 "achieved_is": "FP64-equivalent algorithmic flops of the step's slice products / their launch time",
                 "tensor_work_frac": achieved * pairs / peak}
-    elif kern in ("gemm_f64_kernel", "simt_slices_kernel"):
+    elif kern in ("gemm_fx_kernel", "simt_slices_kernel"):
         achieved = dom["flops"] / (dom["ms"] / 1e3) / 1e12
         peak = 1.25
         roof = {"bound": "fp64", "unit": "TFLOP/s", "peak_source": "nominal GB300 FP64 (no measured FP64 peak)"}

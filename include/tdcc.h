@@ -125,11 +125,12 @@ int tdcc_system_batch(tdcc_system s);   /* nb of the system (0 for NULL) */
 int tdcc_set_fields(tdcc_system s, const tdcc_field* fields, const int* pol);
 
 /* Selects the contraction arithmetic (TDCC_PREC_*) and, for the mixed mode,
-   the number of BF16 slices per operand (2..6; 7 bits each).  With up to 4
-   slices the tensor-core products take the 128-column tile or, for one or
-   two K blocks, the persistent 64-column form; with 5 or 6 the 64-column
-   tile.  4 slices keep |d mu| within 1e-8 a.u. of the FP64 form over 2000
-   steps of the o=10, v=38 system; strongly correlated systems need 5.    */
+   the number of BF16 slices per operand (2..6; 7 bits each).  With up to 5
+   slices long contractions sum all of K in one tile's registers (tiles of 128
+   or 96 columns); with up to 4, those of one or two K blocks of 64 take the
+   persistent 64-column form; the others 64- or 32-column tiles.  4 slices
+   keep |d mu| within 1e-8 a.u. of the FP64 form over 2000 steps of the
+   o=10, v=38 system; strongly correlated systems need 5.                  */
 int tdcc_set_precision(tdcc_system s, int mode, int slices);
 
 /* Ground-state amplitudes by Jacobi sweeps with eigh(F) denominators and
@@ -282,7 +283,9 @@ long long tdcc_adjoint_program_json(int o, int v, int method, int block, int n_m
    mo_spin_eri, CCSD_Helper.py:57-93):
      tei[p,q,r,s] = sum_Q B[Q,p,r] B[Q,q,s] - sum_Q B[Q,p,s] B[Q,q,r]
    B: device float64 [nq][n][n]; tei: device float64 [n][n][n][n] (written).
-   FP64 GEMM over Q, then an in-place antisymmetrisation.                   */
+   A symmetric product over Q (exact digit products or fixed point, FP64
+   accuracy), then an in-place antisymmetrisation.  Scratch: the packed
+   factors, from a pool of the library's own.                              */
 int tdcc_tei_from_df(const double* B, int n, int nq, double* tei, void* stream);
 
 /* Dipole spectrum (Plots.py:20-25): the discrete Fourier transforms of
