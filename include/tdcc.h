@@ -52,12 +52,15 @@ enum { TDCC_T1 = 0, TDCC_T2 = 1, TDCC_L1 = 2, TDCC_L2 = 3 };
 
 /* contraction arithmetic */
 enum {
-  TDCC_PREC_FP64 = 0,      /* the plain form, FP64 accuracy: small
-                              contractions as FP64 dot products, larger ones
-                              in 56-bit fixed point under each row's maximum
-                              with exact sums (integer pipe, or eight-slice
-                              tensor-core products), rounded to FP64 at the
-                              end; FP64 everywhere else                    */
+  TDCC_PREC_FP64 = 0,      /* the plain form: small contractions as FP64 dot
+                              products; larger ones with exact sums of 63-bit
+                              (eight-slice tensor-core products) or some 78-bit
+                              numbers (integer pipe) under each real row's
+                              maximum, and by FP64 multiply-adds where a row
+                              spans too much for that.  An output is off by
+                              no more than 2^-53 of the sum of its products'
+                              magnitudes (rms; FP64 chains: 0.5 to 1), at any
+                              range of the operands.  FP64 everywhere else   */
   TDCC_PREC_MIXED = 1      /* large contractions as split-BF16 tcgen05
                               products, FP64 everywhere else               */
 };

@@ -1776,7 +1776,7 @@ int tdcc_tei_from_df(const double* B, int n, int nq, double* tei, void* stream) 
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cap));
     const long long rows = (n2 + 127) / 128 * 128, kpad = (nq + 63) / 64 * 64LL;
-    const long long exp_off = (long long)TC_DEEP_SLICES * rows * kpad * 2, need = exp_off + rows * 4 + 256;
+    const long long exp_off = (long long)tc_planes(TC_DEEP_SLICES) * rows * kpad * 2, need = exp_off + rows * 4 + 256;
     Scratch w;
     if (nq >= 32 && t_deep < 0.85 * t_fx && cap == cudaStreamCaptureStatusNone && need <= deep_budget()) w.get((size_t)need, st);
     if (w.p) {

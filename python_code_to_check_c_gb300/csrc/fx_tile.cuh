@@ -4,25 +4,28 @@
 // chip), its integer pipe 26 of 32 x 32 + 64 bits (both measured, operands
 // from shared memory).  So a
 // contraction C[m,n] (+)= alpha sum_k A[m,k] B[k,n] is cut into K chunks of
-// at most 60; in a chunk each row of A and column of B is scaled by the power
-// of two above its largest magnitude (real and imaginary parts share it) and
-// written as v = h 2^28 + l, |v| < 2^56, |h| <= 2^28, -2^27 <= l < 2^27: 56
-// bits, three more than an FP64 significand at the row's maximum.  A product
-// is h h' 2^56 + (h l' + l h') 2^28, three multiply-adds into two 64-bit sums
-// that cannot overflow (2 x 60 terms of 2^56, 4 x 60 of 2^55); l l', at most
-// 2^-58 of the product of the two maxima and of either sign, is left out.
-// The sums are exact; each chunk is rounded to FP64 once, where an FP64 chain
-// rounds every term, so the error against 64 bits is no larger than the
-// FP64 kernel's (measured over both on the residuals' own operands and on
-// random ones, K = 2..2000).
+// at most 60; in a chunk each real row of A and column of B (the real and
+// imaginary parts of a complex one are two) is scaled by the power of two
+// above its largest magnitude and written as v = h 2^28 + l + r, |v| < 2^56,
+// |h| <= 2^28, -2^27 <= l < 2^27, |r| <= 1/2: 56 bits as integers, the rest
+// of a small element as an FP32 number.  A product is h h' 2^56 + (h l' + l h')
+// 2^28, three multiply-adds into two 64-bit sums that cannot overflow (60
+// terms of 2^56, 2 x 60 of 2^55), and l l' + v r' + r v', three FP32
+// multiply-adds of at most 2^-57 of the row maxima: about 78 bits under the
+// maxima altogether.  The integer sums are exact; each chunk is rounded to FP64
+// once, where an FP64 chain rounds every term.  Rows that span more still are
+// found by the range guard below and done by FP64 multiply-adds.  So an output's
+// error against the sum of its products' magnitudes is below an FP64 chain's,
+// not only the error against the largest output.
 //
-// Bound: the integer multiply-adds, at 85-90 % of that rate while they run
-// (a complex 16 x 16 x 60 tile: 8.5 of 16.4 k clocks), then index
-// work and cutting; 16 warps (512 threads, 64 registers) gain 8 % on one tile
-// and lose 5 % on many.  Against the FP64 kernel it replaced (64 x 64 tile, at 96
-// % of the FP64 pipe), one launch: real 2304 x 2304 x 144 1324 -> 484 us;
-// complex by real 1444 x 100 x 1444 1450 -> 320 us; the T2 residual at o=10,
-// v=38 5.13 -> 1.66 ms.
+// Bound: issue, the integer multiply-adds (4.9 clocks a warp and scheduler each) and
+// the FP32 ones beside them; then index work and cutting (16 warps, 512 threads and
+// 64 registers, gain 8 % on one tile and lose 5 % on many).  With the integer sums
+// alone, 56 bits and one scale for both parts of a complex row, a launch took 35 us
+// where this takes 49 (100 x 100 x 196 complex, o=10, v=14) and 24 where this takes 37
+// (380 x 38 x 38 complex by 100, o=10, v=38); the FP64 kernel before (64 x 64 tile, at
+// 96 % of the FP64 pipe) 1450 us for 1444 x 100 x 1444 complex by real, where the
+// integers alone took 320.
 //
 // A chunk whose maxima are not finite, or so large or small that scaling by
 // them would leave the normal range, is done by FP64 multiply-adds from
@@ -41,15 +44,10 @@ constexpr int kFxThreads = 256;
 constexpr int kChunk = 60;                 // K per chunk: keeps the 64-bit sums below 2^63
 constexpr int kExpLo = 101, kExpHi = 1946;  // biased exponents of a chunk maximum that scaling handles
 
-template <bool AC>
-struct Limbs;  // one element: h, l (and the imaginary part's h, l)
-template <>
-struct Limbs<true> {
-  using T = int4;
-};
-template <>
-struct Limbs<false> {
-  using T = int2;
+// a real number of a chunk: its limbs, the remainder r and x = v 2^-56, both FP32
+struct __align__(16) FxNum {
+  int h, l;
+  float r, x;
 };
 
 __device__ __forceinline__ void decode2(const ModeGroup& g, int l, long long& o0, long long& o1) {
@@ -74,69 +72,82 @@ __device__ __forceinline__ unsigned upper_abs(double x) {
   return (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
 }
 
-// x 2^(56 - e) rounded to an integer, e = Emax - 1022, as limbs h, l: the
-// significand left-justified in 64 bits, shifted down by Emax - E; h = bits
-// 36.. rounded to nearest, l = the signed 28 bits below it.
-__device__ __forceinline__ int2 limbs(double x, int Emax) {
+// x 2^(56 - e), e = Emax - 1022, as limbs and remainder: the significand
+// left-justified in 64 bits, shifted down by Emax - E; h = bits 36.. rounded to
+// nearest, l = the signed 28 bits below it, r = what rounding at bit 8 left.  A
+// nonzero element too small for FP32 (2^-125 of the maximum) is marked by a NaN.
+__device__ __forceinline__ FxNum cut_number(double x, int Emax) {
   const unsigned bh = (unsigned)__double2hiint(x), bl = (unsigned)__double2loint(x);
   const int E = (int)(bh >> 20) & 0x7FF;
   const unsigned d = (unsigned)(Emax - E);  // 0 .. 2046
-  unsigned uh = 0x80000000u | (bh << 11) | (bl >> 21), ul = bl << 11;
+  unsigned w2 = 0x80000000u | (bh << 11) | (bl >> 21), w1 = bl << 11, w0 = 0u;
   if (d >= 32u) {
-    ul = uh;
-    uh = 0u;
+    w0 = w1;
+    w1 = w2;
+    w2 = 0u;
   }
-  ul = __funnelshift_r(ul, uh, d & 31u);
-  uh >>= (d & 31u);
-  if (d >= 64u || E == 0) uh = ul = 0u;
+  const unsigned out = __funnelshift_r(w0, w1, d & 31u), ul = __funnelshift_r(w1, w2, d & 31u);
+  unsigned uh = w2 >> (d & 31u);
   const unsigned rl = ul + 128u;  // round at bit 8
   uh += rl < ul ? 1u : 0u;
   int h = (int)((uh >> 4) + ((uh >> 3) & 1u));  // up to 2^28
   int l = (int)(__funnelshift_r(rl, uh, 8) << 4) >> 4;
+  float r = (float)(int)((ul << 24) | (out >> 8)) * 0x1p-32f;
+  float f = __uint_as_float(((126u - d) << 23) | ((bh & 0xFFFFFu) << 3) | (bl >> 29));
+  if (E == 0 || d > 125u) f = ((bh << 1) | bl) == 0u ? 0.f : __uint_as_float(0x7FC00000u);
+  if (E == 0 || d >= 64u) {
+    h = l = 0;
+    r = f * 0x1p56f;
+  }
   const int s = (int)bh >> 31;
-  return make_int2((h ^ s) - s, (l ^ s) - s);
+  FxNum q;
+  q.h = (h ^ s) - s;
+  q.l = (l ^ s) - s;
+  q.r = s ? -r : r;
+  q.x = s ? -f : f;
+  return q;
 }
 
 __device__ __forceinline__ void imad(long long& c, int a, int b) { c += (long long)a * (long long)b; }
 
-// one product into its sums: hh and mm hold the real (and imaginary) part
-template <bool AC, bool BC, int NP>
-__device__ __forceinline__ void fx_mac(long long (&hh)[NP], long long (&mm)[NP], const typename Limbs<AC>::T& a,
-                                       const typename Limbs<BC>::T& b) {
-  imad(hh[0], a.x, b.x);
-  imad(mm[0], a.x, b.y);
-  imad(mm[0], a.y, b.x);
-  if constexpr (AC && BC) {
-    const int nh = -a.z, nl = -a.w;
-    imad(hh[1], a.x, b.z);
-    imad(mm[1], a.x, b.w);
-    imad(mm[1], a.y, b.z);
-    imad(hh[0], nh, b.z);
-    imad(mm[0], nh, b.w);
-    imad(mm[0], nl, b.z);
-    imad(hh[1], a.z, b.x);
-    imad(mm[1], a.z, b.y);
-    imad(mm[1], a.w, b.x);
-  } else if constexpr (AC) {
-    imad(hh[1], a.z, b.x);
-    imad(mm[1], a.z, b.y);
-    imad(mm[1], a.w, b.x);
-  } else if constexpr (BC) {
-    imad(hh[1], a.x, b.z);
-    imad(mm[1], a.x, b.w);
-    imad(mm[1], a.y, b.z);
-  }
+// The FP32 companions of a number: l 2^-28, and |x| 2^60 for the range guard.
+struct FxAux {
+  float l, g;
+};
+__device__ __forceinline__ FxAux fx_aux(const FxNum& a) {
+  // (the integer l / 64 in the low bits of a number between 2 and 4)
+  return {__int_as_float((a.l >> 6) + 0x40400000) - 3.f, fabsf(a.x) * 0x1p60f};
 }
 
-// (h 2^28 + m) 2^E as a double: the two sums joined in 64 bits at the top of
+// One product into its sums: hh, mm the integers, f = sum l l' 2^-56 + x r' + r x',
+// s = 2^120 sum |x x'|.
+__device__ __forceinline__ void fx_mac(long long& hh, long long& mm, float& f, float& s, const FxNum& a, const FxAux& ax,
+                                       const FxNum& b, const FxAux& bx) {
+  imad(hh, a.h, b.h);
+  imad(mm, a.h, b.l);
+  imad(mm, a.l, b.h);
+  f = fmaf(ax.l, bx.l, f);
+  f = fmaf(a.x, b.r, f);
+  f = fmaf(a.r, b.x, f);
+  s = fmaf(ax.g, bx.g, s);
+}
+
+// The range guard.  FP32 leaves the small part f of a product off by some 2^-78 of
+// the row maxima, so an output whose products' magnitudes add up to less than 2^-22
+// a product (rows that fall along K by 10^6 against columns that rise by it) is
+// done by FP64 multiply-adds instead.  s = 0 has no product that is not zero.
+__device__ __forceinline__ bool out_of_range(float s, int K) { return !(s == 0.f || s >= 0x1p98f * (float)K); }
+
+// (h 2^SH + m) 2^E as a double: the two sums joined in 64 bits at the top of
 // their common magnitude, then rounded to nearest.
+template <int SH = 28>
 __device__ __forceinline__ double joined(long long h, long long m, int E) {
-  const long long t = h + (m >> 28);                 // top part
-  const unsigned long long lo = (unsigned long long)m & 0xFFFFFFFull;  // 28 bits below it
+  const long long t = h + (m >> SH);                 // top part
+  const unsigned long long lo = (unsigned long long)m & ((1ull << SH) - 1ull);  // SH bits below it
   const int lz = __clzll(t ^ (t >> 63)) - 1;         // redundant sign bits (63 for 0 and -1)
-  const int s = lz < 28 ? lz : 28;
-  const long long X = (long long)(((unsigned long long)t << s) | (lo >> (28 - s)));
-  return scaled_i64_to_double(X, E + 28 - s);
+  const int s = lz < SH ? lz : SH;
+  const long long X = (long long)(((unsigned long long)t << s) | (lo >> (SH - s)));
+  return scaled_i64_to_double(X, E + SH - s);
 }
 
 __device__ __forceinline__ void fmac(double2& c, double2 a, double2 b) {
@@ -154,9 +165,14 @@ __device__ __forceinline__ double2 load1(const double* p, long long off) {
     return make_double2(p[off], 0.0);
 }
 
-// bytes of kc rows of limbs, rounded so that what follows is 16-byte aligned
-__host__ __device__ __forceinline__ size_t limb_bytes(int kc, int pitch, size_t esz) {
-  return ((size_t)kc * pitch * esz + 15) & ~(size_t)15;
+// shared memory of a K index of a tile, rounded so that each operand's planes are
+// whole; K indices per chunk: two blocks on an SM
+__host__ __device__ __forceinline__ constexpr int fx_k_bytes(int bm, int bn, bool ac, bool bc) {
+  return (int)sizeof(FxNum) * ((bm + 1) * (ac ? 2 : 1) + (bn + 1) * (bc ? 2 : 1));
+}
+__host__ __device__ __forceinline__ constexpr int fx_chunk(int bm, int bn, bool ac, bool bc) {
+  const int k = 104 * 1024 / fx_k_bytes(bm, bn, ac, bc);
+  return k < kChunk ? k : kChunk;
 }
 
 // This thread's elements of an R x kn piece of an operand (kn <= kChunk), all
@@ -191,31 +207,27 @@ struct Piece {
       }
     }
   }
-  // the largest upper word of each row, met in shared memory
-  __device__ __forceinline__ void maxima(unsigned* e) const {
+  // the largest upper word of each row, met in shared memory; real and imaginary
+  // parts are rows of their own (e[0][r], e[1][r])
+  __device__ __forceinline__ void maxima(unsigned (*e)[64]) const {
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (at[u] >= 0) {
-        unsigned w = upper_abs(x[u][0]);
-        if constexpr (CX) w = max(w, upper_abs(x[u][1]));
-        unsigned* q = &e[at[u] & 255];
-        if (w > *(volatile unsigned*)q) atomicMax(q, w);
-      }
+      if (at[u] >= 0)
+#pragma unroll
+        for (int p = 0; p < (CX ? 2 : 1); ++p) {
+          const unsigned w = upper_abs(x[u][p]);
+          unsigned* q = &e[p][at[u] & 255];
+          if (w > *(volatile unsigned*)q) atomicMax(q, w);
+        }
   }
-  template <class L>
-  __device__ __forceinline__ void cut(L* s, int pitch, const unsigned* e) const {
+  // into planes [part][k][pitch]
+  __device__ __forceinline__ void cut(FxNum* s, int pitch, int kc, const unsigned (*e)[64]) const {
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (at[u] >= 0) {
         const int r = at[u] & 255, k = at[u] >> 8;
-        const int Em = (int)(e[r] >> 20);
-        const int2 h = limbs(x[u][0], Em);
-        if constexpr (CX) {
-          const int2 q = limbs(x[u][1], Em);
-          s[k * pitch + r] = make_int4(h.x, h.y, q.x, q.y);
-        } else {
-          s[k * pitch + r] = h;
-        }
+#pragma unroll
+        for (int p = 0; p < (CX ? 2 : 1); ++p) s[(p * kc + k) * pitch + r] = cut_number(x[u][p], (int)(e[p][r] >> 20));
       }
   }
 };
@@ -224,7 +236,7 @@ struct Piece {
 struct FxScratch {
   long long aoff[64], boff[64], coffm[64], coffn[64];
   long long kofa[kChunk], kofb[kChunk];
-  unsigned eA[64], eB[64];
+  unsigned eA[2][64], eB[2][64];
 };
 
 // One tile (number `tile` of the output, batch and K split z) by a block of
@@ -238,14 +250,12 @@ __device__ __forceinline__ void fx_tile(const GemmArgs& g, const FxPlan& f, unsi
   constexpr int TM = BM / 16, TN = BN / 16;
   constexpr bool CX = AC || BC;
   constexpr int NP = CX ? 2 : 1;
-  using LA = typename Limbs<AC>::T;
-  using LB = typename Limbs<BC>::T;
   constexpr int PA = BM + 1, PB = BN + 1;  // limb row pitches (a k-fast store strides by them)
   const int kc = f.kc, flags = f.flags, alpha_pow2 = f.p2, alpha_e = f.e2, alpha_neg = f.neg;
-  LA* sA = reinterpret_cast<LA*>(smraw);                                      // [kc][PA]
-  LB* sB = reinterpret_cast<LB*>(smraw + limb_bytes(kc, PA, sizeof(LA)));       // [kc][PB]
+  FxNum* sA = reinterpret_cast<FxNum*>(smraw);       // [part][kc][PA]
+  FxNum* sB = sA + (size_t)kc * PA * (AC ? 2 : 1);  // [part][kc][PB]
   long long *aoff = sh.aoff, *boff = sh.boff, *coffm = sh.coffm, *coffn = sh.coffn, *kofa = sh.kofa, *kofb = sh.kofb;
-  unsigned *eA = sh.eA, *eB = sh.eB;  // upper word of each row's / column's chunk maximum
+  unsigned (*eA)[64] = sh.eA, (*eB)[64] = sh.eB;  // upper word of each row's / column's chunk maximum
   const int tid = threadIdx.x;
   const int mt = (int)(tile % (unsigned)f.mtiles), nt = (int)(tile / (unsigned)f.mtiles);
   const int m0 = mt * BM, n0 = nt * BN;
@@ -261,9 +271,9 @@ __device__ __forceinline__ void fx_tile(const GemmArgs& g, const FxPlan& f, unsi
     // one thread per row, column and k (BM + BN + kc <= 156)
     if (tid < BM + BN) {
       if (tid < BM)
-        eA[tid] = 0;
+        eA[0][tid] = eA[1][tid] = 0;
       else
-        eB[tid - BM] = 0;
+        eB[0][tid - BM] = eB[1][tid - BM] = 0;
       if (k0 == kbeg) {
         long long o0 = -1, o1 = -1;
         if (tid < BM) {
@@ -290,78 +300,120 @@ __device__ __forceinline__ void fx_tile(const GemmArgs& g, const FxPlan& f, unsi
     pb.maxima(eB);
     __syncthreads();
     int bad = 0;
-    if (tid < BM + BN) {
-      const unsigned w = tid < BM ? eA[tid] : eB[tid - BM];
-      if (w != 0u && ((w >> 20) < (unsigned)kExpLo || (w >> 20) > (unsigned)kExpHi)) bad = 1;
-    }
-    if (__syncthreads_or(bad)) {
-      // FP64 multiply-adds on the operands as they are
-      for (int i = 0; i < TM; ++i)
-        for (int j = 0; j < TN; ++j) {
-          const long long ao = aoff[ty + 16 * i], bo = boff[tx + 16 * j];
-          double2 s = make_double2(0.0, 0.0);
-          if (ao >= 0 && bo >= 0)
-            for (int k = 0; k < kn; ++k) {
-              const double2 x = load1<AC>(A, ao + kofa[k]), y = load1<BC>(B, bo + kofb[k]);
-              if constexpr (AC && BC)
-                fmac(s, x, y);
-              else if constexpr (AC)
-                s = make_double2(fma(x.x, y.x, s.x), fma(x.y, y.x, s.y));
-              else
-                s = make_double2(fma(x.x, y.x, s.x), fma(x.x, y.y, s.y));
-            }
-          if (alpha_pow2) {  // the sums below carry alpha
-            s.x *= g.ar;
-            s.y *= g.ar;
-          }
-#pragma unroll
-          for (int ii = 0; ii < TM; ++ii)
-#pragma unroll
-            for (int jj = 0; jj < TN; ++jj)
-              if (ii == i && jj == j) {
-                sum[ii][jj][0] = k0 == kbeg ? s.x : sum[ii][jj][0] + s.x;
-                if constexpr (CX) sum[ii][jj][1] = k0 == kbeg ? s.y : sum[ii][jj][1] + s.y;
-              }
-        }
-      continue;
-    }
-    pa.cut(sA, PA, eA);
-    pb.cut(sB, PB, eB);
-    __syncthreads();
-    long long hh[TM][TN][NP], mm[TM][TN][NP];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j)
-#pragma unroll
-        for (int p = 0; p < NP; ++p) hh[i][j][p] = mm[i][j][p] = 0;
-#pragma unroll 2
-    for (int k = 0; k < kn; ++k) {
-      LA a[TM];
-      LB b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = sA[k * PA + ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = sB[k * PB + tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) fx_mac<AC, BC>(hh[i][j], mm[i][j], a[i], b[j]);
-    }
-    // each chunk is rounded to FP64 once
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        // h carries 2^56 / 2^112: value = (h 2^28 + m) 2^(28 - 112 + ea + eb)
-        const int E = (int)(eA[ty + 16 * i] >> 20) + (int)(eB[tx + 16 * j] >> 20) - 2 * 1022 - 84 + alpha_e;
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const long long h = alpha_neg ? -hh[i][j][p] : hh[i][j][p], m = alpha_neg ? -mm[i][j][p] : mm[i][j][p];
-          const double x = joined(h, m, E);
-          sum[i][j][p] = k0 == kbeg ? x : sum[i][j][p] + x;
-        }
+    if (tid < BM + BN)
+      for (int p = 0; p < 2; ++p) {
+        const unsigned w = tid < BM ? eA[p][tid] : eB[p][tid - BM];
+        if (w != 0u && ((w >> 20) < (unsigned)kExpLo || (w >> 20) > (unsigned)kExpHi)) bad = 1;
       }
+    bad = __syncthreads_or(bad);
+    if (!bad) {
+      pa.cut(sA, PA, kc, eA);
+      pb.cut(sB, PB, kc, eB);
+      __syncthreads();
+    }
+    // complex by complex: the real parts of A by B, then the imaginary parts (a
+    // row's two parts have scales of their own)
+#pragma unroll
+    for (int pass = 0; pass < (AC && BC ? 2 : 1); ++pass) {
+      // outputs to do in FP64, bit (i TN + j) NP + q: the whole chunk, or what the guard finds
+      unsigned direct = 0u;
+      double val[TM][TN][NP];
+      if (!bad) {
+        long long hh[TM][TN][NP], mm[TM][TN][NP];
+        float fs[TM][TN][NP], gs[TM][TN][NP];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+              hh[i][j][p] = mm[i][j][p] = 0;
+              fs[i][j][p] = gs[i][j][p] = 0.f;
+            }
+        // the parts of a complex operand by the real numbers of the other
+        constexpr int QA = AC && !BC ? 2 : 1, QB = BC ? 2 : 1;
+        const FxNum* ra = sA + (AC && BC ? (size_t)pass * kc * PA : 0) + ty;
+        const FxNum* rb = sB + tx;
+#pragma unroll 2
+        for (int k = 0; k < kn; ++k) {
+          FxNum a[TM][QA];
+          FxAux ax[TM][QA];
+#pragma unroll
+          for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int p = 0; p < QA; ++p) {
+              a[i][p] = ra[(p * kc + k) * PA + 16 * i];
+              ax[i][p] = fx_aux(a[i][p]);
+            }
+#pragma unroll
+          for (int j = 0; j < TN; ++j)
+#pragma unroll
+            for (int p = 0; p < QB; ++p) {
+              const FxNum b = rb[(p * kc + k) * PB + 16 * j];
+              const FxAux bx = fx_aux(b);
+#pragma unroll
+              for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int pp = 0; pp < QA; ++pp) {
+                  const int q = QA == 2 ? pp : p;
+                  fx_mac(hh[i][j][q], mm[i][j][q], fs[i][j][q], gs[i][j][q], a[i][pp], ax[i][pp], b, bx);
+                }
+            }
+        }
+        // each chunk is rounded to FP64 once
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j)
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+              // h carries 2^56 / 2^112: value = (h 2^28 + m) 2^(28 - 112 + ea + eb)
+              const int E = (int)(eA[AC && !BC ? q : pass][ty + 16 * i] >> 20) + (int)(eB[BC ? q : 0][tx + 16 * j] >> 20) -
+                            2 * 1022 - 84 + alpha_e;
+              const long long h = hh[i][j][q], m = mm[i][j][q] + __float2ll_rn(fs[i][j][q] * 0x1p28f);
+              val[i][j][q] = joined(alpha_neg ? -h : h, alpha_neg ? -m : m, E);
+              if (out_of_range(gs[i][j][q], kn)) direct |= 1u << ((i * TN + j) * NP + q);
+            }
+      } else {
+        direct = (1u << (TM * TN * NP)) - 1u;
+      }
+      // FP64 multiply-adds on the operands as they are
+      while (direct) {
+        const int bit = __ffs(direct) - 1, q = bit % NP, j = bit / NP % TN, i = bit / (NP * TN);
+        direct &= direct - 1u;
+        const long long ao = aoff[ty + 16 * i], bo = boff[tx + 16 * j];
+        double s = 0.0;
+        if (ao >= 0 && bo >= 0) {
+          const double* x = A + (AC ? 2 * ao + (BC ? pass : q) : ao);
+          const double* y = B + (BC ? 2 * bo + q : bo);
+#pragma unroll 4
+          for (int k = 0; k < kn; ++k) s = fma(x[(AC ? 2 : 1) * kofa[k]], y[(BC ? 2 : 1) * kofb[k]], s);
+        }
+        if (alpha_pow2) s *= g.ar;  // the sums below carry alpha
+#pragma unroll
+        for (int ii = 0; ii < TM; ++ii)
+#pragma unroll
+          for (int jj = 0; jj < TN; ++jj)
+#pragma unroll
+            for (int qq = 0; qq < NP; ++qq)
+              if ((ii * TN + jj) * NP + qq == bit) val[ii][jj][qq] = s;
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          double v[NP];
+#pragma unroll
+          for (int q = 0; q < NP; ++q) v[q] = val[i][j][q];
+          if constexpr (AC && BC)
+            if (pass == 1) {  // i (re + i im)
+              v[0] = -val[i][j][1];
+              v[1] = val[i][j][0];
+            }
+#pragma unroll
+          for (int q = 0; q < NP; ++q) sum[i][j][q] = k0 == kbeg && pass == 0 ? v[q] : sum[i][j][q] + v[q];
+        }
+    }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {

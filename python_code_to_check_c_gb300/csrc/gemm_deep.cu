@@ -1,18 +1,17 @@
 // Exact BF16 slice products on tcgen05 with the sums over all of K in the drain
-// warps' registers: the FP64 form's contractions (8 slices of 7 bits a side,
-// 56 bits under each row's maximum, the last digit rounded) and the mixed
-// form's with up to 5 slices and K beyond two blocks.
+// warps' registers: the FP64 form's contractions (8 slices of 8 bits a side, the
+// first of 7: 63 bits under each real row's maximum, the last digit rounded) and the
+// mixed form's with up to 5 slices of 7 bits and K beyond two blocks.
 //
 // The products A_s B_t with s + t <= S + 1 go to the accumulators of their
 // levels L = s + t, FP32 sums of integers that stay exact over a K chunk
 // (TcDeep::CHUNK_KB).  The S levels of a 128 x BN tile fill TMEM (BN = 128, 96,
 // 64 for S <= 4, 5, 8); after every chunk the drain warps add them to int64
 // sums (two per output for S = 8, levels 2..5 and 6..9), which are rounded to
-// FP64 once at the end.  With 8 slices what is dropped (levels above 9, the
-// operands' rounding) is about 2^-58 of the product of the two row maxima per
-// term and of either sign: against extended precision the four residuals at
-// o=8, v=26 (amplitudes near an MP2 guess or normal) are off by 0.61 to 1.02
-// times what FP64 multiply-add chains gave.
+// FP64 once at the end.  With 8 slices the real and the imaginary part of a complex
+// row have scales of their own (a small imaginary part keeps its bits), so their
+// sums become doubles before they meet; and rows that even 63 bits hold worse than
+// FP64 does are found by the range guard below.
 //
 // Order of a K block: the slices arrive in pairs (A_j, B_j), j = 1..S, and
 // step j runs the products that pair j completes, (j, t <= min(j, S + 1 - j))
@@ -20,7 +19,9 @@
 // pair; a pair is released after its last product.  Bound: shared memory.  A K
 // block's MMAs read their operands at 128 bytes a clock (S = 8: 144 of 48
 // clocks, 6.9 k), its slices arrive by TMA at 32 (192 KB, 6.1 k), and the two
-// add up: 13.3 k clocks measured.  So the wider the tile the better (per
+// add up: 13.3 k clocks measured (with a drain every 6 blocks; 8-bit digits drain
+// every 2, and the guard takes 0.4 k a block: the ladder at o=10, v=38, 1444 x 200 x
+// 1444 real, 70 us with 7-bit digits, 78 so).  So the wider the tile the better (per
 // output column and K block 52, 82 and 204 clocks for S = 4, 5, 8).  Measured:
 // the 24-trajectory ladder at o=10, v=38 (S = 4, 1444 x 4800 x 1444 real) 210
 // us, 335 as single-chunk 128-column tiles over split K; the ladder
@@ -29,8 +30,8 @@
 // row finish a column each (the ring terms of the former, K = 380: 174 -> 139 us).
 //
 // A row whose maximum is not finite (or that holds subnormals only) is marked
-// by the packing with 8 slices; its outputs are done by FP64 dot products over
-// the operands.
+// by the packing with 8 slices; its outputs, and those that the range guard sends
+// on, are done by FP64 multiply-adds over the operands, a warp for four rows of a column.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -49,6 +50,17 @@ CUtensorMap slice_map(const void* base, int S, int rows_pad, int K_pad, int box_
 
 namespace {
 
+// The range guard.  Digits under the maximum of a row hold its small elements worse
+// than FP64 does: with the factors in units of their rows' powers of two, K products
+// are off by about 2^-63.6 sqrt(K) in all (the levels left out 2^-64.2 a product, the
+// rounding of each factor 2^-64.8).  A plane of each packed operand holds the magnitudes
+// x, y in 8 bits; after the slices one more product on the tensor cores gives S = sum
+// x y, against which FP64 chains are off by 0.46 x 2^-53 (normal rows) to 0.9 (the
+// residuals' own, K = 81 .. 1444).  An output with S < kGuardDeep sqrt(K), that is with
+// an error above 0.65 x 2^-53 S (rms), is done by FP64 multiply-adds; S = 0 has no product
+// that is not zero.  A part of a K split takes its S for its share of the whole.
+constexpr float kGuardDeep = 0x1p-10f;
+
 template <class C>
 struct DeepShared {
   uint64_t full[C::STAGES], empty[C::STAGES];
@@ -60,29 +72,71 @@ struct DeepShared {
   long long col_offT[C::S > 5 ? C::BN : 1];  // offset of each column as a row (symmetric products)
 };
 
-// sum over k in [k0, k1) of A[m, k] B[k, n] of batch z, operands as they are
-__device__ __noinline__ double2 direct_dot(const TcArgs& g, int m, int n, int z, int k0, int k1) {
-  long long ao, bo, dummy;
-  decode2(g.gmA, m, ao, dummy);
+// Rows m[0 .. 3] of A times column n of B over k in [k0, k1), batch z, the operands
+// as they are: FP64 multiply-adds, the lanes of the warp over k (every lane returns
+// the sums).
+constexpr int kDirect = 4;
+template <bool AC, bool BC>
+__device__ __noinline__ void direct_dots(const TcArgs& g, const int (&m)[kDirect], int n, int z, int k0, int k1,
+                                         double2 (&s)[kDirect]) {
+  const int lane = threadIdx.x & 31;
+  long long ao[kDirect], bo, dummy;
+  double2 c[kDirect];
+#pragma unroll
+  for (int i = 0; i < kDirect; ++i) {
+    decode2(g.gmA, m[i], ao[i], dummy);
+    ao[i] += z * g.bsA;
+    c[i] = make_double2(0.0, 0.0);
+  }
   decode2(g.gnB, n, bo, dummy);
-  ao += z * g.bsA;
   bo += z * g.bsB;
   const double *A = static_cast<const double*>(g.srcA), *B = static_cast<const double*>(g.srcB);
-  double2 s = make_double2(0.0, 0.0);
-  for (int k = k0; k < k1; ++k) {
+#pragma unroll 2
+  for (int k = k0 + lane; k < k1; k += 32) {
     long long ka, kb;
     decode2(g.gkAB, k, ka, kb);
-    const double2 x = g.ac ? load1<true>(A, ao + ka) : load1<false>(A, ao + ka);
-    const double2 y = g.bc ? load1<true>(B, bo + kb) : load1<false>(B, bo + kb);
-    if (g.ac && g.bc) {
-      fmac(s, x, y);
-    } else if (g.ac) {
-      s = make_double2(fma(x.x, y.x, s.x), fma(x.y, y.x, s.y));
-    } else {
-      s = make_double2(fma(x.x, y.x, s.x), fma(x.x, y.y, s.y));
+    const double2 y = load1<BC>(B, bo + kb);
+#pragma unroll
+    for (int i = 0; i < kDirect; ++i) {
+      const double2 x = load1<AC>(A, ao[i] + ka);
+      if constexpr (AC && BC) {
+        fmac(c[i], x, y);
+      } else if constexpr (AC) {
+        c[i] = make_double2(fma(x.x, y.x, c[i].x), fma(x.y, y.x, c[i].y));
+      } else {
+        c[i].x = fma(x.x, y.x, c[i].x);
+        if constexpr (BC) c[i].y = fma(x.x, y.y, c[i].y);
+      }
     }
   }
-  return s;
+  // the 4 or 8 sums meet across the warp, halving what a lane holds while it can (9
+  // additions instead of 40)
+  constexpr int NV = AC || BC ? 2 * kDirect : kDirect;
+  double v[NV];
+#pragma unroll
+  for (int i = 0; i < kDirect; ++i) {
+    if constexpr (AC || BC) {
+      v[2 * i] = c[i].x;
+      v[2 * i + 1] = c[i].y;
+    } else {
+      v[i] = c[i].x;
+    }
+  }
+  int d = 16;
+#pragma unroll
+  for (int n = NV / 2; n >= 1; n >>= 1, d >>= 1)
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const double send = lane & d ? v[i] : v[i + n], keep = lane & d ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+    }
+  for (; d > 0; d >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], d);
+  constexpr int LV = 32 / NV;  // lanes that hold the same sum
+#pragma unroll
+  for (int i = 0; i < kDirect; ++i) {
+    s[i].x = __shfl_sync(0xffffffffu, v[0], LV * (AC || BC ? 2 * i : i));
+    s[i].y = AC || BC ? __shfl_sync(0xffffffffu, v[0], LV * (2 * i + 1)) : 0.0;
+  }
 }
 
 template <class C, bool AC, bool BC>
@@ -128,23 +182,31 @@ __global__ void __launch_bounds__(C::THREADS, 1)
   const int kb1 = skip ? kb0 : min(g.kblocks, kb0 + g.kb_per_split);
   const int rowA0 = g.bat_a ? zb * g.rowsA_pad : 0, rowB0 = g.bat_b ? zb * g.rowsB_pad : 0;
   const int nchunks = (kb1 - kb0 + C::CHUNK_KB - 1) / C::CHUNK_KB;
+  // 8 slices: digits of 8 bits, a scale for each real row; after the chunks, the range
+  // guard over the same K
+  constexpr bool GUARD = S == TC_DEEP_SLICES;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       int it = 0;
-      for (int kb = kb0; kb < kb1 && !sh->abort; ++kb)
-        for (int s = 0; s < S && !sh->abort; ++s, ++it) {
-          const int st = it % C::STAGES;
-          if (!mbar_wait(smem_u32(&sh->empty[st]), (uint32_t)((it / C::STAGES) & 1) ^ 1u, kWaitLimit)) {
-            fail(sh, g.err, 1);
-            break;
-          }
-          const uint32_t fb = smem_u32(&sh->full[st]);
-          mbar_expect_tx(fb, C::A_BYTES + C::B_BYTES);
-          tma3d(smem_u32(stA + st * C::A_BYTES), &tmA, kb * TC_BK, rowA0 + mt * TC_BM, s, fb);
-          tma3d(smem_u32(stB + st * C::B_BYTES), &tmB, kb * TC_BK, rowB0 + nt * C::BN, s, fb);
+      auto load = [&](int kb, int s) {
+        const int st = it % C::STAGES;
+        if (!mbar_wait(smem_u32(&sh->empty[st]), (uint32_t)((it / C::STAGES) & 1) ^ 1u, kWaitLimit)) {
+          fail(sh, g.err, 1);
+          return;
         }
+        const uint32_t fb = smem_u32(&sh->full[st]);
+        mbar_expect_tx(fb, C::A_BYTES + C::B_BYTES);
+        const int x = GUARD && s == S ? kb * (TC_BK / 2) : kb * TC_BK;  // (a byte a number)
+        tma3d(smem_u32(stA + st * C::A_BYTES), &tmA, x, rowA0 + mt * TC_BM, s, fb);
+        tma3d(smem_u32(stB + st * C::B_BYTES), &tmB, x, rowB0 + nt * C::BN, s, fb);
+        ++it;
+      };
+      for (int kb = kb0; kb < kb1 && !sh->abort; ++kb)
+        for (int s = 0; s < S && !sh->abort; ++s) load(kb, s);
+      if (GUARD)
+        for (int kb = kb0; kb < kb1 && !sh->abort; kb += 2) load(kb, S);
       // every issued load lands before the CTA exits
       for (int j = (it > C::STAGES ? it - C::STAGES : 0); j < it; ++j)
         mbar_wait(smem_u32(&sh->full[j % C::STAGES]), (uint32_t)((j / C::STAGES) & 1), kWaitLimit);
@@ -167,6 +229,17 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       if (!ok) fail(sh, g.err, 3);
       if (ok) umma_commit_warp(smem_u32(&sh->accfull), on);
       ok = __all_sync(0xffffffffu, ok && sh->abort == 0) != 0;
+    }
+    if (GUARD && ok && nchunks > 0) {
+      ok = mbar_wait_warp(smem_u32(&sh->accempty), (uint32_t)((nchunks - 1) & 1), kWaitLimit);
+      if (!ok) fail(sh, g.err, 2);
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+      for (int kb = kb0; kb < kb1 && ok; kb += 2) {
+        ok = ring.template guard<C::BN>(tmem, id, kb == kb0, kb + 1 == kb1, on);
+        if (!ok) fail(sh, g.err, 3);
+      }
+      if (ok) umma_commit_warp(smem_u32(&sh->accfull), on);
     }
     // all issued MMAs complete before TMEM is released
     umma_commit_warp(smem_u32(&sh->done), on);
@@ -198,13 +271,14 @@ __global__ void __launch_bounds__(C::THREADS, 1)
     const int ea = prow < g.rowsA_pad ? g.expA[rowA0 + prow] : 0;
     const uint32_t tl = (uint32_t)(q * 32) << 16;
     // exact sums in units of 2^-u: all levels (u = 7 (S + 1)), or with S = 8
-    // levels 2..5 (u = 35) and 6..9 (u = 63)
+    // levels 2..5 (u = 38) and 6..9 (u = 70)
     long long acc[HL][NC];
 #pragma unroll
     for (int h = 0; h < HL; ++h)
 #pragma unroll
       for (int j = 0; j < NC; ++j) acc[h][j] = 0;
     bool ok = true;
+    unsigned direct = 0u;  // this row's columns that the guard sends to FP64 multiply-adds
     for (int c = 0; c < nchunks; ++c) {
       if (__any_sync(0xffffffffu, sh->abort != 0)) {
         ok = false;
@@ -217,7 +291,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-      constexpr int SL = S / HL;  // levels per sum
+      constexpr int SL = S / HL, BITS = HL == 2 ? 8 : 7;  // levels per sum, bits between them
 #pragma unroll
       for (int h = 0; h < HL; ++h)
 #pragma unroll
@@ -231,12 +305,37 @@ __global__ void __launch_bounds__(C::THREADS, 1)
             // |v| <= 2^24: exact in 32 bits, Horner in 64
             long long x = (long long)__float2int_rn(__uint_as_float(v[0][j]));
 #pragma unroll
-            for (int p = 1; p < SL; ++p) x = (x << 7) + (long long)__float2int_rn(__uint_as_float(v[p][j]));
+            for (int p = 1; p < SL; ++p) x = (x << BITS) + (long long)__float2int_rn(__uint_as_float(v[p][j]));
             acc[h][w + j] += x;
           }
         }
       asm volatile("tcgen05.fence::before_thread_sync;");
       mbar_arrive(smem_u32(&sh->accempty));
+    }
+    const int k0 = kb0 * TC_BK, k1 = min(g.K, kb1 * TC_BK);  // (with 8 slices)
+    if (GUARD && ok && nchunks > 0) {
+      const bool got = mbar_wait(smem_u32(&sh->accfull), (uint32_t)(nchunks & 1), kWaitLimit);
+      if (!__all_sync(0xffffffffu, got)) {
+        fail(sh, g.err, 4);
+        ok = false;
+      } else {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const float share = (float)(k1 - k0) / (float)g.K, limit = kGuardDeep * sqrtf((float)g.K) * share;
+#pragma unroll
+        for (int w = 0; w < NC; w += 8) {
+          uint32_t a8[8];
+          tmem_ld8_nowait(tmem + tl + (uint32_t)(j0 + w), a8);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float sxy = __uint_as_float(a8[j]);
+            if ((sxy != 0.f && !(sxy >= limit)) || sh->col_exp[j0 + w + j] == kExpMarked)
+              direct |= 1u << (w + j);
+          }
+        }
+        if (ea == kExpMarked) direct = ~0u;
+        if (AC) direct |= __shfl_xor_sync(0xffffffffu, direct, 1);  // the row's other part
+      }
     }
     if (skip || (ok && __any_sync(0xffffffffu, sh->abort != 0))) ok = false;
     if (ok) {
@@ -250,7 +349,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       const int lr = AC ? (lane >> 1) : lane;
       const int m = AC ? (prow >> 1) : prow;
       const bool neg = g.alpha_pow2 && g.alpha_neg;
-      const int ebase = row_exp(ea) - 7 * (S + 1) + (g.alpha_pow2 ? g.alpha_e : 0);
+      const int ebase = row_exp(ea) - (HL == 2 ? 70 : 7 * (S + 1)) + (g.alpha_pow2 ? g.alpha_e : 0);
       long long coffm = 0;
       if (m < g.M) decomp_tc(g.gmC, m, coffm);
       long long coffT = 0;  // this row as a column
@@ -263,68 +362,94 @@ __global__ void __launch_bounds__(C::THREADS, 1)
 #pragma unroll
       for (int g0 = 0; g0 < NC; g0 += GC) {
         if (g0) __syncwarp();  // the previous group's stores have read the staging area
-        // value of the staged column k from its exact sums
-        auto put = [&](int k, const long long (&re)[HL], const long long (&im)[HL]) {
-          const int jj = (BC ? (j0 + g0) / 2 : j0 + g0) + k;  // logical column within the tile
-          const int eb = sh->col_exp[BC ? 2 * jj : jj];
-          const int E = ebase + row_exp(eb);
-          auto value = [&](const long long (&x)[HL]) {
-            if constexpr (HL == 2)
-              return joined(neg ? -x[0] : x[0], neg ? -x[1] : x[1], E);
-            else
-              return scaled_i64_to_double(neg ? -x[0] : x[0], E);
-          };
-          double2 v = make_double2(value(re), (AC || BC) ? value(im) : 0.0);
-          if (HL == 2 && (ea == kExpMarked || eb == kExpMarked)) {
-            const int n = nt * (BC ? C::BN / 2 : C::BN) + jj;
-            v = make_double2(0.0, 0.0);
-            if (m < g.M && n < g.N) v = direct_dot(g, m, n, zb, kb0 * TC_BK, min(g.K, kb1 * TC_BK));
-            if (g.alpha_pow2) {
-              v.x *= g.ar;
-              v.y *= g.ar;
-            }
-          }
+        auto put = [&](int k, double2 v) {
           if (!g.alpha_pow2) v = make_double2(g.ar * v.x - g.ai * v.y, g.ar * v.y + g.ai * v.x);
           stage[lr * RS + k] = v;
         };
-        if constexpr (AC) {
-          // a row's real and imaginary parts lie in neighbouring lanes: the even
-          // one finishes column k, the odd one k + 1, each with what the other
-          // holds of it
-          static_assert(NL % 2 == 0, "columns in pairs");
+        if constexpr (HL == 2) {
+          // every real row and column has a scale of its own: the sums become
+          // doubles first.  A complex row's two parts lie in neighbouring lanes:
+          // the even one finishes column k, the odd one k + 1, each with what the
+          // other holds of it
+          auto value = [&](int j) {
+            const int E = ebase + row_exp(sh->col_exp[j0 + g0 + j]);
+            const long long h = acc[0][g0 + j], l = acc[HL - 1][g0 + j];
+            return joined<32>(neg ? -h : h, neg ? -l : l, E);
+          };
+          if constexpr (AC) {
+            static_assert(NL % 2 == 0, "columns in pairs");
 #pragma unroll
-          for (int k = 0; k < NL; k += 2) {
-            long long re[HL], im[HL];
-#pragma unroll
-            for (int h = 0; h < HL; ++h) {
+            for (int k = 0; k < NL; k += 2) {
               if constexpr (BC) {
-                const long long* c = &acc[h][g0 + 2 * k];
+                const double x0 = value(2 * k), x1 = value(2 * k + 1), y0 = value(2 * k + 2), y1 = value(2 * k + 3);
+                const double p0 = __shfl_xor_sync(0xffffffffu, odd ? x0 : y0, 1);
+                const double p1 = __shfl_xor_sync(0xffffffffu, odd ? x1 : y1, 1);
+                // even: (re re, re im) own, (im re, im im) the partner's
+                put(k + (odd ? 1 : 0), odd ? make_double2(p0 - y1, p1 + y0) : make_double2(x0 - p1, x1 + p0));
+              } else {
+                const double x = value(k), y = value(k + 1);
+                const double p = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
+                put(k + (odd ? 1 : 0), odd ? make_double2(p, y) : make_double2(x, p));
+              }
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < NL; ++k)
+              put(k, BC ? make_double2(value(2 * k), value(2 * k + 1)) : make_double2(value(k), 0.0));
+          }
+          // what the guard found, four rows of a column at a time
+#pragma unroll 1
+          for (int k = 0; __any_sync(0xffffffffu, direct != 0u) && k < NL; ++k) {
+            const int n = nt * (BC ? C::BN / 2 : C::BN) + (BC ? (j0 + g0) / 2 : j0 + g0) + k;
+            const bool mine = m < g.M && n < g.N && !(AC && odd) && ((direct >> (BC ? g0 + 2 * k : g0 + k)) & (BC ? 3u : 1u));
+            unsigned rows = __ballot_sync(0xffffffffu, mine);
+            __syncwarp();  // the staged values are written
+            while (rows) {
+              int src[kDirect], mm[kDirect];
+#pragma unroll
+              for (int i = 0; i < kDirect; ++i) {
+                src[i] = rows ? __ffs(rows) - 1 : -1;
+                rows &= rows - 1u;
+                mm[i] = __shfl_sync(0xffffffffu, m, max(src[i], src[0]));
+              }
+              double2 s[kDirect];
+              direct_dots<AC, BC>(g, mm, n, zb, k0, k1, s);
+#pragma unroll
+              for (int i = 0; i < kDirect; ++i)
+                if (lane == src[i]) {
+                  if (g.alpha_pow2) s[i] = make_double2(g.ar * s[i].x, g.ar * s[i].y);
+                  put(k, s[i]);
+                }
+            }
+          }
+        } else {
+          // value of the staged column k from its exact sums
+          auto finish = [&](int k, long long re, long long im) {
+            const int E = ebase + row_exp(sh->col_exp[(BC ? 2 * ((j0 + g0) / 2 + k) : j0 + g0 + k)]);
+            put(k, make_double2(scaled_i64_to_double(neg ? -re : re, E),
+                                (AC || BC) ? scaled_i64_to_double(neg ? -im : im, E) : 0.0));
+          };
+          if constexpr (AC) {
+            // (lanes as above; the two parts share a scale, so the sums meet exactly)
+            static_assert(NL % 2 == 0, "columns in pairs");
+#pragma unroll
+            for (int k = 0; k < NL; k += 2) {
+              if constexpr (BC) {
+                const long long* c = &acc[0][g0 + 2 * k];
                 const long long p0 = __shfl_xor_sync(0xffffffffu, odd ? c[0] : c[2], 1);
                 const long long p1 = __shfl_xor_sync(0xffffffffu, odd ? c[1] : c[3], 1);
                 const long long x0 = odd ? c[2] : c[0], x1 = odd ? c[3] : c[1];
-                // even: (re re, re im) own, (im re, im im) the partner's
-                re[h] = odd ? p0 - x1 : x0 - p1;
-                im[h] = odd ? p1 + x0 : x1 + p0;
+                finish(k + (odd ? 1 : 0), odd ? p0 - x1 : x0 - p1, odd ? p1 + x0 : x1 + p0);
               } else {
-                const long long* c = &acc[h][g0 + k];
+                const long long* c = &acc[0][g0 + k];
                 const long long p = __shfl_xor_sync(0xffffffffu, odd ? c[0] : c[1], 1);
                 const long long x = odd ? c[1] : c[0];
-                re[h] = odd ? p : x;
-                im[h] = odd ? x : p;
+                finish(k + (odd ? 1 : 0), odd ? p : x, odd ? x : p);
               }
             }
-            put(k + (odd ? 1 : 0), re, im);
-          }
-        } else {
+          } else {
 #pragma unroll
-          for (int k = 0; k < NL; ++k) {
-            long long re[HL], im[HL];
-#pragma unroll
-            for (int h = 0; h < HL; ++h) {
-              re[h] = BC ? acc[h][g0 + 2 * k] : acc[h][g0 + k];
-              im[h] = BC ? acc[h][g0 + 2 * k + 1] : 0;
-            }
-            put(k, re, im);
+            for (int k = 0; k < NL; ++k) finish(k, BC ? acc[0][g0 + 2 * k] : acc[0][g0 + k], BC ? acc[0][g0 + 2 * k + 1] : 0);
           }
         }
         __syncwarp();
@@ -333,7 +458,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
 #pragma unroll 4
             for (int k = 0; k < NL; ++k) {
               const long long cT = sh->col_offT[j0 + g0 + k];
-              if (cT >= 0) Cr[cT + coffT] = stage[lane * RS + k].x;
+              if (cT >= 0 && m <= nt * C::BN + j0 + g0 + k) Cr[cT + coffT] = stage[lane * RS + k].x;
             }
         }
         // every lane owns a (row, column) pair per pass
@@ -343,6 +468,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
           const long long cm = __shfl_sync(0xffffffffu, coffm, (AC ? 2 * r : r) & 31);
           const long long cn = sh->col_off[(BC ? (j0 + g0) / 2 : j0 + g0) + lc];
           if (r >= nrows || cn < 0) continue;
+          if (SYM && g.sym && m0w + r > nt * C::BN + j0 + g0 + lc) continue;  // stored by the mirror image's tile
           const long long off = cm + cn;
           const double2 v = stage[r * RS + lc];
           if (g.cc) {
@@ -391,8 +517,8 @@ cudaError_t launch_deep_form(const TcArgs& a0, const void* packA, const void* pa
     return cudaErrorInvalidValue;
   if (a.S != C::S || a.rowsB_pad < 1 || a.rowsA_pad % TC_BM != 0) return cudaErrorInvalidValue;
   a.tmem_cols = 512;
-  const CUtensorMap ma = slice_map(packA, a.S, (a.bat_a ? a.nb : 1) * a.rowsA_pad, a.kblocks * TC_BK, TC_BM);
-  const CUtensorMap mb = slice_map(packB, a.S, (a.bat_b ? a.nb : 1) * a.rowsB_pad, a.kblocks * TC_BK, C::BN);
+  const CUtensorMap ma = slice_map(packA, tc_planes(a.S), (a.bat_a ? a.nb : 1) * a.rowsA_pad, a.kblocks * TC_BK, TC_BM);
+  const CUtensorMap mb = slice_map(packB, tc_planes(a.S), (a.bat_b ? a.nb : 1) * a.rowsB_pad, a.kblocks * TC_BK, C::BN);
   // the tiles of the smaller operand side vary fastest: that side stays in L2
   const unsigned mtiles = (unsigned)(a.rowsA_pad / TC_BM);
   const unsigned ntiles = (unsigned)(((long long)a.N * (a.bc ? 2 : 1) + C::BN - 1) / C::BN);

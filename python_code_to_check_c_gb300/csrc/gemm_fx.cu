@@ -31,11 +31,11 @@ int dot_lanes(long long outputs, long long K) {
 // cutting of its operands and its multiply-adds; blocks beyond one per SM
 // share the SM's pipes; splits cost a second pass of the outputs through L2
 // and, when not accumulating, a zeroing launch before.  Dot products: see
-// dot_tile.  The multiply-add and cutting rates lie between those of one
-// tile alone (26 and 2 per clock) and twice them, since the ops of a step run
-// several at a time: with the single-tile rates the propagation at o=10,
-// v=14 took 7.73 ms for 8 steps (too many dot products, which share one
-// narrow pipe), with twice them a step at o=6, v=12 0.55 ms instead of 0.45.
+// dot_tile.  The rates are fitted to whole calls, whose ops run several at a
+// time.  Integer multiply-adds a clock and cutting clocks a number (26, 0.7) against
+// (40, 0.3) and (31, 0.45): a gradient of 8 steps at o=6, v=12 17.7 ms, 22.7 and 26.4;
+// the propagation at o=10, v=14 10.06 ms for 8 steps, 9.81 and 9.96; 60 residuals of
+// o=5..14, v=14..50 32.7 ms in all, 32.9 and 32.8.
 void choose_fx(long long M, long long N, long long K, long long nb, bool ac, bool bc, bool allow_split, int tile,
                int* best_tile, int* best_splits) {
   const double im = (ac && bc) ? 12.0 : (ac || bc) ? 6.0 : 3.0;
@@ -62,10 +62,10 @@ void choose_fx(long long M, long long N, long long K, long long nb, bool ac, boo
     const long long bm = kTiles[t][0], bn = kTiles[t][1];
     const long long tiles = ((M + bm - 1) / bm) * ((N + bn - 1) / bn) * nb;
     for (long long sp = 1; sp <= (allow_split ? std::max<long long>(1, K / 16) : 1); sp += sp < 8 ? 1 : sp / 4) {
-      const long long kper = (K + sp - 1) / sp, chunks = (kper + kChunk - 1) / kChunk;
+      const long long kper = (K + sp - 1) / sp, most = fx_chunk((int)bm, (int)bn, ac, bc), chunks = (kper + most - 1) / most;
       const double fixed = 3400.0 + 1500.0 * (double)(chunks - 1) + (sp > 1 ? 2500.0 : 0.0);
-      const double cut = (double)kper * (double)(bm * (ac ? 2 : 1) + bn * (bc ? 2 : 1)) * 0.3;
-      const double mul = (double)(bm * bn) * (double)kper * im / 40.0;
+      const double cut = (double)kper * (double)(bm * (ac ? 2 : 1) + bn * (bc ? 2 : 1)) * 0.7;
+      const double mul = (double)(bm * bn) * (double)kper * im / 26.0;
       const double out = (double)(bm * bn) * (double)chunks * 1.2 + (sp > 1 ? (double)(bm * bn) * 0.5 : 0.0);
       const double per_sm = std::ceil((double)(tiles * sp) / 152.0);
       const double cost = fixed + cut / (double)chunks + per_sm * (cut + mul + out + 400.0);
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) gemm_fx_kernel(const GemmArgs g
 
 template <bool AC, bool BC, bool CC, int BM, int BN>
 cudaError_t launch_fx_tile(const GemmArgs& g, const FxPlan& f, cudaStream_t st) {
-  constexpr size_t ea = sizeof(typename Limbs<AC>::T), eb = sizeof(typename Limbs<BC>::T);
+  constexpr int kbytes = fx_k_bytes(BM, BN, AC, BC);
   constexpr int kMaxDev = 64;
   static std::once_flag once[kMaxDev];
   static cudaError_t attr_err[kMaxDev] = {};
@@ -98,12 +98,12 @@ cudaError_t launch_fx_tile(const GemmArgs& g, const FxPlan& f, cudaStream_t st) 
   std::call_once(once[dev], [dev] {
     attr_err[dev] =
         cudaFuncSetAttribute(gemm_fx_kernel<AC, BC, CC, BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(limb_bytes(kChunk, BM + 1, ea) + limb_bytes(kChunk, BN + 1, eb)));
+                             kbytes * fx_chunk(BM, BN, AC, BC));
   });
   if (attr_err[dev] != cudaSuccess) return attr_err[dev];
   const long long z = (long long)g.nb * g.nsplit;
   if (f.tiles > 0x7FFFFFFFLL || z > 65535) return cudaErrorInvalidConfiguration;
-  const size_t smem = limb_bytes(f.kc, BM + 1, ea) + limb_bytes(f.kc, BN + 1, eb);
+  const size_t smem = (size_t)kbytes * f.kc;
   gemm_fx_kernel<AC, BC, CC, BM, BN><<<dim3((unsigned)f.tiles, 1, (unsigned)z), kFxThreads, smem, st>>>(g, f);
   return cudaGetLastError();
 }
@@ -175,8 +175,8 @@ cudaError_t fx_plan(const Op& op, GemmArgs& g, FxPlan& f) {
   const int bm = kTiles[f.tile][0], bn = kTiles[f.tile][1];
   f.mtiles = (g.M + bm - 1) / bm;
   f.tiles = (long long)f.mtiles * ((g.N + bn - 1) / bn);
-  const int chunks = (g.kchunk + kChunk - 1) / kChunk;
-  f.kc = std::min(kChunk, (std::min(g.kchunk, std::max(g.K, 1)) + chunks - 1) / chunks);
+  const int most = fx_chunk(bm, bn, f.ac, f.bc), chunks = (g.kchunk + most - 1) / most;
+  f.kc = std::min(most, (std::min(g.kchunk, std::max(g.K, 1)) + chunks - 1) / chunks);
   auto kfast = [&](const long long* ks, const ModeGroup& rows) {
     const int q = g.gk.n - 1;
     if (q < 0 || ks[q] != 1 || g.gk.dim[q] < 4) return 0;

@@ -37,6 +37,7 @@
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp8.h>
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -69,27 +70,46 @@ __device__ __forceinline__ int packed_exponent(unsigned long long mx, int E) {
   return (E > 0 ? E - 1022 : -1022) + kExpBias;
 }
 
+// |x| 2^-e in FP32, x < 2^e; below the normal range zero
+__device__ __forceinline__ float scaled_magnitude(double x, int e) {
+  const uint32_t h = (uint32_t)__double2hiint(x) & 0x7FFFFFFFu;
+  const int E = (int)(h >> 20) - 1023 + 127 - e;
+  return (h >> 20) == 0u || E < 1 ? 0.f : __uint_as_float(((uint32_t)min(E, 126) << 23) | ((h & 0xFFFFFu) << 3) | ((uint32_t)__double2loint(x) >> 29));
+}
+
 // Digits of two neighbouring elements of a packed row (same exponent e), one
 // BF16 pair per slice: out is the packed buffer as BF16 pairs, plane2 the
-// pairs per slice, idx2 the pair's index within a slice.
+// pairs per slice, idx2 the pair's index within a slice, k its place in the row.
 template <int SMAX>
-__device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, size_t idx2, double x0, double x1,
-                                                 int e, int S) {
+__device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, size_t idx2, int k, double x0, double x1,
+                                                  int e, int S) {
   uint32_t h0, l0, h1, l1;
   cut_digits<SMAX>(x0, e, S, h0, l0);
   cut_digits<SMAX>(x1, e, S, h1, l1);
   const uint32_t sgn = (((uint32_t)__double2hiint(x0) >> 16) & 0x8000u) | ((uint32_t)__double2hiint(x1) & 0x80000000u);
   out += idx2;
+  if constexpr (SMAX == 8) {
+    out[0] = digit_pair<24, true>(h0, h1, sgn);
+    out[plane2] = digit_pair<16, false, 8>(h0, h1, sgn);
+    out[2 * plane2] = digit_pair<8, false, 8>(h0, h1, sgn);
+    out[3 * plane2] = digit_pair<0, false, 8>(h0, h1, sgn);
+    out[4 * plane2] = digit_pair<24, false, 8>(l0, l1, sgn);
+    out[5 * plane2] = digit_pair<16, false, 8>(l0, l1, sgn);
+    out[6 * plane2] = digit_pair<8, false, 8>(l0, l1, sgn);
+    out[7 * plane2] = digit_pair<0, false, 8>(l0, l1, sgn);
+    // the range guard's plane (gemm_deep.cu): the magnitudes in 8 bits, only zeros as
+    // zero; a row fills half of a slice's
+    const float f0 = scaled_magnitude(x0, e), f1 = scaled_magnitude(x1, e);
+    const float2 f = make_float2(x0 != 0.0 ? fmaxf(f0, 0x1p-16f) : 0.f, x1 != 0.0 ? fmaxf(f1, 0x1p-16f) : 0.f);
+    const size_t row = 2 * (idx2 - k / 2);  // the row's first BF16
+    reinterpret_cast<uint16_t*>(out - idx2)[16 * plane2 + row + k / 2] = __nv_cvt_float2_to_fp8x2(f, __NV_SATFINITE, __NV_E5M2);
+    return;
+  }
   out[0] = digit_pair<21, true>(h0, h1, sgn);
   if (S > 1) out[plane2] = digit_pair<14, false>(h0, h1, sgn);
   if (S > 2) out[2 * plane2] = digit_pair<7, false>(h0, h1, sgn);
   if (S > 3) out[3 * plane2] = digit_pair<0, false>(h0, h1, sgn);
-  if constexpr (SMAX == 8) {
-    out[4 * plane2] = digit_pair<21, false>(l0, l1, sgn);
-    out[5 * plane2] = digit_pair<14, false>(l0, l1, sgn);
-    out[6 * plane2] = digit_pair<7, false>(l0, l1, sgn);
-    out[7 * plane2] = digit_pair<0, false>(l0, l1, sgn);
-  } else if constexpr (SMAX == 6) {
+  if constexpr (SMAX == 6) {
     if (S > 4) out[4 * plane2] = digit_pair<7, false>(l0, l1, sgn);
     if (S > 5) out[5 * plane2] = digit_pair<0, false>(l0, l1, sgn);
   }
@@ -103,7 +123,8 @@ __device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, s
 // gives them the sign of x:
 //   x 2^-e ~= sum_s q_s 2^(-7s).
 // The real and imaginary rows share e, so that the slice-product epilogue
-// combines re*re - im*im and re*im + im*re exactly in integers.  K padding
+// combines re*re - im*im and re*im + im*re exactly in integers; with 8 slices
+// each has its own (a small imaginary part keeps all of its bits).  K padding
 // is written as zero; padding rows (up to the tile multiple of each batch)
 // are not written at all: they only feed accumulator rows (A) or columns (B)
 // that the product kernel never stores, and their exponent entries only
@@ -144,7 +165,8 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
   const unsigned long long* bits = static_cast<const unsigned long long*>(p.src);
   const double* src = static_cast<const double*>(p.src);
   constexpr unsigned long long kAbs = 0x7FFFFFFFFFFFFFFFull;
-  unsigned long long mx = 0;
+  constexpr int PX = SMAX == TC_DEEP_SLICES ? 2 : 1;  // exponents per logical row
+  unsigned long long mx[PX] = {};
   // four independent loads in flight per thread (complex elements as one 16-byte load)
   constexpr int U = 4;
   for (int k0 = kb + threadIdx.x; k0 < ke; k0 += U * blockDim.x) {
@@ -165,31 +187,46 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
       }
     }
 #pragma unroll
-    for (int j = 0; j < U; ++j) mx = max(mx, max(v[j][0] & kAbs, v[j][1] & kAbs));
+    for (int j = 0; j < U; ++j) {
+      mx[0] = max(mx[0], v[j][0] & kAbs);
+      mx[PX - 1] = max(mx[PX - 1], v[j][1] & kAbs);
+    }
   }
-  for (int d = 16; d > 0; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
-  __shared__ unsigned long long wmax[32];
-  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
+  __shared__ unsigned long long wmax[32][PX];
+#pragma unroll
+  for (int x = 0; x < PX; ++x) {
+    for (int d = 16; d > 0; d >>= 1) mx[x] = max(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], d));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5][x] = mx[x];
+  }
   __syncthreads();
-  mx = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx = max(mx, wmax[w]);
+#pragma unroll
+  for (int x = 0; x < PX; ++x) {
+    mx[x] = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx[x] = max(mx[x], wmax[w][x]);
+  }
   if constexpr (CL > 1) {
     namespace cg = cooperative_groups;
-    __shared__ unsigned long long cmax;
+    __shared__ unsigned long long cmax[PX];
     cg::cluster_group cl = cg::this_cluster();
-    if (threadIdx.x == 0) cmax = mx;
+    if (threadIdx.x == 0)
+      for (int x = 0; x < PX; ++x) cmax[x] = mx[x];
     cl.sync();
-    for (int r = 0; r < CL; ++r) mx = max(mx, *cl.map_shared_rank(&cmax, r));
+#pragma unroll
+    for (int x = 0; x < PX; ++x)
+      for (int r = 0; r < CL; ++r) mx[x] = max(mx[x], cl.map_shared_rank(cmax, r)[x]);
     cl.sync();  // every block has read the others'
   }
-  const int E = (int)(mx >> 52);
-  const int eb = packed_exponent<SMAX>(mx, E);
+  int eb[2], e[2];
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    eb[x] = packed_exponent<SMAX>(mx[x < PX ? x : 0], (int)(mx[x < PX ? x : 0] >> 52));
+    e[x] = row_exp(eb[x]);
+  }
   const size_t prow = (size_t)z * p.rows_pad + (size_t)m * per;  // first packed row
   if (threadIdx.x == 0 && part_k == 0) {
-    p.exps[prow] = eb;
-    if (p.cplx) p.exps[prow + 1] = eb;
+    p.exps[prow] = eb[0];
+    if (p.cplx) p.exps[prow + 1] = eb[1];
   }
-  const int e = row_exp(eb);
   uint32_t* out = static_cast<uint32_t*>(p.out);  // BF16 pairs (K_pad is even)
   const size_t plane2 = (size_t)p.nb * p.rows_pad * (p.K_pad / 2);
   // pass 2 over pairs of neighbouring K indices (one 4-byte store per slice
@@ -219,7 +256,8 @@ __global__ void __launch_bounds__(1024) pack_kernel(const PackArgs p, int tab) {
       const int k = k0 + 2 * j * blockDim.x;
       if (k >= kpe) break;
       for (int part = 0; part < per; ++part)
-        store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, p.S);
+        store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, k, x[j][0][part], x[j][1][part],
+                               part ? e[1] : e[0], p.S);
     }
   }
 }
@@ -246,7 +284,8 @@ __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
   const double* src = static_cast<const double*>(p.src);
   constexpr unsigned long long kAbs = 0x7FFFFFFFFFFFFFFFull;
   double x[KP][2][2];  // [pair][element][part]
-  unsigned long long mx = 0;
+  constexpr int PX = SMAX == TC_DEEP_SLICES ? 2 : 1;  // exponents per logical row
+  unsigned long long mx[PX] = {};
 #pragma unroll
   for (int j = 0; j < KP; ++j)
 #pragma unroll
@@ -265,27 +304,35 @@ __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
           x[j][h][0] = src[el];
         }
       }
-      mx = max(mx, max((unsigned long long)__double_as_longlong(x[j][h][0]) & kAbs,
-                       (unsigned long long)__double_as_longlong(x[j][h][1]) & kAbs));
+      mx[0] = max(mx[0], (unsigned long long)__double_as_longlong(x[j][h][0]) & kAbs);
+      mx[PX - 1] = max(mx[PX - 1], (unsigned long long)__double_as_longlong(x[j][h][1]) & kAbs);
     }
-  for (int d = 16; d > 0; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+#pragma unroll
+  for (int q = 0; q < PX; ++q)
+    for (int d = 16; d > 0; d >>= 1) mx[q] = max(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], d));
   if (W > 1) {
-    __shared__ unsigned long long wmax[8];
-    if (lane == 0) wmax[warp] = mx;
+    __shared__ unsigned long long wmax[8][PX];
+    if (lane == 0)
+      for (int q = 0; q < PX; ++q) wmax[warp][q] = mx[q];
     __syncthreads();  // every thread of the block arrives (no return above)
     const int w0 = warp - wr;
 #pragma unroll
-    for (int w = 0; w < W; ++w) mx = max(mx, wmax[w0 + w]);
+    for (int w = 0; w < W; ++w)
+#pragma unroll
+      for (int q = 0; q < PX; ++q) mx[q] = max(mx[q], wmax[w0 + w][q]);
   }
   if (!live) return;
-  const int E = (int)(mx >> 52);
-  const int eb = packed_exponent<SMAX>(mx, E);
+  int eb[2], e[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    eb[q] = packed_exponent<SMAX>(mx[q < PX ? q : 0], (int)(mx[q < PX ? q : 0] >> 52));
+    e[q] = row_exp(eb[q]);
+  }
   const size_t prow = (size_t)z * p.rows_pad + (size_t)m * per;
   if (wr == 0 && lane == 0) {
-    p.exps[prow] = eb;
-    if (p.cplx) p.exps[prow + 1] = eb;
+    p.exps[prow] = eb[0];
+    if (p.cplx) p.exps[prow + 1] = eb[1];
   }
-  const int e = row_exp(eb);
   uint32_t* out = static_cast<uint32_t*>(p.out);  // BF16 pairs (K_pad is even)
   const size_t plane2 = (size_t)p.nb * p.rows_pad * (p.K_pad / 2);
 #pragma unroll
@@ -293,7 +340,8 @@ __global__ void __launch_bounds__(256) pack_rows_regs_kernel(const PackArgs p) {
     const int k = 2 * (32 * wr + lane + 32 * W * j);
     if (k >= p.K_pad) break;
     for (int part = 0; part < per; ++part)
-      store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, x[j][0][part], x[j][1][part], e, p.S);
+      store_digit_pair<SMAX>(out, plane2, ((prow + part) * p.K_pad + k) / 2, k, x[j][0][part], x[j][1][part],
+                               part ? e[1] : e[0], p.S);
   }
 }
 

@@ -15,6 +15,8 @@ constexpr int TC_CHUNK_KB = 8;               // 512-wide K chunks (exact FP32 le
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;
 constexpr int TC_MAX_SLICES = 6;
 constexpr int TC_DEEP_SLICES = 8;            // the FP64 form's tensor-core contractions
+// planes of a packed operand: its slices, and with 8 the range guard's (gemm_deep.cu)
+constexpr int tc_planes(int S) { return S + (S == TC_DEEP_SLICES ? 1 : 0); }
 
 // Kernel variants: tile width BN (UMMA N), ring depth, TMEM-drain warps and
 // CTAs per SM.  The ring must hold the S slices of one K block (STAGES >= S).
@@ -53,8 +55,8 @@ struct TcPersist {
 // Deep form (gemm_deep.cu): a 128 x BN tile whose S level accumulators fill
 // TMEM, a ring of (A, B) slice pairs, sums over K in the drain warps'
 // registers across exact chunks of CHUNK_KB K blocks: a level of p pairs grows
-// by at most 2 x 128 x 64 + (p - 2) x 64 x 64 per K index and must stay within
-// 2^24.
+// by at most 2 x 128 x 64 + (p - 2) x 64 x 64 per K index (7-bit digits; the 8-bit
+// ones of S = 8: p x 128 x 128) and must stay within 2^24.
 template <int S_, int BN_, int STAGES_>
 struct TcDeep {
   static constexpr int S = S_, BN = BN_, STAGES = STAGES_, EPI = 16;
@@ -62,7 +64,8 @@ struct TcDeep {
   static constexpr int THREADS = 64 + 32 * EPI;
   static constexpr int TAIL = 2048;
   static constexpr int SMEM = 1024 + STAGES * (A_BYTES + B_BYTES) + TAIL;
-  static constexpr int CHUNK_KB = (1 << 24) / ((16384 + (S > 2 ? S - 2 : 0) * 4096) * TC_BK);
+  static constexpr int CHUNK_KB =
+      (1 << 24) / ((S == TC_DEEP_SLICES ? S * 16384 : 16384 + (S > 2 ? S - 2 : 0) * 4096) * TC_BK);
   static_assert(S * BN <= 512 && STAGES >= S, "TMEM columns, ring");
 };
 

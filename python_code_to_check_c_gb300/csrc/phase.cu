@@ -667,8 +667,7 @@ void PhaseKernel::build(const Program& p, Program::Phase ph, std::vector<void*>&
         r.gemm.f = f;
         tiles = f.tiles * g.nb * g.nsplit;
         const int bm = kTiles[f.tile][0], bn = kTiles[f.tile][1];
-        smem_ = std::max(smem_, limb_bytes(f.kc, bm + 1, f.ac ? sizeof(int4) : sizeof(int2)) +
-                                    limb_bytes(f.kc, bn + 1, f.bc ? sizeof(int4) : sizeof(int2)));
+        smem_ = std::max(smem_, (size_t)fx_k_bytes(bm, bn, f.ac, f.bc) * f.kc);
         const size_t w = offsetof(PhaseOp, gemm) + offsetof(GemmRec, g);
         pa = w + offsetof(GemmArgs, A);
         pb = w + offsetof(GemmArgs, B);
@@ -790,7 +789,7 @@ cudaError_t PhaseKernel::launch(const std::vector<void*>& bases, int blocks, cud
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
   std::call_once(once[dev], [dev] {
-    const int most = (int)(2 * limb_bytes(kChunk, 17, sizeof(int4)));
+    const int most = fx_k_bytes(16, 16, true, true) * fx_chunk(16, 16, true, true);
     int sms = 0, per = 0;
     cudaError_t e = cudaFuncSetAttribute(phase_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

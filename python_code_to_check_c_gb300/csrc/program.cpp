@@ -909,15 +909,11 @@ static void merge_pack_modes(ModeGroup& g) {
 
 // K splits of a contraction of the FP64 form on the tensor cores (deep form),
 // 0 where the integer pipe is expected to be faster.  Model, in microseconds:
-// the fixed-point tiles reach 4.3 real multiply-adds per clock and SM in large
-// grids, 3.0 at the sizes where the choice lies; a deep
-// tile takes 6.5 per K block and 13 for its first loads and its drain, one per
-// SM; packing an operand that is not an integral block 3 and its traffic at 3
-// TB/s.  Measured at o=10, v=38: the ladder (1444 x 200 x 1444 real) 320 us
-// on the integer pipe, 70 deep; residuals T2, L1, L2 of one trajectory in us with
-// 4.3, 3.0, 2.2 here: 842 852 704, 764 794 630, 783 787 610; at o=9, v=31 570 539
-// 445, 557 525 436, 566 537 456; at o=14, v=20 627 554 473, 573 504 449, 573 503
-// 445.
+// the fixed-point tiles reach 2.2 real multiply-adds per clock and SM at the sizes
+// where the choice lies (3.0, 2.2 and 1.7 here: residuals of 20 systems, o = 5..14 and
+// v = 14..50, within 1 % of each other); a deep tile takes 7.3 per K block and 15 for
+// its first loads, its drain and the guard, one per SM; packing an operand that is not
+// an integral block 3 and its traffic at 3 TB/s.
 static int deep_splits(const Op& op) {
   constexpr int BM = 128, BN = 64, BK = 64, kMinK = 32;
   const GemmArgs& g = op.g;
@@ -925,13 +921,14 @@ static int deep_splits(const Op& op) {
   const bool ac = op.dta == C64, bc = op.dtb == C64;
   if (g.K < kMinK || (op.dtc != C64 && (ac || bc))) return 0;
   const double ra = (double)g.M * (ac ? 2 : 1), rb = (double)g.N * (bc ? 2 : 1);
-  const double fx = 6.0 + ra * rb * K * nb / (152.0 * 3.0 * 2070.0);
+  const double fx = 6.0 + ra * rb * K * nb / (152.0 * 2.2 * 2070.0);
   const long long tiles = (long long)(std::ceil(ra / BM) * std::ceil(rb / BN) * nb), kb = (g.K + BK - 1) / BK;
   double best = 1e300;
   int splits = 0;
-  for (long long sp = 1; sp <= std::min<long long>(kb, 64); ++sp) {
+  // (at most 4096 K blocks a CTA: its 64-bit sums then hold any digits)
+  for (long long sp = (kb + 4095) / 4096; sp <= std::max<long long>((kb + 4095) / 4096, std::min<long long>(kb, 64)); ++sp) {
     const double per = (double)((kb + sp - 1) / sp);
-    const double t = std::ceil((double)(tiles * sp) / 152.0) * (per * 6.5 + 13.0) + (sp > 1 ? 2.0 : 0.0);
+    const double t = std::ceil((double)(tiles * sp) / 152.0) * (per * 7.3 + 15.0) + (sp > 1 ? 2.0 : 0.0);
     if (t < best * 0.999) {
       best = t;
       splits = (int)sp;
@@ -939,7 +936,7 @@ static int deep_splits(const Op& op) {
   }
   double deep = best + 4.0;
   auto pack = [&](int slot, double rows, int dt) {
-    if (slot != S_TEI) deep += 3.0 + rows * K * ((double)elem_bytes(dt) + 2.0 * TC_DEEP_SLICES * (dt == C64 ? 2 : 1)) / 3e6;
+    if (slot != S_TEI) deep += 3.0 + rows * K * ((double)elem_bytes(dt) + 2.0 * tc_planes(TC_DEEP_SLICES) * (dt == C64 ? 2 : 1)) / 3e6;
   };
   pack(op.sa, (double)g.M * (g.bsA ? nb : 1), op.dta);
   pack(op.sb, (double)g.N * (g.bsB ? nb : 1), op.dtb);
@@ -955,7 +952,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     double need = 0.0;
     for (const auto& op : ops)
       if (op.kind == OP_GEMM && deep_splits(op) > 0) {
-        const double nb = std::max(op.g.nb, 1), kp = (double)rup(op.g.K, 64) * 2.0 * S;
+        const double nb = std::max(op.g.nb, 1), kp = (double)rup(op.g.K, 64) * 2.0 * tc_planes(S);
         need += kp * ((double)rup(op.g.M * (op.dta == C64 ? 2LL : 1LL), 128) * (op.g.bsA ? nb : 1.0) +
                       (double)rup(op.g.N * (op.dtb == C64 ? 2LL : 1LL), 64) * (op.g.bsB ? nb : 1.0));
       }
@@ -1037,7 +1034,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     const int nbt = std::max(op.g.nb, 1);
     const int nbA = (nbt > 1 && op.g.bsA != 0) ? nbt : 1, nbB = (nbt > 1 && op.g.bsB != 0) ? nbt : 1;
     auto packed_slot = [&](const std::string& nm, long long rows, long long& exp_off) {
-      exp_off = rup((long long)S * rows * Kp * 2, 256);
+      exp_off = rup((long long)tc_planes(S) * rows * Kp * 2, 256);
       int d1[1] = {(int)0};
       const long long bytes = exp_off + rup(rows * 4, 256);
       if (bytes > (1LL << 31) - 1) {
@@ -1071,7 +1068,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     pa.pk_dt = op.dta;
     pa.reads = {op.sa};
     pa.write = pa.pk_dst;
-    pa.bytes = nbA * (M * K * elem_bytes(op.dta) + (long long)S * rA * Kp * 2);
+    pa.bytes = nbA * (M * K * elem_bytes(op.dta) + (long long)tc_planes(S) * rA * Kp * 2);
     // B: rows = N modes (strides g.gn.s0), K modes strides g.gk.s1
     pb.pk = PackArgs{};
     pb.pk.cplx = bc;
@@ -1089,7 +1086,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     pb.pk_off = op.ob;
     pb.pk_dt = op.dtb;
     pb.reads = {op.sb};
-    pb.bytes = nbB * (N * K * elem_bytes(op.dtb) + (long long)S * rB * Kp * 2);
+    pb.bytes = nbB * (N * K * elem_bytes(op.dtb) + (long long)tc_planes(S) * rB * Kp * 2);
     merge_pack_modes(pa.pk.gr);
     merge_pack_modes(pa.pk.gk);
     merge_pack_modes(pb.pk.gr);
@@ -1205,7 +1202,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
     t.zeroed = a.acc || a.atomic;  // split K is allowed (a zero op precedes when not accumulating)
     // short K: the narrow variant (two CTAs per SM overlap their latencies)
     a.variant = deep || long_k ? 3 : persist ? 2 : (a.kb_per_split == 1 && S <= 5) ? 1 : 0;
-    t.bytes = (long long)S * (nbA * rA + nbB * rB) * Kp * 2 + nbt * M * N * elem_bytes(op.dtc);
+    t.bytes = (long long)tc_planes(S) * (nbA * rA + nbB * rB) * Kp * 2 + nbt * M * N * elem_bytes(op.dtc);
     t.reads = {pa.pk_dst, pb.pk_dst};
     if (deep) {  // the drain reads the operands of rows that digits cannot hold
       t.tc_sa = op.sa;

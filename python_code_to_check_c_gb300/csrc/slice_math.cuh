@@ -38,7 +38,7 @@ constexpr int kExpMarked = 1 << 30;  // a row that digits cannot hold (deep form
 __device__ __forceinline__ int row_exp(int biased) { return biased > 0 ? biased - kExpBias : 0; }
 
 // |x| 2^(nbits - e) rounded to the nearest integer (ties away) from the bits of x
-// (no FP64 arithmetic).  Requires |x| < 2^e and nbits <= 56: at most 2^nbits.
+// (no FP64 arithmetic).  Requires |x| < 2^e and nbits <= 63: at most 2^nbits.
 __device__ __forceinline__ unsigned long long fixed_point_rounded(double x, int e, int nbits) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
   const int E = (int)(u >> 52);
@@ -54,7 +54,8 @@ __device__ __forceinline__ unsigned long long fixed_point_rounded(double x, int 
 // in two words: hi holds digits 1 .. 4, the first in [0, 128] at bit 21, lo the
 // others.  The digits after the first are biased by 64: f plus 64 at each of their
 // places has them in its 7-bit fields, carries included.  SMAX = 4 and 6 cut after
-// 7 S bits, 8 rounds to 56.  |x| < 2^e; integer operations only, of 32 bits for
+// 7 S bits; SMAX = 8 has digits of 8 bits (the first in [0, 128] at bit 24, the
+// others biased by 128) and rounds to 63.  |x| < 2^e; integer operations only, of 32 bits for
 // SMAX = 4.  (Packing 6.9 M numbers, o=10, v=38 with 24 trajectories: 51 us with
 // digits cut one by one in 64 bits, 38 so, 16 for their bytes.)
 template <int SMAX>
@@ -62,9 +63,9 @@ __device__ __forceinline__ void cut_digits(double x, int e, int S, uint32_t& hi,
   constexpr uint32_t kB3 = 64u * (1u + (1u << 7) + (1u << 14)), kB2 = 64u * (1u + (1u << 7));
   lo = 0u;
   if constexpr (SMAX == 8) {
-    const unsigned long long f = fixed_point_rounded(x, e, 56);
-    lo = (uint32_t)(f & 0xFFFFFFFull) + kB3 + (64u << 21);
-    hi = (uint32_t)(f >> 28) + (lo >> 28) + kB3;
+    const unsigned long long f = fixed_point_rounded(x, e, 63) + 0x0080808080808080ull;
+    lo = (uint32_t)f;
+    hi = (uint32_t)(f >> 32);
   } else {
     const uint32_t xh = (uint32_t)__double2hiint(x) & 0x7FFFFFFFu, xl = (uint32_t)__double2loint(x);
     const int E = (int)(xh >> 20);
@@ -90,12 +91,18 @@ __device__ __forceinline__ void cut_digits(double x, int e, int S, uint32_t& hi,
 // A digit of two neighbouring elements as a BF16 pair, w0's in the low half (the
 // lower address): 0x4300 + u is the BF16 number 128 + u (u <= 128), so the
 // subtraction of the bias is exact.  sgn: the elements' signs in bits 15 and 31.
-template <int BIT, bool TOP>
+// BITS = 8: u + 128 with u's upper bit in the bias, 256 or 128.
+template <int BIT, bool TOP, int BITS = 7>
 __device__ __forceinline__ uint32_t digit_pair(uint32_t w0, uint32_t w1, uint32_t sgn) {
-  constexpr uint32_t m = TOP ? 0xFFu : 0x7Fu;
+  constexpr uint32_t m = TOP || BITS == 8 ? 0xFFu : 0x7Fu;
   const uint32_t a = w0 >> BIT, b = BIT <= 16 ? w1 << (16 - BIT) : w1 >> (BIT - 16);
-  const uint32_t p = (a & m) | (b & (m << 16)) | 0x43004300u;
-  const uint32_t bias = TOP ? 0x43004300u : 0x43404340u;  // 128, 192
+  uint32_t p = (a & m) | (b & (m << 16));
+  uint32_t bias = TOP ? 0x43004300u : 0x43404340u;  // 128, 192
+  if (!TOP && BITS == 8) {
+    bias = (p & 0x00800080u) ^ 0x43804380u;
+    p &= 0x007F007Fu;
+  }
+  p |= 0x43004300u;
   const __nv_bfloat162 r = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&p), *reinterpret_cast<const __nv_bfloat162*>(&bias));
   return *reinterpret_cast<const uint32_t*>(&r) ^ sgn;
 }

@@ -73,6 +73,13 @@ __device__ __forceinline__ void umma_warp(uint32_t d, uint64_t a, uint64_t b, ui
       " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
       "l"(a), "l"(b), "r"(id), "r"(acc), "r"(lane_on));
 }
+// 8-bit floating-point operands (E5M2, 32 K a step), the same descriptor bits as idesc_bf16
+__device__ __forceinline__ void umma_f8_warp(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc, uint32_t lane_on) {
+  asm volatile(
+      "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 e, %5, 0;\n"
+      " @e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(d),
+      "l"(a), "l"(b), "r"(id), "r"(acc), "r"(lane_on));
+}
 __device__ __forceinline__ void umma_commit_warp(uint32_t mbar, uint32_t lane_on) {
   asm volatile(
       "{\n .reg .pred e;\n setp.ne.b32 e, %1, 0;\n"
@@ -188,6 +195,26 @@ struct PairRing {
     st0 += S;
     if (st0 >= STAGES) {
       st0 -= STAGES;
+      ph ^= 1u;
+    }
+    return ok;
+  }
+  // The range guard's plane of 128 K (64 where `half`) into columns [0, BN).
+  template <int BN>
+  __device__ __forceinline__ bool guard(uint32_t tmem, uint32_t id, bool first, bool half, uint32_t on) {
+    const bool ok = mbar_wait_warp(full0 + 8 * st0, ph, kWaitLimit);
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (ok) {
+      const uint32_t la = a0 + st0 * (A_BYTES >> 4), lb = b0 + st0 * (B_BYTES >> 4);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < 2 || !half)
+          umma_f8_warp(tmem, hi64 | (uint64_t)(la + 2 * k), hi64 | (uint64_t)(lb + 2 * k), id, (k == 0 && first) ? 0u : 1u,
+                       on);
+      umma_commit_warp(empty0 + 8 * st0, on);
+    }
+    if (++st0 == STAGES) {
+      st0 = 0;
       ph ^= 1u;
     }
     return ok;
