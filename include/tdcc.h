@@ -100,7 +100,11 @@ long long tdcc_launch_count(void);
 /* Builds a system from device-resident integrals (replaces
    CCSD_Helper.__init__ / TEI_MO / F_MO / Defd_dipole,
    CCSD_Helper.py:26-54, 57-93, 970-980).  tei/fock/mu are borrowed: they
-   must stay valid until tdcc_system_destroy.  Allocates workspace lazily.  */
+   must stay valid until tdcc_system_destroy.  The FP64 form reads them at
+   each call, as they are in its stream's order; the mixed form packs blocks of
+   tei when a right-hand side is first used and keeps them (until
+   tdcc_set_precision or another policy call changes something): write tei
+   before that.  Allocates workspace lazily.                               */
 int tdcc_system_create(int o, int v, const double* tei, const double* fock,
                        const double* mu, int n_mu, tdcc_system* out);
 int tdcc_system_destroy(tdcc_system s);

@@ -53,17 +53,24 @@ struct ProgInst {
   std::vector<void*> owned;  // this program's workspace allocations
   long long bytes = 0;
   bool setup_done = false;   // integral-only ops (e.g. packed integral blocks) ran
+  bool each_call = false;    // FP64 form: they run again in every call, so that it reads the integrals as they are
   DagExec dag;               // streams/events for concurrent execution of the ops
   PhaseKernel phase[5];      // phases that run as one launch (small FP64 programs)
   void build_phases(std::initializer_list<Program::Phase> phs) {
     for (Program::Phase ph : phs) phase[ph].build(*prog, ph, owned, bytes);
   }
-  // runs the integral-only ops once, eagerly, on `st`
+  // runs the integral-only ops eagerly on `st`, where they have not run yet (FP64
+  // form: in this call)
   cudaError_t setup(cudaStream_t st) {
     if (setup_done) return cudaSuccess;
-    const cudaError_t e = prog->run(bases, st, Program::SETUP);
+    const cudaError_t e = prog->run_dag(bases, st, Program::SETUP, dag);
     if (e == cudaSuccess) setup_done = true;
     return e;
+  }
+  bool has_setup() const {
+    for (const Op& op : prog->ops)
+      if (op.is_const) return true;
+    return false;
   }
   ~ProgInst() {
     dag.destroy();
@@ -308,6 +315,7 @@ ProgInst& get_rhs(tdcc_system s, int method, int block) {
   p.analyse({S_T1 + block, S_F});
   if (s->share_mem && workspace_estimate(p) > (s->share_min < 0 ? kShareMinBytes : s->share_min)) p.plan_memory();
   pi->bases.assign(p.slots.size(), nullptr);
+  pi->each_call = s->prec_mode == TDCC_PREC_FP64;
   pi->bytes = p.allocate(pi->bases, pi->owned);
   s->ws_bytes += pi->bytes;
   bind_fixed(s, pi->bases);
@@ -656,6 +664,12 @@ void reset_programs(tdcc_system s) {
     }
 }
 
+// the start of a call: what the FP64 form packs of the integrals is packed anew
+void begin_call(tdcc_system s) {
+  for (auto* slot : all_programs(s))
+    if (*slot && (*slot)->each_call) (*slot)->setup_done = false;
+}
+
 bool valid_method(int m) { return m == TDCC_CCSD || m == TDCC_CC2; }
 
 }  // namespace
@@ -852,6 +866,7 @@ int tdcc_ground_state(tdcc_system s, int method, int mode, void* t1, void* t2, v
     };
     d2d(x1, mode == 0 ? t1 : l1, n1 * 16);
     d2d(x2, mode == 0 ? t2 : l2, n2 * 16);
+    begin_call(s);
     ProgInst& P1 = get_rhs(s, method, mode == 0 ? TDCC_T1 : TDCC_L1);
     ProgInst& P2 = get_rhs(s, method, mode == 0 ? TDCC_T2 : TDCC_L2);
     double last_res = INFINITY;
@@ -1097,8 +1112,14 @@ int tdcc_rhs(tdcc_system s, int method, int block, const void* t1, const void* t
     B[S_L2] = const_cast<void*>(l2);
     B[S_F] = const_cast<void*>(F);
     B[S_OUT] = out;
-    cudaError_t e = pi.setup(static_cast<cudaStream_t>(stream));
-    if (e == cudaSuccess) e = pi.exec(static_cast<cudaStream_t>(stream), Program::DYNAMIC);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t e = cudaSuccess;
+    if (pi.each_call && pi.has_setup()) {  // the integrals' packing beside the other ops
+      e = pi.exec(st, Program::ALL);
+    } else {
+      e = pi.setup(st);
+      if (e == cudaSuccess) e = pi.exec(st, Program::DYNAMIC);
+    }
     if (e != cudaSuccess) return TDCC_ERR_CUDA;
   } catch (const std::exception& ex) {
     return fail(TDCC_ERR_CUDA, ex.what());
@@ -1141,6 +1162,7 @@ int tdcc_rk4_step(tdcc_system s, int method, const void* t1, const void* t2, con
     CK(cudaEventRecord(s->ev_user, user));
     CK(cudaStreamWaitEvent(s->main, s->ev_user, 0));
     set_ctx(s, t_prev, dt, field, s->main);
+    begin_call(s);
     double2* in[4] = {(double2*)t1, (double2*)t2, (double2*)l1, (double2*)l2};
     double2* tmp[4] = {s->st[1][0], s->st[1][1], s->st[1][2], s->st[1][3]};
     run_step(s, method, in, tmp, dt, precs, nullptr);
@@ -1181,6 +1203,9 @@ int propagate_impl(tdcc_system s, int method, void* t1, void* t2, void* l1, void
     for (int b = 0; b < 4; ++b)
       CK(cudaMemcpyAsync(s->st[0][b], st_user[b], s->nelb(b) * sizeof(double2), cudaMemcpyDeviceToDevice, s->main));
     set_ctx(s, t0, dt, field, s->main);
+    // build programs (allocations) before capture; the step graphs read what their
+    // integral-only ops leave
+    for (int b = 0; b < 4; ++b) CK(get_rhs(s, method, b).setup(s->main));
     // (re)capture the two ping-pong step graphs when the configuration changed
     if (s->g_method != method || s->g_dt != dt || s->g_precs != precs || s->g_prec_mode != s->prec_mode ||
         s->g_traj != mu_traj || !s->gexec[0] || s->g_store_set != (ss != nullptr) ||
@@ -1190,8 +1215,6 @@ int propagate_impl(tdcc_system s, int method, void* t1, void* t2, void* l1, void
           cudaGraphExecDestroy(g);
           g = nullptr;
         }
-      // build programs (allocations) before capture
-      for (int b = 0; b < 4; ++b) CK(get_rhs(s, method, b).setup(s->main));
       CK(cudaStreamSynchronize(s->main));
       get_density(s);
       const long long before_capture = launch_count();
@@ -1265,6 +1288,7 @@ extern "C" {
 int tdcc_propagate(tdcc_system s, int method, void* t1, void* t2, void* l1, void* l2, double t0,
                    double dt, int nsteps, int precs, const tdcc_field* field, void* mu_traj,
                    void* stream) {
+  if (s) begin_call(s);
   return propagate_impl(s, method, t1, t2, l1, l2, t0, dt, nsteps, precs, field, mu_traj, stream, 1, nullptr);
 }
 
@@ -1423,14 +1447,15 @@ int tdcc_adjoint(tdcc_system s, int method, const void* t1, const void* t2, cons
   };
   try {
     ensure_rk(s);
-    for (int b = 0; b < 4; ++b) {
-      get_adj(s, method, b);
-      CK(get_rhs(s, method, b).setup(s->main));
-    }
-    get_adj(s, method, 4);
     cudaStream_t user = static_cast<cudaStream_t>(stream), m = s->main;
     CK(cudaEventRecord(s->ev_user, user));
     CK(cudaStreamWaitEvent(m, s->ev_user, 0));
+    begin_call(s);
+    for (int b = 0; b < 4; ++b) {
+      get_adj(s, method, b);
+      CK(get_rhs(s, method, b).setup(m));
+    }
+    get_adj(s, method, 4);
     auto nel = [&](int b) { return (size_t)s->nelb(b); };
     const size_t maxel = nel(1);
     // ---- working memory for the call ----
@@ -1695,6 +1720,7 @@ int tdcc_profile_step(tdcc_system s, int method, const void* t1, const void* t2,
     ensure_rk(s);
     CK(cudaDeviceSynchronize());
     set_ctx(s, t_prev, dt, field, s->main);
+    begin_call(s);
     double2* in[4] = {(double2*)t1, (double2*)t2, (double2*)l1, (double2*)l2};
     double2* tmp[4] = {s->st[1][0], s->st[1][1], s->st[1][2], s->st[1][3]};
     run_step(s, method, in, tmp, dt, precs, nullptr, &pf);

@@ -226,7 +226,7 @@ struct Op {
   std::vector<int> reads;
   int write = -1;
   bool varying = true;
-  bool is_const = false;   // depends on the integrals only: run once per system
+  bool is_const = false;   // depends on the integrals only: run once per system (FP64 form: per call)
 };
 
 struct SlotInfo {
@@ -322,7 +322,7 @@ class Program {
   long long allocate(std::vector<void*>& bases, std::vector<void*>& owned, size_t first = 0, bool zero = false);
 
   // ALL: every op.  SETUP: ops that depend on the integrals only (once per
-  // system).  PROLOGUE: the rest of the ops independent of the varying
+  // system; FP64 form: once per call).  PROLOGUE: the rest of the ops independent of the varying
   // slots (once per RK4 step).  STAGE: ops on the varying slots.  DYNAMIC:
   // every op except SETUP ones.
   enum Phase { ALL = 0, PROLOGUE = 1, STAGE = 2, SETUP = 3, DYNAMIC = 4 };
