@@ -186,9 +186,15 @@ int tdcc_set_memory_sharing(tdcc_system s, long long min_bytes);
 int tdcc_set_adjoint_store(tdcc_system s, int mode);
 
 /* Synchronises the device and reports TDCC_ERR_CUDA if a kernel of this
-   system recorded an error (a tensor-core kernel whose bounded wait
-   expired); clears the flag.                                              */
+   system recorded an error (a kernel whose bounded wait expired); clears the
+   flag.  In the FP64 form such a kernel also leaves NaN in what it was to
+   write, so that no call passes stale numbers on.                          */
 int tdcc_check_errors(tdcc_system s);
+
+/* Diagnostics: the polls after which the FP64 form's kernels give up a wait
+   (0: their own limit; negative: every wait gives up at once, which tests the
+   path above without a hang).                                              */
+int tdcc_set_wait_limit(tdcc_system s, int polls);
 
 /* Bytes of device workspace currently held by the system.                 */
 long long tdcc_workspace_bytes(tdcc_system s);

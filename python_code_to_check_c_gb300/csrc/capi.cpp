@@ -59,6 +59,11 @@ struct ProgInst {
   void build_phases(std::initializer_list<Program::Phase> phs) {
     for (Program::Phase ph : phs) phase[ph].build(*prog, ph, owned, bytes);
   }
+  void set_wait_limit(int polls) {
+    for (Op& op : prog->ops)
+      if (op.kind == OP_TCGEMM) op.tc.wait = polls;
+    for (PhaseKernel& k : phase) k.wait = polls;
+  }
   // runs the integral-only ops eagerly on `st`, where they have not run yet (FP64
   // form: in this call)
   cudaError_t setup(cudaStream_t st) {
@@ -158,6 +163,7 @@ struct tdcc_system_s {
   int tc_min_mn = kTcMinMN;
   int simt_max_k = kSimtMaxKDefault;   // short contractions on the FP32 pipe (mixed mode)
   long long simt_min_macs = kSimtMinMacs;
+  int wait_limit = 0;                  // polls of the kernels' bounded waits (0: their own limits)
   int device = 0;
   int nb = 1;                       // trajectories advanced together
   bool share_mem = true;            // workspace slots with disjoint lifetimes share memory (off once
@@ -323,6 +329,7 @@ ProgInst& get_rhs(tdcc_system s, int method, int block) {
   const long long ws0 = pi->bytes;
   pi->build_phases({Program::PROLOGUE, Program::STAGE, Program::DYNAMIC});
   s->ws_bytes += pi->bytes - ws0;
+  pi->set_wait_limit(s->wait_limit);
   slot = std::move(pi);
   return *slot;
 }
@@ -346,6 +353,7 @@ ProgInst& get_density(tdcc_system s) {
   const long long ws0 = pi->bytes;
   pi->build_phases({Program::ALL});
   s->ws_bytes += pi->bytes - ws0;
+  pi->set_wait_limit(s->wait_limit);
   s->dens = std::move(pi);
   return *s->dens;
 }
@@ -400,6 +408,7 @@ ProgInst& get_adj(tdcc_system s, int method, int block) {
     pi->act_pro8 = ap.pro8;
     pi->act_stage8 = ap.stage8;
   }
+  pi->set_wait_limit(s->wait_limit);
   slot = std::move(pi);
   return *slot;
 }
@@ -769,6 +778,20 @@ int tdcc_set_precision(tdcc_system s, int mode, int slices) {
   reset_programs(s);
   s->prec_mode = mode;
   s->slices = slices;
+  return TDCC_OK;
+}
+
+int tdcc_set_wait_limit(tdcc_system s, int polls) {
+  if (!s) return fail(TDCC_ERR_ARG, "null system");
+  cudaDeviceSynchronize();
+  s->wait_limit = polls;
+  for (auto* slot : all_programs(s))
+    if (*slot) (*slot)->set_wait_limit(polls);
+  for (auto& g : s->gexec)  // captured with the limits before
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
   return TDCC_OK;
 }
 

@@ -176,6 +176,7 @@ struct TcArgs {
   ModeGroup gmA, gnB, gkAB;  // offsets in s0 (A / B); gkAB: A in s0, B in s1
   long long bsA, bsB;
   int K;
+  int wait;  // polls of a wait (deep form; 0: kTcWaitLimit; negative: none, for tests)
   int sym;  // deep form, real, B is A: tiles on and above the diagonal only, each stored both ways
 };
 

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
   const int kb1 = skip ? kb0 : min(g.kblocks, kb0 + g.kb_per_split);
   const int rowA0 = g.bat_a ? zb * g.rowsA_pad : 0, rowB0 = g.bat_b ? zb * g.rowsB_pad : 0;
   const int nchunks = (kb1 - kb0 + C::CHUNK_KB - 1) / C::CHUNK_KB;
+  const int wait = g.wait == 0 ? kWaitLimit : g.wait;
   // 8 slices: digits of 8 bits, a scale for each real row; after the chunks, the range
   // guard over the same K
   constexpr bool GUARD = S == TC_DEEP_SLICES;
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       int it = 0;
       auto load = [&](int kb, int s) {
         const int st = it % C::STAGES;
-        if (!mbar_wait(smem_u32(&sh->empty[st]), (uint32_t)((it / C::STAGES) & 1) ^ 1u, kWaitLimit)) {
+        if (!mbar_wait(smem_u32(&sh->empty[st]), (uint32_t)((it / C::STAGES) & 1) ^ 1u, wait)) {
           fail(sh, g.err, 1);
           return;
         }
@@ -216,9 +217,10 @@ __global__ void __launch_bounds__(C::THREADS, 1)
     constexpr uint32_t id = idesc_bf16(TC_BM, C::BN);
     const uint32_t on = lane == 0 ? 1u : 0u;
     PairRing<C::STAGES, C::A_BYTES, C::B_BYTES> ring(stA, stB, &sh->full[0], &sh->empty[0]);
+    ring.wait = wait;
     bool ok = true;
     for (int c = 0; c < nchunks && ok; ++c) {
-      if (c > 0 && !mbar_wait_warp(smem_u32(&sh->accempty), (uint32_t)((c - 1) & 1), kWaitLimit)) {
+      if (c > 0 && !mbar_wait_warp(smem_u32(&sh->accempty), (uint32_t)((c - 1) & 1), wait)) {
         fail(sh, g.err, 2);
         break;
       }
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       ok = __all_sync(0xffffffffu, ok && sh->abort == 0) != 0;
     }
     if (GUARD && ok && nchunks > 0) {
-      ok = mbar_wait_warp(smem_u32(&sh->accempty), (uint32_t)((nchunks - 1) & 1), kWaitLimit);
+      ok = mbar_wait_warp(smem_u32(&sh->accempty), (uint32_t)((nchunks - 1) & 1), wait);
       if (!ok) fail(sh, g.err, 2);
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
         ok = false;
         break;
       }
-      const bool got = mbar_wait(smem_u32(&sh->accfull), (uint32_t)(c & 1), kWaitLimit);
+      const bool got = mbar_wait(smem_u32(&sh->accfull), (uint32_t)(c & 1), wait);
       if (!__all_sync(0xffffffffu, got)) {
         fail(sh, g.err, 4);
         ok = false;
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
     }
     const int k0 = kb0 * TC_BK, k1 = min(g.K, kb1 * TC_BK);  // (with 8 slices)
     if (GUARD && ok && nchunks > 0) {
-      const bool got = mbar_wait(smem_u32(&sh->accfull), (uint32_t)(nchunks & 1), kWaitLimit);
+      const bool got = mbar_wait(smem_u32(&sh->accfull), (uint32_t)(nchunks & 1), wait);
       if (!__all_sync(0xffffffffu, got)) {
         fail(sh, g.err, 4);
         ok = false;
@@ -337,8 +339,11 @@ __global__ void __launch_bounds__(C::THREADS, 1)
         if (AC) direct |= __shfl_xor_sync(0xffffffffu, direct, 1);  // the row's other part
       }
     }
-    if (skip || (ok && __any_sync(0xffffffffu, sh->abort != 0))) ok = false;
-    if (ok) {
+    if (__any_sync(0xffffffffu, sh->abort != 0)) ok = false;
+    // a wait that ran out leaves no numbers behind: NaN, straight from the registers
+    // (loads may still be on their way to the ring)
+    const bool lost = !ok;
+    if (!skip) {
       const bool odd = AC && (lane & 1);
       constexpr int GC = NC > 24 ? NC / 2 : NC;  // packed columns staged at a time
       constexpr int NL = BC ? GC / 2 : GC;       // logical columns of them
@@ -359,10 +364,12 @@ __global__ void __launch_bounds__(C::THREADS, 1)
       const int m0w = AC ? ((mt * TC_BM + q * 32) >> 1) : (mt * TC_BM + q * 32);
       const int nrows = min(rows_out, g.M - m0w);
       const bool red = g.acc || g.atomic;
+      const double nan = __longlong_as_double(0x7FF8000000000000ll);
 #pragma unroll
       for (int g0 = 0; g0 < NC; g0 += GC) {
         if (g0) __syncwarp();  // the previous group's stores have read the staging area
         auto put = [&](int k, double2 v) {
+          if (lost) return;
           if (!g.alpha_pow2) v = make_double2(g.ar * v.x - g.ai * v.y, g.ar * v.y + g.ai * v.x);
           stage[lr * RS + k] = v;
         };
@@ -399,7 +406,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
           }
           // what the guard found, four rows of a column at a time
 #pragma unroll 1
-          for (int k = 0; __any_sync(0xffffffffu, direct != 0u) && k < NL; ++k) {
+          for (int k = 0; !lost && __any_sync(0xffffffffu, direct != 0u) && k < NL; ++k) {
             const int n = nt * (BC ? C::BN / 2 : C::BN) + (BC ? (j0 + g0) / 2 : j0 + g0) + k;
             const bool mine = m < g.M && n < g.N && !(AC && odd) && ((direct >> (BC ? g0 + 2 * k : g0 + k)) & (BC ? 3u : 1u));
             unsigned rows = __ballot_sync(0xffffffffu, mine);
@@ -458,7 +465,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
 #pragma unroll 4
             for (int k = 0; k < NL; ++k) {
               const long long cT = sh->col_offT[j0 + g0 + k];
-              if (cT >= 0 && m <= nt * C::BN + j0 + g0 + k) Cr[cT + coffT] = stage[lane * RS + k].x;
+              if (cT >= 0 && m <= nt * C::BN + j0 + g0 + k) Cr[cT + coffT] = lost ? nan : stage[lane * RS + k].x;
             }
         }
         // every lane owns a (row, column) pair per pass
@@ -470,7 +477,7 @@ __global__ void __launch_bounds__(C::THREADS, 1)
           if (r >= nrows || cn < 0) continue;
           if (SYM && g.sym && m0w + r > nt * C::BN + j0 + g0 + lc) continue;  // stored by the mirror image's tile
           const long long off = cm + cn;
-          const double2 v = stage[r * RS + lc];
+          const double2 v = lost ? make_double2(nan, nan) : stage[r * RS + lc];
           if (g.cc) {
             if (red) {
               atomicAdd(&Cc[off].x, v.x);

@@ -13,6 +13,7 @@ constexpr int TC_BN = 64;                    // packed B rows are padded to this
 constexpr int TC_BK = 64;                    // K per TMA box (128 B of BF16)
 constexpr int TC_CHUNK_KB = 8;               // 512-wide K chunks (exact FP32 level sums)
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;
+constexpr int kTcWaitLimit = 1 << 22;        // polls after which a tensor-core kernel gives up a wait
 constexpr int TC_MAX_SLICES = 6;
 constexpr int TC_DEEP_SLICES = 8;            // the FP64 form's tensor-core contractions
 // planes of a packed operand: its slices, and with 8 the range guard's (gemm_deep.cu)

@@ -14,7 +14,7 @@
 //
 // The launch is cooperative, so all blocks are resident; every wait on the
 // barrier has an iteration limit, after which the kernel records an error
-// code, stops and returns.
+// code, stops, leaves NaN in all that it writes and returns.
 #include <algorithm>
 #include <cstddef>
 #include <cstdlib>
@@ -34,6 +34,7 @@ namespace {
 constexpr int kPhaseSlots = 128;   // pointers passed by value
 constexpr int kPhaseOps = 160;
 constexpr int kBarrierLimit = 1 << 21;
+constexpr unsigned kLost = 1u << 16;  // in the count of blocks that are out: one gave up a wait
 // Phases with more work keep a launch per op: there the blocks of several ops
 // fill the chip without waiting for one another.  Measured (one launch per
 // phase against one per op): T2 residual 86 and 243 us at o=3, v=8, 105 and
@@ -99,8 +100,15 @@ struct alignas(16) PhaseOp {
   };
 };
 
+struct PhaseOut {  // a buffer that the phase writes
+  int slot, pad;
+  long long doubles;
+};
+
 struct PhaseArgs {
   const PhaseOp* ops;
+  const PhaseOut* outs;
+  int nouts, wait;
   const int* tab;      // [nlevels + 1] first op of each level, [nops] first tile within its level, [nops] end tile
   int nops, nlevels;
   unsigned* bar;
@@ -115,10 +123,10 @@ __device__ __forceinline__ void grid_arrive(unsigned* bar) {
   __syncthreads();
   if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
 }
-__device__ __forceinline__ bool grid_wait(unsigned* bar, unsigned target, int* err, int* shared_ok) {
+__device__ __forceinline__ bool grid_wait(unsigned* bar, unsigned target, int limit, int* err, int* shared_ok) {
   if (threadIdx.x == 0) {
     int good = 0;
-    for (int i = 0; i < kBarrierLimit; ++i) {
+    for (int i = 0; i < limit; ++i) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
       if (v >= target) {
@@ -126,7 +134,10 @@ __device__ __forceinline__ bool grid_wait(unsigned* bar, unsigned target, int* e
         break;
       }
     }
-    if (!good) atomicCAS(err, 0, 9);
+    if (!good) {
+      atomicCAS(err, 0, 9);
+      atomicAdd(bar + 1, kLost);  // this launch's results are lost
+    }
     *shared_ok = good;
   }
   __syncthreads();
@@ -408,16 +419,28 @@ __global__ void __launch_bounds__(kFxThreads, 2) phase_kernel(const __grid_const
         if (rec[w].kind == OP_GEMM && rec[w].form >= 3) dot_ahead(rec[w].dot, (unsigned)((int)blockIdx.x - beg[o]), ahead);
         have = true;
       }
-      good = grid_wait(p.bar, (unsigned)(l + 1) * gridDim.x, p.err, &ok);
+      good = grid_wait(p.bar, (unsigned)(l + 1) * gridDim.x, p.wait, p.err, &ok);
     }
   }
-  // the last block out resets the barrier for the next launch
+  // The last block out resets the barrier for the next launch.  Where a wait ran
+  // out it first writes NaN over all that the phase writes: by then no other block
+  // has anything left to store.
   if (tid == 0) {
     __threadfence();
-    if (atomicAdd(p.bar + 1, 1u) == gridDim.x - 1) {
+    const unsigned out = atomicAdd(p.bar + 1, 1u);  // blocks out before; what is lost, above
+    ok = 0;
+    if ((out & (kLost - 1u)) == gridDim.x - 1) {
       p.bar[0] = 0u;
       p.bar[1] = 0u;
       __threadfence();
+      ok = out >= kLost ? 1 : 0;
+    }
+  }
+  if (__syncthreads_or(tid == 0 && ok)) {
+    const double nan = __longlong_as_double(0x7FF8000000000000ll);
+    for (int i = 0; i < p.nouts; ++i) {
+      double* x = static_cast<double*>(p.base[p.outs[i].slot]);
+      for (long long k = tid; k < p.outs[i].doubles; k += kFxThreads) x[k] = nan;
     }
   }
 }
@@ -445,6 +468,29 @@ bool covers(const Program& p, const Op& op) {
     }
   }
   return n == numel && last == numel - 1;
+}
+
+// doubles of the op's output buffer up to the last one that it writes
+long long out_doubles(const Op& op) {
+  long long last = 0;
+  if (op.kind == OP_GEMM) {
+    last = op.oc + (op.g.nb > 1 ? (op.g.nb - 1) * op.g.bsC : 0);
+    for (const ModeGroup* g : {&op.g.gm, &op.g.gn})
+      for (int i = 0; i < g->n; ++i) last += (g->dim[i] - 1) * g->s1[i];
+    return (last + 1) * (op.dtc == C64 ? 2 : 1);
+  }
+  if (op.kind == OP_ADD) {
+    last = op.add_oc;
+    for (int i = 0; i < op.a.nd; ++i) last += (op.a.d[i] - 1) * op.a.sC[i];
+    return (last + 1) * (op.a.cc ? 2 : 1);
+  }
+  if (op.kind == OP_REDUCE) {
+    last = op.rd_oout;
+    for (int i = 0; i < op.rd.no; ++i) last += (op.rd.dout[i] - 1) * op.rd.so_out[i];
+    return 2 * (last + 1);
+  }
+  const int nb = std::max(op.tr_nb, 1);
+  return 2 * ((nb > 1 ? (nb - 1) * op.tr_bsres : 0) + op.tr_n_mu);
 }
 
 }  // namespace
@@ -750,27 +796,41 @@ void PhaseKernel::build(const Program& p, Program::Phase ph, std::vector<void*>&
   nlevels_ = (int)first.size();
   nops_ = n;
   nslots_ = n0;
+  std::vector<PhaseOut> outs;
+  for (const Op& op : q.ops) {
+    if (op.write < 0 || op.write >= n0) continue;
+    const long long doubles = out_doubles(op);
+    bool known = false;
+    for (PhaseOut& x : outs)
+      if (x.slot == op.write) {
+        known = true;
+        x.doubles = std::max(x.doubles, doubles);
+      }
+    if (!known) outs.push_back(PhaseOut{op.write, 0, doubles});
+  }
+  nouts_ = (int)outs.size();
   first.push_back(n);
   std::vector<int> tab(first);
   tab.insert(tab.end(), beg.begin(), beg.end());
   tab.insert(tab.end(), end.begin(), end.end());
   const size_t rb = recs.size() * sizeof(PhaseOp), tb = (tab.size() * sizeof(int) + 255) / 256 * 256,
-               ob = (tables.size() * sizeof(int2) + 255) / 256 * 256;
+               ob = (tables.size() * sizeof(int2) + 255) / 256 * 256, wb = (outs.size() * sizeof(PhaseOut) + 255) / 256 * 256;
   char* d = nullptr;
-  if (cudaMalloc(&d, rb + tb + 256 + ob) != cudaSuccess) {
+  if (cudaMalloc(&d, rb + tb + 256 + ob + wb) != cudaSuccess) {
     cudaGetLastError();
     return;  // a launch per op needs no records
   }
   owned.push_back(d);
-  bytes += (long long)(rb + tb + 256 + ob);
+  bytes += (long long)(rb + tb + 256 + ob + wb);
   for (const auto& at : table_at) {
     recs[at.first].pslot[at.second] = -2;
     recs[at.first].pbyte[at.second] += (long long)(uintptr_t)(d + rb + tb + 256);
   }
-  std::vector<char> host(rb + tb + 256 + ob, 0);  // one copy, the barrier's words zero
+  std::vector<char> host(rb + tb + 256 + ob + wb, 0);  // one copy, the barrier's words zero
   memcpy(host.data(), recs.data(), rb);
   memcpy(host.data() + rb, tab.data(), tab.size() * sizeof(int));
   if (!tables.empty()) memcpy(host.data() + rb + tb + 256, tables.data(), tables.size() * sizeof(int2));
+  if (!outs.empty()) memcpy(host.data() + rb + tb + 256 + ob, outs.data(), outs.size() * sizeof(PhaseOut));
   if (cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaDeviceSynchronize() != cudaSuccess)
     throw std::runtime_error("uploading the phase records failed");
@@ -778,6 +838,7 @@ void PhaseKernel::build(const Program& p, Program::Phase ph, std::vector<void*>&
   tab_ = reinterpret_cast<int*>(d + rb);
   bar_ = reinterpret_cast<unsigned*>(d + rb + tb);
   err_ = reinterpret_cast<int*>(d + rb + tb + 128);
+  outs_ = d + rb + tb + 256 + ob;
   ok = true;
 }
 
@@ -801,6 +862,9 @@ cudaError_t PhaseKernel::launch(const std::vector<void*>& bases, int blocks, cud
   PhaseArgs a;
   a.ops = static_cast<const PhaseOp*>(ops_);
   a.tab = tab_;
+  a.outs = static_cast<const PhaseOut*>(outs_);
+  a.nouts = nouts_;
+  a.wait = wait == 0 ? kBarrierLimit : wait;
   a.nops = nops_;
   a.nlevels = nlevels_;
   a.bar = bar_;

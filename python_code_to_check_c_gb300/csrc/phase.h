@@ -18,13 +18,15 @@ class PhaseKernel {
   // `blocks`: at most this many thread blocks (several phases may run at once)
   cudaError_t launch(const std::vector<void*>& bases, int blocks, cudaStream_t st) const;
   int* error_flag() const { return err_; }
+  int wait = 0;  // polls of the grid barrier (0: the kernel's limit; negative: none, for tests)
 
  private:
   void* ops_ = nullptr;
   int* tab_ = nullptr;
   unsigned* bar_ = nullptr;
   int* err_ = nullptr;
-  int nops_ = 0, nlevels_ = 0, nslots_ = 0, widest_ = 0;
+  const void* outs_ = nullptr;
+  int nops_ = 0, nlevels_ = 0, nslots_ = 0, widest_ = 0, nouts_ = 0;
   size_t smem_ = 0;
 };
 

@@ -136,7 +136,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-constexpr int kWaitLimit = 1 << 22;
+constexpr int kWaitLimit = kTcWaitLimit;
 
 // The MMA warp's side of a ring of slice pairs (A_j, B_j): the products of one
 // K block with s + t <= S + 1 into the accumulators of their levels, BN columns
@@ -148,6 +148,7 @@ template <int STAGES, int A_BYTES, int B_BYTES>
 struct PairRing {
   uint64_t hi64;
   uint32_t a0, b0, full0, empty0;
+  int wait = kWaitLimit;     // polls of a wait
   uint32_t st0 = 0, ph = 0;  // ring slot and phase of the block's first pair
   __device__ __forceinline__ PairRing(const uint8_t* stA, const uint8_t* stB, const uint64_t* full, const uint64_t* empty)
       : hi64(sdesc(0)),
@@ -169,7 +170,7 @@ struct PairRing {
     bool ok = true;
 #pragma unroll
     for (int j = 1; j <= S; ++j) {
-      if (ok) ok = mbar_wait_warp(full0 + 8 * slot[j - 1], st0 + j - 1 < STAGES ? ph : ph ^ 1u, kWaitLimit);
+      if (ok) ok = mbar_wait_warp(full0 + 8 * slot[j - 1], st0 + j - 1 < STAGES ? ph : ph ^ 1u, wait);
       asm volatile("tcgen05.fence::after_thread_sync;");
       if (ok) {
         auto product = [&](int s, int t) {
@@ -202,7 +203,7 @@ struct PairRing {
   // The range guard's plane of 128 K (64 where `half`) into columns [0, BN).
   template <int BN>
   __device__ __forceinline__ bool guard(uint32_t tmem, uint32_t id, bool first, bool half, uint32_t on) {
-    const bool ok = mbar_wait_warp(full0 + 8 * st0, ph, kWaitLimit);
+    const bool ok = mbar_wait_warp(full0 + 8 * st0, ph, wait);
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (ok) {
       const uint32_t la = a0 + st0 * (A_BYTES >> 4), lb = b0 + st0 * (B_BYTES >> 4);
