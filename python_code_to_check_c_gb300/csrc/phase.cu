@@ -423,20 +423,20 @@ __global__ void __launch_bounds__(kFxThreads, 2) phase_kernel(const __grid_const
     }
   }
   // The last block out resets the barrier for the next launch.  Where a wait ran
-  // out it first writes NaN over all that the phase writes: by then no other block
-  // has anything left to store.
+  // out it then writes NaN over all that the phase writes: no other block has
+  // anything left to store.
+  int lost = 0;
   if (tid == 0) {
     __threadfence();
     const unsigned out = atomicAdd(p.bar + 1, 1u);  // blocks out before; what is lost, above
-    ok = 0;
     if ((out & (kLost - 1u)) == gridDim.x - 1) {
       p.bar[0] = 0u;
       p.bar[1] = 0u;
       __threadfence();
-      ok = out >= kLost ? 1 : 0;
+      lost = out >= kLost ? 1 : 0;
     }
   }
-  if (__syncthreads_or(tid == 0 && ok)) {
+  if (__syncthreads_or(lost)) {
     const double nan = __longlong_as_double(0x7FF8000000000000ll);
     for (int i = 0; i < p.nouts; ++i) {
       double* x = static_cast<double*>(p.base[p.outs[i].slot]);
