@@ -238,16 +238,11 @@ void bind_fixed(tdcc_system s, std::vector<void*>& b) {
   b[S_MU] = const_cast<double*>(s->mu);
 }
 
-// bytes the packed operands of one FP64 program may take: a sixth of what is
-// free (a step holds four programs and the density's, reverse mode as many again)
-long long deep_budget() {
-  size_t fr = 0, tot = 0;
-  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return (long long)(fr / 6);
-}
+// Bytes the packed operands of one FP64 program may take: a fixed number, so that
+// the arithmetic follows from the problem alone.  (The ladder at o=24, v=160 packs
+// 12 GB.)  A program that then finds no memory is built again without them
+// (with_or_without_deep): where a call ran before, it runs.
+constexpr long long kDeepBytes = 32LL << 30;
 
 // Scratch of a call without a system, from a pool of the library's own per
 // device.  The device's default pool gives everything back at each
@@ -292,9 +287,19 @@ struct Scratch {
   }
 };
 
-ProgInst& get_rhs(tdcc_system s, int method, int block) {
-  auto& slot = s->rhs[method][block];
-  if (slot) return *slot;
+// `build` with the FP64 form's tensor-core contractions, without them where the
+// device's memory does not hold their packed operands
+template <class F>
+std::unique_ptr<ProgInst> with_or_without_deep(tdcc_system s, F&& build) {
+  try {
+    return build(kDeepBytes);
+  } catch (const OutOfMemory&) {
+    if (s->prec_mode != TDCC_PREC_FP64) throw;
+  }
+  return build(0);
+}
+
+std::unique_ptr<ProgInst> build_rhs(tdcc_system s, int method, int block, long long deep_bytes) {
   auto pi = std::make_unique<ProgInst>();
   static const char* names[2][4] = {{"ccsd_t1", "ccsd_t2", "ccsd_l1", "ccsd_l2"},
                                     {"cc2_t1", "cc2_t2", "cc2_l1", "cc2_l2"}};
@@ -316,45 +321,51 @@ ProgInst& get_rhs(tdcc_system s, int method, int block) {
     build_l2_cc2(p, p.ones("ones_v", s->dims.v));
   p.batch(s->nb);
   p.select_backend(s->prec_mode, s->tc_min_macs, s->slices, s->tc_min_k, s->tc_min_mn, s->simt_max_k,
-                          s->simt_min_macs, deep_budget());
+                   s->simt_min_macs, deep_bytes);
   // the block's own amplitude and the dressed Fock vary across RK4 stages
   p.analyse({S_T1 + block, S_F});
   if (s->share_mem && workspace_estimate(p) > (s->share_min < 0 ? kShareMinBytes : s->share_min)) p.plan_memory();
   pi->bases.assign(p.slots.size(), nullptr);
   pi->each_call = s->prec_mode == TDCC_PREC_FP64;
   pi->bytes = p.allocate(pi->bases, pi->owned);
-  s->ws_bytes += pi->bytes;
   bind_fixed(s, pi->bases);
   pi->dag.init(p.ops.size(), 4);
-  const long long ws0 = pi->bytes;
   pi->build_phases({Program::PROLOGUE, Program::STAGE, Program::DYNAMIC});
-  s->ws_bytes += pi->bytes - ws0;
   pi->set_wait_limit(s->wait_limit);
-  slot = std::move(pi);
+  return pi;
+}
+
+ProgInst& get_rhs(tdcc_system s, int method, int block) {
+  auto& slot = s->rhs[method][block];
+  if (slot) return *slot;
+  slot = with_or_without_deep(s, [&](long long deep) { return build_rhs(s, method, block, deep); });
+  s->ws_bytes += slot->bytes;
   return *slot;
 }
 
-ProgInst& get_density(tdcc_system s) {
-  if (s->dens) return *s->dens;
+std::unique_ptr<ProgInst> build_density_inst(tdcc_system s, long long deep_bytes) {
   auto pi = std::make_unique<ProgInst>();
   pi->prog = std::make_unique<Program>(s->dims, "density");
   build_density(*pi->prog, s->n_mu);
   pi->prog->batch(s->nb);
   pi->prog->select_backend(s->prec_mode, s->tc_min_macs, s->slices, s->tc_min_k, s->tc_min_mn, s->simt_max_k,
-                          s->simt_min_macs, deep_budget());
+                           s->simt_min_macs, deep_bytes);
   pi->prog->analyse({});
   if (s->share_mem && workspace_estimate(*pi->prog) > (s->share_min < 0 ? kShareMinBytes : s->share_min))
     pi->prog->plan_memory();
   pi->bases.assign(pi->prog->slots.size(), nullptr);
   pi->bytes = pi->prog->allocate(pi->bases, pi->owned);
-  s->ws_bytes += pi->bytes;
   bind_fixed(s, pi->bases);
   pi->dag.init(pi->prog->ops.size(), 4);
-  const long long ws0 = pi->bytes;
   pi->build_phases({Program::ALL});
-  s->ws_bytes += pi->bytes - ws0;
   pi->set_wait_limit(s->wait_limit);
-  s->dens = std::move(pi);
+  return pi;
+}
+
+ProgInst& get_density(tdcc_system s) {
+  if (s->dens) return *s->dens;
+  s->dens = with_or_without_deep(s, [&](long long deep) { return build_density_inst(s, deep); });
+  s->ws_bytes += s->dens->bytes;
   return *s->dens;
 }
 
@@ -370,6 +381,27 @@ void reset_programs(tdcc_system s);
 
 // Reverse-mode program of (method, block); block 4 = density.  Its slots
 // [0, nfwd) are bound to the forward instance's buffers before every run.
+std::unique_ptr<ProgInst> build_adj(tdcc_system s, int method, int block, long long deep_bytes) {
+  Program f(s->dims, "fwd");
+  build_program(f, method, block, s->n_mu, s->nb);
+  auto pi = std::make_unique<ProgInst>();
+  pi->prog = std::make_unique<Program>(s->dims, "adj");
+  build_adjoint(f, *pi->prog, s->adj_of[method][block]);
+  pi->prog->select_backend(s->prec_mode, s->tc_min_macs, s->slices, s->tc_min_k, s->tc_min_mn, s->simt_max_k,
+                           s->simt_min_macs, deep_bytes);
+  pi->nfwd = f.slots.size();
+  pi->bases.assign(pi->prog->slots.size(), nullptr);
+  pi->bytes = pi->prog->allocate(pi->bases, pi->owned, pi->nfwd, true);
+  pi->setup_done = true;  // no integral-only ops in a reverse-mode program
+  pi->dag.init(pi->prog->ops.size(), 4);
+  if (block == 4)
+    pi->build_phases({Program::ALL});
+  else
+    pi->build_phases({Program::PROLOGUE, Program::STAGE});
+  pi->set_wait_limit(s->wait_limit);
+  return pi;
+}
+
 ProgInst& get_adj(tdcc_system s, int method, int block) {
   auto& slot = s->adjp[method][block];
   if (slot) return *slot;
@@ -381,25 +413,8 @@ ProgInst& get_adj(tdcc_system s, int method, int block) {
     get_density(s);
   else
     get_rhs(s, method, block);
-  Program f(s->dims, "fwd");
-  build_program(f, method, block, s->n_mu, s->nb);
-  auto pi = std::make_unique<ProgInst>();
-  pi->prog = std::make_unique<Program>(s->dims, "adj");
-  build_adjoint(f, *pi->prog, s->adj_of[method][block]);
-  pi->prog->select_backend(s->prec_mode, s->tc_min_macs, s->slices, s->tc_min_k, s->tc_min_mn, s->simt_max_k,
-                          s->simt_min_macs, deep_budget());
-  pi->nfwd = f.slots.size();
-  pi->bases.assign(pi->prog->slots.size(), nullptr);
-  pi->bytes = pi->prog->allocate(pi->bases, pi->owned, pi->nfwd, true);
+  auto pi = with_or_without_deep(s, [&](long long deep) { return build_adj(s, method, block, deep); });
   s->ws_bytes += pi->bytes;
-  pi->setup_done = true;  // no integral-only ops in a reverse-mode program
-  pi->dag.init(pi->prog->ops.size(), 4);
-  const long long ws0 = pi->bytes;
-  if (block == 4)
-    pi->build_phases({Program::ALL});
-  else
-    pi->build_phases({Program::PROLOGUE, Program::STAGE});
-  s->ws_bytes += pi->bytes - ws0;
   if (block < 4) {
     const ActPlan ap = plan_activations(*pi->prog, pi->nfwd, *get_rhs(s, method, block).prog);
     pi->act_slot = ap.slot;
@@ -408,7 +423,6 @@ ProgInst& get_adj(tdcc_system s, int method, int block) {
     pi->act_pro8 = ap.pro8;
     pi->act_stage8 = ap.stage8;
   }
-  pi->set_wait_limit(s->wait_limit);
   slot = std::move(pi);
   return *slot;
 }
@@ -1827,7 +1841,7 @@ int tdcc_tei_from_df(const double* B, int n, int nq, double* tei, void* stream) 
     const long long rows = (n2 + 127) / 128 * 128, kpad = (nq + 63) / 64 * 64LL;
     const long long exp_off = (long long)tc_planes(TC_DEEP_SLICES) * rows * kpad * 2, need = exp_off + rows * 4 + 256;
     Scratch w;
-    if (nq >= 32 && t_deep < 0.85 * t_fx && cap == cudaStreamCaptureStatusNone && need <= deep_budget()) w.get((size_t)need, st);
+    if (nq >= 32 && t_deep < 0.85 * t_fx && cap == cudaStreamCaptureStatusNone) w.get((size_t)need, st);
     if (w.p) {
       char* base = static_cast<char*>(w.p);
       int* err = reinterpret_cast<int*>(base + exp_off + rows * 4);

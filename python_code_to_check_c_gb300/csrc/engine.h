@@ -7,6 +7,7 @@
 
 #include <cstdint>
 #include <map>
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -242,6 +243,11 @@ struct SlotInfo {
 
 struct Dims {  // system sizes
   int o, v, n;
+};
+
+// Device memory that a program could not have (Program::allocate).
+struct OutOfMemory : std::runtime_error {
+  using std::runtime_error::runtime_error;
 };
 
 // Streams and per-op events for executing a program as a dependency DAG.

@@ -258,7 +258,8 @@ void Program::ein(const char* spec, double ar, double ai, const View& A, const V
 // Form and K splits (splits only where the output is zeroed or accumulated
 // into: they add with atomics), from the kernels' cost model.  Dot products or
 // fixed-point tiles is decided once, from the extents the op is first planned
-// with: a batched program then rounds as its single-trajectory one does.
+// with; K splits and the tensor-core form (deep_splits) follow the batch, so a
+// batched program's last bits may differ from its single-trajectory one's.
 void Program::plan_gemm(Op& op, bool allow_split, int tile) {
   GemmArgs& g = op.g;
   const long long K = g.K, nb = std::max(g.nb, 1);
@@ -661,7 +662,7 @@ long long Program::allocate(std::vector<void*>& bases, std::vector<void*>& owned
     void* p = nullptr;
     if (cudaMalloc(&p, pool_bytes[q]) != cudaSuccess) {
       cudaGetLastError();
-      throw std::runtime_error("cudaMalloc failed for a shared workspace buffer in " + name);
+      throw OutOfMemory("cudaMalloc failed for a shared workspace buffer in " + name);
     }
     owned.push_back(p);
     pool_ptr[q] = p;
@@ -680,7 +681,7 @@ long long Program::allocate(std::vector<void*>& bases, std::vector<void*>& owned
     void* p = nullptr;
     if (cudaMalloc(&p, b) != cudaSuccess) {
       cudaGetLastError();
-      throw std::runtime_error("cudaMalloc failed for workspace " + slots[i].name + " in " + name);
+      throw OutOfMemory("cudaMalloc failed for workspace " + slots[i].name + " in " + name);
     }
     owned.push_back(p);
     bases[i] = p;
