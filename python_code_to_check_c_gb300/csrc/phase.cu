@@ -426,6 +426,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) phase_kernel(const __grid_const
   // out it then writes NaN over all that the phase writes: no other block has
   // anything left to store.
   int lost = 0;
+  __syncthreads();  // this block has stored all it will
   if (tid == 0) {
     __threadfence();
     const unsigned out = atomicAdd(p.bar + 1, 1u);  // blocks out before; what is lost, above
