@@ -53,7 +53,7 @@ struct ProgInst {
   std::vector<void*> owned;  // this program's workspace allocations
   long long bytes = 0;
   bool setup_done = false;   // integral-only ops (e.g. packed integral blocks) ran
-  bool each_call = false;    // FP64 form: they run again in every call, so that it reads the integrals as they are
+  bool each_call = false;    // FP64 form, reverse mode: they run again in every call, so that it reads the integrals as they are
   DagExec dag;               // streams/events for concurrent execution of the ops
   PhaseKernel phase[5];      // phases that run as one launch (small FP64 programs)
   void build_phases(std::initializer_list<Program::Phase> phs) {
@@ -392,7 +392,14 @@ std::unique_ptr<ProgInst> build_adj(tdcc_system s, int method, int block, long l
   pi->nfwd = f.slots.size();
   pi->bases.assign(pi->prog->slots.size(), nullptr);
   pi->bytes = pi->prog->allocate(pi->bases, pi->owned, pi->nfwd, true);
-  pi->setup_done = true;  // no integral-only ops in a reverse-mode program
+  bind_fixed(s, pi->bases);
+  // packings of the integrals: once per call, in either form, not at every stage
+  for (Op& op : pi->prog->ops)
+    if (op.kind == OP_PACK && op.pk_src == S_TEI) {
+      op.is_const = true;
+      op.varying = false;
+    }
+  pi->each_call = true;
   pi->dag.init(pi->prog->ops.size(), 4);
   if (block == 4)
     pi->build_phases({Program::ALL});
@@ -1489,7 +1496,7 @@ int tdcc_adjoint(tdcc_system s, int method, const void* t1, const void* t2, cons
     CK(cudaStreamWaitEvent(m, s->ev_user, 0));
     begin_call(s);
     for (int b = 0; b < 4; ++b) {
-      get_adj(s, method, b);
+      CK(get_adj(s, method, b).setup(m));
       CK(get_rhs(s, method, b).setup(m));
     }
     get_adj(s, method, 4);
