@@ -1406,8 +1406,10 @@ static PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 }
 
 // [S][rows_pad][K_pad] BF16, box = (64 K, box_rows rows, 1 slice).
-// Encoded maps are cached by (address, layout): a packed buffer keeps its
-// address for the life of its program.
+// Encoded maps are cached by (address, layout), which determine them: a packed
+// buffer keeps its address for the life of its program.  The cache is emptied when
+// it has grown to kMapsMax (scratch addresses come and go).
+constexpr size_t kMapsMax = 4096;
 CUtensorMap slice_map(const void* base, int S, int rows_pad, int K_pad, int box_rows) {
   static std::mutex mu;
   static std::map<std::tuple<const void*, int, int, int, int>, CUtensorMap> cache;
@@ -1427,6 +1429,7 @@ CUtensorMap slice_map(const void* base, int S, int rows_pad, int K_pad, int box_
                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
   std::lock_guard<std::mutex> lk(mu);
+  if (cache.size() >= kMapsMax) cache.clear();
   cache[key] = m;
   return m;
 }
