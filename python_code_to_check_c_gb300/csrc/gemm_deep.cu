@@ -548,7 +548,6 @@ cudaError_t launch_deep_form(const TcArgs& a0, const void* packA, const void* pa
 
 cudaError_t launch_deep(const TcArgs& a, const void* packA, const void* packB, cudaStream_t st) {
   switch (a.S) {
-    case 1: return launch_deep_form<TcDeep<1, 128, 6>>(a, packA, packB, st);
     case 2: return launch_deep_form<TcDeep<2, 128, 6>>(a, packA, packB, st);
     case 3: return launch_deep_form<TcDeep<3, 128, 6>>(a, packA, packB, st);
     case 4: return launch_deep_form<TcDeep<4, 128, 6>>(a, packA, packB, st);

@@ -440,7 +440,6 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 #pragma unroll 1
       for (int kb = kbs; kb < kbe && ok; ++kb)
         switch (S) {
-          case 1: ok = ring.template issue<1, C::BN>(tmem, id, kb == kbs, on); break;
           case 2: ok = ring.template issue<2, C::BN>(tmem, id, kb == kbs, on); break;
           case 3: ok = ring.template issue<3, C::BN>(tmem, id, kb == kbs, on); break;
           case 4: ok = ring.template issue<4, C::BN>(tmem, id, kb == kbs, on); break;
@@ -887,7 +886,6 @@ __global__ void __launch_bounds__(TcPersist::THREADS, 1)
   } else if (warp == 1) {
     // ---------------- MMA issuer (the whole warp, one lane executing) ----------------
     switch (S) {
-      case 1: persist_issue<1>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
       case 2: persist_issue<2>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
       case 3: persist_issue<3>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
       default: persist_issue<4>(g, sh, ringA, ringB, tmem, ntiles_total, mtiles, ntiles, lane); break;
@@ -1554,7 +1552,7 @@ static cudaError_t launch_variant(const TcArgs& a0, const void* packA, const voi
   });
   if (attr_err[dev] != cudaSuccess) return attr_err[dev];
   TcArgs a = a0;
-  if (a.S > C::STAGES) return cudaErrorInvalidValue;  // the ring holds one K block's slices
+  if (a.S < 2 || a.S > C::STAGES) return cudaErrorInvalidValue;  // the ring holds one K block's slices
   int cols = 32;
   while (cols < (a.S + 2) * C::BN) cols *= 2;  // level accumulators + int64 partial sums
   if (cols > 512 / C::MINB) return cudaErrorInvalidValue;
@@ -1602,7 +1600,7 @@ static cudaError_t launch_persist(const TcArgs& a0, const void* packA, const voi
   if (attr_err[dev] != cudaSuccess) return attr_err[dev];
   TcArgs a = a0;
   // two TMEM buffers of S levels, short K per tile
-  if (a.S < 1 || a.S > TC_PERSIST_MAX_S || a.kb_per_split > C::MAX_KB) return cudaErrorInvalidValue;
+  if (a.S < 2 || a.S > TC_PERSIST_MAX_S || a.kb_per_split > C::MAX_KB) return cudaErrorInvalidValue;
   int cols = 32;
   while (cols < 2 * a.S * C::BN) cols *= 2;
   a.tmem_cols = cols;

@@ -494,7 +494,14 @@ long long out_doubles(const Op& op) {
   return 2 * ((nb > 1 ? (nb - 1) * op.tr_bsres : 0) + op.tr_n_mu);
 }
 
-}  // namespace
+// The ops of a phase with their dependency levels, sums into one output taken
+// apart into temporaries (slots from p.slots.size() on, complex elements in
+// `temps`; 0: unused) and one addition.
+struct PhaseOps {
+  std::vector<Op> ops;
+  std::vector<int> level;
+  std::vector<long long> temps;
+};
 
 // Several ops that add to one output wait for one another in program order
 // (a fixed order of the roundings).  Here they write to temporaries instead,
@@ -587,6 +594,8 @@ PhaseOps phase_ops(const Program& p, Program::Phase ph) {
   }
   return r;
 }
+
+}  // namespace
 
 void PhaseKernel::build(const Program& p, Program::Phase ph, std::vector<void*>& owned, long long& bytes) {
   ok = false;

@@ -30,14 +30,4 @@ class PhaseKernel {
   size_t smem_ = 0;
 };
 
-// The ops of a phase with their dependency levels, sums into one output taken
-// apart into temporaries (slots from p.slots.size() on, complex elements in
-// `temps`; 0: unused) and one addition.
-struct PhaseOps {
-  std::vector<Op> ops;
-  std::vector<int> level;
-  std::vector<long long> temps;
-};
-PhaseOps phase_ops(const Program& p, Program::Phase ph);
-
 }  // namespace tdcc

@@ -958,8 +958,8 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
                       (double)rup(op.g.N * (op.dtb == C64 ? 2LL : 1LL), 64) * (op.g.bsB ? nb : 1.0));
       }
     if (need == 0.0 || need > (double)deep_bytes) return;
-  } else if (S < 1 || S > 6) {
-    throw std::runtime_error("slices must be 1..6");
+  } else if (S < 2 || S > 6) {
+    throw std::runtime_error("slices must be 2..6");
   }
   constexpr int BM = 128, BN = 64, BK = 64;  // tensor-core tile (gemm_tc.h)
   std::vector<Op> out;
