@@ -529,7 +529,8 @@ cudaError_t launch_deep_form(const TcArgs& a0, const void* packA, const void* pa
   // the tiles of the smaller operand side vary fastest: that side stays in L2
   const unsigned mtiles = (unsigned)(a.rowsA_pad / TC_BM);
   const unsigned ntiles = (unsigned)(((long long)a.N * (a.bc ? 2 : 1) + C::BN - 1) / C::BN);
-  a.m_fast = (a.rowsA_pad < a.rowsB_pad && ntiles <= 65535u) ? 1 : 0;
+  // (a side of more than 65535 tiles, v^3 rows at v > 203, has to)
+  a.m_fast = mtiles > 65535u || (a.rowsA_pad < a.rowsB_pad && ntiles <= 65535u) ? 1 : 0;
   if ((a.m_fast ? ntiles : mtiles) > 65535u || (long long)a.nb * a.nsplit > 65535LL) return cudaErrorInvalidConfiguration;
   dim3 grid(a.m_fast ? mtiles : ntiles, a.m_fast ? ntiles : mtiles, (unsigned)((long long)a.nb * a.nsplit));
   if (a.ac && a.bc)
