@@ -379,8 +379,10 @@ void build_adjoint(const Program& f, Program& a, std::vector<int>& adj_of);
 constexpr int kNumTiles = 6;
 extern const int kTiles[kNumTiles][2];
 bool tile_fits(int tile, bool real_operands);
-void choose_fx(long long M, long long N, long long K, long long nb, bool ac, bool bc, bool allow_split, int tile,
-               int* best_tile, int* best_splits);
+// (returns the model's clocks; dot_cost: those of dot products with 2^lw lanes an output)
+double choose_fx(long long M, long long N, long long K, long long nb, bool ac, bool bc, bool allow_split, int tile,
+                 int* best_tile, int* best_splits);
+double dot_cost(long long outputs, long long K, int lw, bool ac, bool bc);
 int dot_lanes(long long outputs, long long K);
 
 // how a block walks a contraction (after the operands are put in order)

@@ -26,6 +26,13 @@ int dot_lanes(long long outputs, long long K) {
   return lw;
 }
 
+// clocks of the dot products (dot_tile) with 2^lw lanes per output
+double dot_cost(long long outputs, long long K, int lw, bool ac, bool bc) {
+  const double warps = std::ceil((double)outputs * (double)(1 << lw) / 32.0);
+  const double per = std::ceil((double)K / (double)(1 << lw)) * ((ac && bc) ? 4.0 : (ac || bc) ? 2.0 : 1.0) + 2.0 * lw;
+  return 2200.0 + std::ceil(warps / 608.0) * per * 66.0;
+}
+
 // Form and K splits of a contraction, by a model in SM clocks.  Fixed-point
 // tiles: a fixed part (index decoding, the loads' latency, the stores), the
 // cutting of its operands and its multiply-adds; blocks beyond one per SM
@@ -36,8 +43,8 @@ int dot_lanes(long long outputs, long long K) {
 // (40, 0.3) and (31, 0.45): a gradient of 8 steps at o=6, v=12 17.7 ms, 22.7 and 26.4;
 // the propagation at o=10, v=14 10.06 ms for 8 steps, 9.81 and 9.96; 60 residuals of
 // o=5..14, v=14..50 32.7 ms in all, 32.9 and 32.8.
-void choose_fx(long long M, long long N, long long K, long long nb, bool ac, bool bc, bool allow_split, int tile,
-               int* best_tile, int* best_splits) {
+double choose_fx(long long M, long long N, long long K, long long nb, bool ac, bool bc, bool allow_split, int tile,
+                 int* best_tile, int* best_splits) {
   const double im = (ac && bc) ? 12.0 : (ac || bc) ? 6.0 : 3.0;
   double best = 1e300;
   *best_tile = 0;
@@ -48,10 +55,7 @@ void choose_fx(long long M, long long N, long long K, long long nb, bool ac, boo
     if (t == 5 && tile != -3) continue;
     if (!tile_fits(t, !ac && !bc)) continue;
     if (t == 5) {
-      const int lw = dot_lanes(M * N * nb, K);
-      const double warps = std::ceil((double)(M * N * nb) * (double)(1 << lw) / 32.0);
-      const double per = std::ceil((double)K / (double)(1 << lw)) * ((ac && bc) ? 4.0 : (ac || bc) ? 2.0 : 1.0) + 2.0 * lw;
-      const double cost = 2200.0 + std::ceil(warps / 608.0) * per * 66.0;
+      const double cost = dot_cost(M * N * nb, K, dot_lanes(M * N * nb, K), ac, bc);
       if (cost < best * 0.999) {
         best = cost;
         *best_tile = t;
@@ -76,6 +80,7 @@ void choose_fx(long long M, long long N, long long K, long long nb, bool ac, boo
       }
     }
   }
+  return best;
 }
 
 namespace {

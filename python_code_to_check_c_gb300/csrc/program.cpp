@@ -257,9 +257,11 @@ void Program::ein(const char* spec, double ar, double ai, const View& A, const V
 
 // Form and K splits (splits only where the output is zeroed or accumulated
 // into: they add with atomics), from the kernels' cost model.  Dot products or
-// fixed-point tiles is decided once, from the extents the op is first planned
-// with; K splits and the tensor-core form (deep_splits) follow the batch, so a
-// batched program's last bits may differ from its single-trajectory one's.
+// fixed-point tiles is decided from the extents the op is first planned with and
+// kept for a batch, whose roundings are then a single trajectory's, until another
+// form is twice as fast (T2 at o=4, v=8 with 96 trajectories: 1085 us as dot products
+// throughout).  K splits and the tensor-core form (deep_splits) follow the batch too, so
+// the last bits of a batched program may differ from a single one's.
 void Program::plan_gemm(Op& op, bool allow_split, int tile) {
   GemmArgs& g = op.g;
   const long long K = g.K, nb = std::max(g.nb, 1);
@@ -268,6 +270,12 @@ void Program::plan_gemm(Op& op, bool allow_split, int tile) {
   if (op.dot == -2) {
     choose_fx(g.M, g.N, K, nb, ac, bc, allow_split, -3, &op.tile, &splits);
     op.dot = op.tile == 5 ? dot_lanes((long long)g.M * g.N * nb, K) : -1;
+  }
+  if (op.dot >= 0 && tile == -1) {
+    const long long outputs = (long long)g.M * g.N * nb;
+    const double now = dot_cost(outputs, K, op.dot, ac, bc);
+    if (now > 2.0 * choose_fx(g.M, g.N, K, nb, ac, bc, allow_split, -3, &op.tile, &splits))
+      op.dot = op.tile == 5 ? dot_lanes(outputs, K) : -1;
   }
   if (op.dot >= 0) {
     op.tile = 5;
