@@ -36,10 +36,12 @@ constexpr int kPhaseOps = 160;
 constexpr int kBarrierLimit = 1 << 21;
 constexpr unsigned kLost = 1u << 16;  // in the count of blocks that are out: one gave up a wait
 // Phases with more work keep a launch per op: there the blocks of several ops
-// fill the chip without waiting for one another.  Measured (one launch per
-// phase against one per op): T2 residual 86 and 243 us at o=3, v=8, 105 and
-// 248 at o=4, v=8 (2 Mflop a phase); a step at o=6, v=12 (15 Mflop) 0.91 and
-// 0.49 ms; a gradient's host side (capture, instantiation) 1.1 and 7.3 ms.
+// fill the chip without waiting for one another.  Measured (one launch per phase
+// against one per op; Mflop of the phase, us): T2 residuals of o=4..6, v=8..13 2.5 111
+// 248, 4.7 130 220, 8.2 155 225, 16 200 226, 27 262 242.  But a phase of few large
+// contractions, as T1's and L1's of larger systems are, loses far below that: with the
+// line at 9 instead of 3 8 steps at o=10, v=14 took 15.2 ms for 10.1, a step at o=8, v=12
+// 1.63 for 1.28, the ground state at o=10, v=14 16.6 for 9.9.
 constexpr double kPhaseFlops = 3e6;
 constexpr size_t kPhaseTempMax = 64u << 20;
 constexpr size_t kPhaseTableMax = 1u << 20;   // index table entries (8 bytes each)
