@@ -31,7 +31,12 @@
 //
 // A row whose maximum is not finite (or that holds subnormals only) is marked
 // by the packing with 8 slices; its outputs, and those that the range guard sends
-// on, are done by FP64 multiply-adds over the operands, a warp for four rows of a column.
+// on, are done by FP64 multiply-adds over the operands: where few of a warp's outputs are
+// marked, its lanes over k for four rows of a column; where many are, a lane a row for
+// four columns.  Many are where a molecule's symmetry forbids elements and leaves noise
+// in them (10^-16 of the others, three quarters of the outputs): the FP64 pipe is then
+// the bound, T2 residual at o=10, v=38 7.5 ms by the former alone, 5.2 so, 0.9 without
+// noise, and 5.1 with or without it on the FP64 pipe throughout.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -137,6 +142,62 @@ __device__ __noinline__ void direct_dots(const TcArgs& g, const int (&m)[kDirect
     s[i].x = __shfl_sync(0xffffffffu, v[0], LV * (AC || BC ? 2 * i : i));
     s[i].y = AC || BC ? __shfl_sync(0xffffffffu, v[0], LV * (2 * i + 1)) : 0.0;
   }
+}
+
+// The same for row m of each lane and columns n .. n + 3, one lane over all of k (the
+// two lanes of a complex row share it): nothing to meet but those two, and the four
+// columns read a row's elements once.  m, n may lie outside (their sums are not used).
+template <bool AC, bool BC>
+__device__ __noinline__ void direct_rows(const TcArgs& g, int m, int n, int z, int k0, int k1, double2 (&s)[kDirect]) {
+  const int lane = threadIdx.x & 31;
+  long long ao, bo[kDirect], dummy;
+  decode2(g.gmA, min(m, g.M - 1), ao, dummy);
+  ao += z * g.bsA;
+#pragma unroll
+  for (int i = 0; i < kDirect; ++i) {
+    decode2(g.gnB, min(n + i, g.N - 1), bo[i], dummy);
+    bo[i] += z * g.bsB;
+    s[i] = make_double2(0.0, 0.0);
+  }
+  const double *A = static_cast<const double*>(g.srcA), *B = static_cast<const double*>(g.srcB);
+  for (int kk = k0; kk < k1; kk += 32) {  // a K offset a lane, handed round
+    const int kn = min(32, k1 - kk);
+    long long ka = 0, kb = 0;
+    if (lane < kn) decode2(g.gkAB, kk + lane, ka, kb);
+    double2 c[kDirect];
+#pragma unroll
+    for (int i = 0; i < kDirect; ++i) c[i] = make_double2(0.0, 0.0);
+#pragma unroll 2
+    for (int j = 0; j < kn; j += AC ? 2 : 1) {
+      const int k = AC ? j + (lane & 1) : j;
+      const long long xa = __shfl_sync(0xffffffffu, ka, k), yb = __shfl_sync(0xffffffffu, kb, k);
+      if (k >= kn) continue;
+      const double2 x = load1<AC>(A, ao + xa);
+#pragma unroll
+      for (int i = 0; i < kDirect; ++i) {
+        const double2 y = load1<BC>(B, bo[i] + yb);
+        if constexpr (AC && BC) {
+          fmac(c[i], x, y);
+        } else if constexpr (AC) {
+          c[i] = make_double2(fma(x.x, y.x, c[i].x), fma(x.y, y.x, c[i].y));
+        } else {
+          c[i].x = fma(x.x, y.x, c[i].x);
+          if constexpr (BC) c[i].y = fma(x.x, y.y, c[i].y);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kDirect; ++i) {
+      s[i].x += c[i].x;
+      if constexpr (AC || BC) s[i].y += c[i].y;
+    }
+  }
+  if constexpr (AC)
+#pragma unroll
+    for (int i = 0; i < kDirect; ++i) {
+      s[i].x += __shfl_xor_sync(0xffffffffu, s[i].x, 1);
+      s[i].y += __shfl_xor_sync(0xffffffffu, s[i].y, 1);
+    }
 }
 
 template <class C, bool AC, bool BC>
@@ -404,29 +465,52 @@ __global__ void __launch_bounds__(C::THREADS, 1)
             for (int k = 0; k < NL; ++k)
               put(k, BC ? make_double2(value(2 * k), value(2 * k + 1)) : make_double2(value(k), 0.0));
           }
-          // what the guard found, four rows of a column at a time
+          // what the guard found, four columns at a time: where few of their outputs
+          // are marked, the warp's lanes over k for four rows of one column
 #pragma unroll 1
-          for (int k = 0; !lost && __any_sync(0xffffffffu, direct != 0u) && k < NL; ++k) {
-            const int n = nt * (BC ? C::BN / 2 : C::BN) + (BC ? (j0 + g0) / 2 : j0 + g0) + k;
-            const bool mine = m < g.M && n < g.N && !(AC && odd) && ((direct >> (BC ? g0 + 2 * k : g0 + k)) & (BC ? 3u : 1u));
-            unsigned rows = __ballot_sync(0xffffffffu, mine);
-            __syncwarp();  // the staged values are written
-            while (rows) {
-              int src[kDirect], mm[kDirect];
+          for (int kq = 0; !lost && __any_sync(0xffffffffu, direct != 0u) && kq < NL; kq += kDirect) {
+            static_assert(NL % kDirect == 0, "columns in fours");
+            const int n = nt * (BC ? C::BN / 2 : C::BN) + (BC ? (j0 + g0) / 2 : j0 + g0) + kq;
+            unsigned mine = 0u;  // bit i: this row's column n + i
 #pragma unroll
-              for (int i = 0; i < kDirect; ++i) {
-                src[i] = rows ? __ffs(rows) - 1 : -1;
-                rows &= rows - 1u;
-                mm[i] = __shfl_sync(0xffffffffu, m, max(src[i], src[0]));
-              }
+            for (int i = 0; i < kDirect; ++i)
+              if (m < g.M && n + i < g.N && !(AC && odd) && ((direct >> (BC ? g0 + 2 * (kq + i) : g0 + kq + i)) & (BC ? 3u : 1u)))
+                mine |= 1u << i;
+            __syncwarp();  // the staged values are written
+            const int marked = (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(mine));
+            // (the lanes over k: a quarter of K and some 64 multiply-adds' time to meet for
+            // four outputs; a lane a row: 8 K for 128)
+            if (marked * (k1 - k0 + 256) > (AC ? 64 : 128) * (k1 - k0)) {
               double2 s[kDirect];
-              direct_dots<AC, BC>(g, mm, n, zb, k0, k1, s);
+              direct_rows<AC, BC>(g, m, n, zb, k0, k1, s);
 #pragma unroll
               for (int i = 0; i < kDirect; ++i)
-                if (lane == src[i]) {
+                if (mine >> i & 1u) {
                   if (g.alpha_pow2) s[i] = make_double2(g.ar * s[i].x, g.ar * s[i].y);
-                  put(k, s[i]);
+                  put(kq + i, s[i]);
                 }
+              continue;
+            }
+#pragma unroll 1
+            for (int k = 0; k < kDirect; ++k) {
+              unsigned rows = __ballot_sync(0xffffffffu, (mine >> k) & 1u);
+              while (rows) {
+                int src[kDirect], mm[kDirect];
+#pragma unroll
+                for (int i = 0; i < kDirect; ++i) {
+                  src[i] = rows ? __ffs(rows) - 1 : -1;
+                  rows &= rows - 1u;
+                  mm[i] = __shfl_sync(0xffffffffu, m, max(src[i], src[0]));
+                }
+                double2 s[kDirect];
+                direct_dots<AC, BC>(g, mm, n + k, zb, k0, k1, s);
+#pragma unroll
+                for (int i = 0; i < kDirect; ++i)
+                  if (lane == src[i]) {
+                    if (g.alpha_pow2) s[i] = make_double2(g.ar * s[i].x, g.ar * s[i].y);
+                    put(kq + k, s[i]);
+                  }
+              }
             }
           }
         } else {
