@@ -347,7 +347,8 @@ typedef struct tdcc_op_record {
   int kind;       /* 0 contraction, 1 elementwise, 2 trace, 3 RK4 / field    */
   int block;      /* 0..3 = T1, T2, L1, L2 block; 4 = density; 5 = step      */
   int stage;      /* 0 = prologue (once per step), 1..4 = RK4 stage          */
-  int backend;    /* contractions: 0 FP64 CUDA cores, 1 tensor cores         */
+  int backend;    /* contractions: 0 the FP64 form on CUDA cores, 1 tensor
+                     cores, 2 slice products on the FP32 pipe              */
   double flops;   /* real floating-point operations of the op               */
   double bytes;   /* compulsory bytes read + written by the op              */
   double ms;      /* device time from CUDA events on the launching stream    */

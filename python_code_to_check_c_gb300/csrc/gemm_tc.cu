@@ -17,11 +17,11 @@
 // at one K index add up to at most 2^14 + 2^13 + 2^13 = 2^15 in magnitude
 // (level 7 of S = 6; 2^14 + 2^13 + 2^12 for level 6), so the FP32 level sums
 // over a 512-wide K chunk stay within 2^24 and are exact integers; after
-// every chunk the epilogue warps drain the TMEM
-// accumulators into FP64 registers with their 2^(-7L) weights.  The final
-// value is scaled back by 2^(e_row + e_col); real/imaginary rows of complex
-// operands are combined with a lane-pair shuffle and written through the
-// same strided output decoder as the FP64 kernel.
+// every chunk the drain warps join the levels exactly, as integers (sums over
+// several chunks as int64 in spare TMEM columns).  The final sum becomes a
+// double once, scaled back by 2^(e_row + e_col); real/imaginary rows of complex
+// operands are combined with a lane-pair shuffle and written through a
+// strided output decoder.
 //
 // Pipeline (two variants, TcCfg in gemm_tc.h): warp 0 issues TMA loads
 // (SWIZZLE_128B) into a shared-memory ring, one (A_s, B_s) slice pair per
