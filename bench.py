@@ -538,7 +538,8 @@ def run_ours(args, rank, world, local_rank):
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
     except Exception:
         pass
-    pairs = args.slices * (args.slices + 1) // 2  # slice products per FP64 product (levels 2..S+1)
+    slices = 8 if prec == "fp64" else args.slices
+    pairs = slices * (slices + 1) // 2  # slice products per FP64 product (levels 2..S+1)
     if kern == "ozaki_kernel":
         achieved = dom["flops"] / (dom["ms"] / 1e3) / 1e12
         peak = peaks.get("bf16_tflops", 1900.0)
@@ -546,10 +547,19 @@ def run_ours(args, rank, world, local_rank):
                 "peak_source": "measured bf16 burst (MEASURED_PEAKS.json)" if "bf16_tflops" in peaks else "fallback",
                 "achieved_is": "FP64-equivalent algorithmic flops of the step's slice products / their launch time",
                 "tensor_work_frac": achieved * pairs / peak}
-    elif kern in ("gemm_fx_kernel", "simt_slices_kernel"):
+    elif kern == "gemm_fx_kernel":
+        # 26 wide integer multiply-adds a clock and SM (measured), three a real product; the
+        # group's FP64 dot products (small contractions) count at the same rate
         achieved = dom["flops"] / (dom["ms"] / 1e3) / 1e12
-        peak = 1.25
-        roof = {"bound": "fp64", "unit": "TFLOP/s", "peak_source": "nominal GB300 FP64 (no measured FP64 peak)"}
+        peak = 2 * 26 / 3 * 152 * 2.07e9 / 1e12
+        roof = {"bound": "integer", "unit": "TFLOP/s",
+                "peak_source": "measured wide integer multiply-adds (26 a clock and SM), three a real product",
+                "includes": "the FP64 dot products of small contractions"}
+    elif kern == "simt_slices_kernel":
+        achieved = dom["flops"] / (dom["ms"] / 1e3) / 1e12
+        peak = 2 * 128 * 152 * 2.07e9 / 1e12 / pairs
+        roof = {"bound": "fp32", "unit": "TFLOP/s",
+                "peak_source": f"nominal FP32 multiply-adds (128 a clock and SM), {pairs} a real product"}
     else:
         achieved = dom["bytes"] / (dom["ms"] / 1e3) / 1e9
         peak = peaks.get("hbm_gbs", 6800.0)
