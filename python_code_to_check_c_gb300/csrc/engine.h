@@ -354,7 +354,7 @@ class Program {
   // contractions left out with K <= simt_max_k and at least simt_min_macs
   // multiply-adds run as slice products on the FP32 pipe (GB_SIMT)
   // prec_mode 0 (FP64): the contractions that are faster so become 8-slice
-  // products (deep form), if their packed operands fit in deep_bytes
+  // products (deep form), as many as have their packed operands in deep_bytes
   void select_backend(int prec_mode, long long min_macs, int slices, int min_k, int min_mn, int simt_max_k,
                       long long simt_min_macs, long long deep_bytes);
   int err_slot = -1;  // U8 slot holding the tensor-core kernels' error flag

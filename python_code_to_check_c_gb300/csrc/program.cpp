@@ -922,8 +922,8 @@ static void merge_pack_modes(ModeGroup& g) {
 // where the choice lies (3.0, 2.2 and 1.7 here: residuals of 20 systems, o = 5..14 and
 // v = 14..50, within 1 % of each other); a deep tile takes 7.3 per K block and 15 for
 // its first loads, its drain and the guard, one per SM; packing an operand that is not
-// an integral block 3 and its traffic at 3 TB/s.
-static int deep_splits(const Op& op) {
+// an integral block 3 and its traffic at 3 TB/s.  gain: what the model saves.
+static int deep_splits(const Op& op, double* gain) {
   constexpr int BM = 128, BN = 64, BK = 64, kMinK = 32;
   const GemmArgs& g = op.g;
   const double K = g.K, nb = std::max(g.nb, 1);
@@ -949,23 +949,42 @@ static int deep_splits(const Op& op) {
   };
   pack(op.sa, (double)g.M * (g.bsA ? nb : 1), op.dta);
   pack(op.sb, (double)g.N * (g.bsB ? nb : 1), op.dtb);
+  *gain = fx - deep;
   return deep < 0.85 * fx ? splits : 0;
 }
 
 void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k, int min_mn, int simt_max_k,
                              long long simt_min_macs, long long deep_bytes) {
   const bool deep = prec_mode == 0;
+  std::vector<int> dsplit(ops.size(), 0);
   if (deep) {
     S = TC_DEEP_SLICES;
-    // all of them or none: the packed operands have to fit
+    // the packed operands have to fit: those that save most for their bytes stay (T2 at
+    // o=24, v=160 packs 41 GB in all, of which the ladder, a third of the step, 11)
+    struct Cand {
+      size_t op;
+      double bytes, gain;
+    };
+    std::vector<Cand> cand;
     double need = 0.0;
-    for (const auto& op : ops)
-      if (op.kind == OP_GEMM && deep_splits(op) > 0) {
-        const double nb = std::max(op.g.nb, 1), kp = (double)rup(op.g.K, 64) * 2.0 * tc_planes(S);
-        need += kp * ((double)rup(op.g.M * (op.dta == C64 ? 2LL : 1LL), 128) * (op.g.bsA ? nb : 1.0) +
-                      (double)rup(op.g.N * (op.dtb == C64 ? 2LL : 1LL), 64) * (op.g.bsB ? nb : 1.0));
-      }
-    if (need == 0.0 || need > (double)deep_bytes) return;
+    for (size_t i = 0; i < ops.size(); ++i) {
+      const Op& op = ops[i];
+      double gain = 0.0;
+      if (op.kind != OP_GEMM || (dsplit[i] = deep_splits(op, &gain)) == 0) continue;
+      const double nb = std::max(op.g.nb, 1), kp = (double)rup(op.g.K, 64) * 2.0 * tc_planes(S);
+      cand.push_back({i, kp * ((double)rup(op.g.M * (op.dta == C64 ? 2LL : 1LL), 128) * (op.g.bsA ? nb : 1.0) +
+                               (double)rup(op.g.N * (op.dtb == C64 ? 2LL : 1LL), 64) * (op.g.bsB ? nb : 1.0)),
+                      gain});
+      need += cand.back().bytes;
+    }
+    std::stable_sort(cand.begin(), cand.end(),
+                     [](const Cand& x, const Cand& y) { return x.gain * y.bytes < y.gain * x.bytes; });
+    size_t out = 0;
+    for (; out < cand.size() && need > (double)deep_bytes; ++out) {
+      dsplit[cand[out].op] = 0;
+      need -= cand[out].bytes;
+    }
+    if (out == cand.size()) return;
   } else if (S < 2 || S > 6) {
     throw std::runtime_error("slices must be 2..6");
   }
@@ -1001,7 +1020,7 @@ void Program::select_backend(int prec_mode, long long min_macs, int S, int min_k
       continue;
     }
     const long long M = op.g.M, N = op.g.N, K = op.g.K;
-    const int dsplits = deep ? deep_splits(op) : 0;
+    const int dsplits = dsplit[&op - ops.data()];
     if (deep && dsplits == 0) {
       push_op(op);
       continue;
