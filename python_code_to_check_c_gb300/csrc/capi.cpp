@@ -1836,13 +1836,15 @@ int tdcc_tei_from_df(const double* B, int n, int nq, double* tei, void* stream) 
     g.acc = 0;
     g.nb = 1;
     // The two operands are one matrix of n^2 rows: packed once, and the product
-    // is symmetric, so the tensor cores do the tiles on and above its diagonal
-    // (5 us to pack, 32 us a wave of 152 tiles at K = 144; the fixed-point tiles
-    // do 4.3 multiply-adds a clock and SM).  n = 48, K = 144: 526 -> 146 us in
-    // all.  Short of scratch, or inside a capture, the fixed-point tiles.
+    // is symmetric, so the tensor cores do the tiles on and above its diagonal (packing
+    // and launches 20 us, a wave of 152 tiles 15 and 7.3 a K block); the fixed-point tiles
+    // do 2.2 multiply-adds a clock and SM where the choice lies, up to 3.7 on large grids.
+    // Tiles against tensor cores, us in all: n = 24, K = 200 115, 63; n = 28, K = 84 79,
+    // 49; n = 30, K = 90 92, 50; n = 48, K = 144 670, 150.  Short of scratch, or inside a
+    // capture, the fixed-point tiles.
     const double kb = std::ceil(nq / 64.0), half = 0.5 * std::ceil(n2 / 128.0) * (std::ceil(n2 / 64.0) + 1.0);
-    const double t_deep = 12.0 + std::ceil(half / 152.0) * (kb * 6.5 + 13.0);
-    const double t_fx = 6.0 + (double)n2 * n2 * nq / (152.0 * 4.3 * 2070.0);
+    const double t_deep = 20.0 + std::ceil(half / 152.0) * (kb * 7.3 + 15.0);
+    const double t_fx = 6.0 + (double)n2 * n2 * nq / (152.0 * 2.2 * 2070.0);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cap));
     const long long rows = (n2 + 127) / 128 * 128, kpad = (nq + 63) / 64 * 64LL;
