@@ -61,10 +61,13 @@ namespace {
 // rounding of each factor 2^-64.8).  A plane of each packed operand holds the magnitudes
 // x, y in 8 bits; after the slices one more product on the tensor cores gives S = sum
 // x y, against which FP64 chains are off by 0.46 x 2^-53 (normal rows) to 0.9 (the
-// residuals' own, K = 81 .. 1444).  An output with S < kGuardDeep sqrt(K), that is with
+// residuals' own, K = 81 .. 1444).  An output with S < 2^-10 sqrt(K), that is with
 // an error above 0.65 x 2^-53 S (rms), is done by FP64 multiply-adds; S = 0 has no product
-// that is not zero.  A part of a K split takes its S for its share of the whole.
-constexpr float kGuardDeep = 0x1p-10f;
+// that is not zero.  A part of a K split takes its S for its share of the whole.  The
+// planes hold 2^15 x, from 2^-31 of a row's maximum up, and what lies below it as that:
+// K such products reach the limit for no K below 2^42 (2^-16, without the factor, did
+// from K = 4096 on).
+constexpr float kGuardDeep = 0x1p20f;  // 2^-10 in the planes' units
 
 template <class C>
 struct DeepShared {

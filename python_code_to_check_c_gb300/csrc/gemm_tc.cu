@@ -97,9 +97,9 @@ __device__ __forceinline__ void store_digit_pair(uint32_t* out, size_t plane2, s
     out[5 * plane2] = digit_pair<16, false, 8>(l0, l1, sgn);
     out[6 * plane2] = digit_pair<8, false, 8>(l0, l1, sgn);
     out[7 * plane2] = digit_pair<0, false, 8>(l0, l1, sgn);
-    // the range guard's plane (gemm_deep.cu): the magnitudes in 8 bits, only zeros as
-    // zero; a row fills half of a slice's
-    const float f0 = scaled_magnitude(x0, e), f1 = scaled_magnitude(x1, e);
+    // the range guard's plane (gemm_deep.cu): 2^15 |x| 2^-e in 8 bits, which reach down to
+    // 2^-31 of the maximum; only zeros as zero; a row fills half of a slice's
+    const float f0 = scaled_magnitude(x0, e) * 0x1p15f, f1 = scaled_magnitude(x1, e) * 0x1p15f;
     const float2 f = make_float2(x0 != 0.0 ? fmaxf(f0, 0x1p-16f) : 0.f, x1 != 0.0 ? fmaxf(f1, 0x1p-16f) : 0.f);
     const size_t row = 2 * (idx2 - k / 2);  // the row's first BF16
     reinterpret_cast<uint16_t*>(out - idx2)[16 * plane2 + row + k / 2] = __nv_cvt_float2_to_fp8x2(f, __NV_SATFINITE, __NV_E5M2);
