@@ -564,7 +564,8 @@ def run_ours(args, rank, world, local_rank):
         achieved = dom["bytes"] / (dom["ms"] / 1e3) / 1e9
         peak = peaks.get("hbm_gbs", 6800.0)
         roof = {"bound": "hbm", "unit": "GB/s", "peak_source": "measured HBM copy (MEASURED_PEAKS.json)"}
-    traffic = TRAFFIC_RATIO[kern] * dom["bytes"] / dom["n"] if kern in TRAFFIC_RATIO else None
+    # (the ratio was measured on the mixed form's products)
+    traffic = TRAFFIC_RATIO[kern] * dom["bytes"] / dom["n"] if kern in TRAFFIC_RATIO and prec == "mixed" else None
     roof.update({"kernel": kern, "achieved": achieved, "peak": peak, "frac": achieved / peak,
                  "traffic": traffic,
                  "traffic_source": TRAFFIC_SOURCE if traffic else None,

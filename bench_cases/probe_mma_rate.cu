@@ -6,8 +6,8 @@
 // product on the same stage (mode 1); operand values constant (data 0) or
 // random integers in [-64, 64] (data 1); one CTA or one per SM.
 //
-//   nvcc -gencode arch=compute_103a,code=sm_103a -O3 -o gpurun_out/probe_mma_rate bench_cases/probe_mma_rate.cu
-//   gpurun_out/probe_mma_rate
+//   nvcc -gencode arch=compute_103a,code=sm_103a -O3 -o build/probe_mma_rate bench_cases/probe_mma_rate.cu
+//   build/probe_mma_rate
 #include <cstdio>
 #include <cstdint>
 #include <cuda_runtime.h>

@@ -5,8 +5,8 @@
 // issues the loads; each stage is issued again as soon as it lands.  Every
 // wait is bounded.
 //
-//   nvcc -gencode arch=compute_103a,code=sm_103a -O3 -o gpurun_out/probe_tma_bw bench_cases/probe_tma_bw.cu -lcuda
-//   gpurun_out/probe_tma_bw
+//   nvcc -gencode arch=compute_103a,code=sm_103a -O3 -o build/probe_tma_bw bench_cases/probe_tma_bw.cu -lcuda
+//   build/probe_tma_bw
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
