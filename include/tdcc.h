@@ -57,10 +57,12 @@ enum {
                               (eight-slice tensor-core products) or some 78-bit
                               numbers (integer pipe) under each real row's
                               maximum, and by FP64 multiply-adds where a row
-                              spans too much for that.  An output is off by
-                              no more than 2^-53 of the sum of its products'
-                              magnitudes (rms; FP64 chains: 0.5 to 1), at any
-                              range of the operands.  FP64 everywhere else   */
+                              spans too much for that.  At any range of the
+                              operands an output is off by no more than a chain
+                              of FP64 multiply-adds leaves (rms): 2^-53 of the
+                              sum of its products' magnitudes, up to twice
+                              that where a few products outweigh the others
+                              (chains: 0.5 to 12).  FP64 everywhere else       */
   TDCC_PREC_MIXED = 1      /* large contractions as split-BF16 tcgen05
                               products, FP64 everywhere else               */
 };
